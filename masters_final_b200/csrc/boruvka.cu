@@ -2286,9 +2286,7 @@ static int csr_graph_run(int mode, const int32_t *dest, const WT *weight, int wb
             // the first phase reads every row and needs many warps to keep
             // its loads in flight; the skipping phase touches few rows
             // the kept-entry records (dynamic) on top of the static staging pass 48 KB
-            EACB_CUDA(cudaFuncSetAttribute((const void *)k_phase_csr<SEL_MST, WT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)kPhRecBytes));
+            EACB_CUDA((allow_max_dyn_smem(k_phase_csr<SEL_MST, WT>)));
             k_phase_csr<SEL_MST, WT><<<ph.slot == 0 ? gr : gph, kPhThreads, kPhRecBytes, st>>>(
                 first, deg, dest, weight, V, E, wbits, 0, 0, g.lohi, ph.slot, ph.slot == 0 ? 1 : 0,
                 ph.slot > 0 ? g.giant : nullptr, g.label, pk, g.ea,
@@ -2305,9 +2303,7 @@ static int csr_graph_run(int mode, const int32_t *dest, const WT *weight, int wb
         // every entry with identity labels: one word per undirected edge and
         // each vertex's first selection (the reference's round one)
         if (E > 0) {
-            EACB_CUDA(cudaFuncSetAttribute((const void *)k_phase_csr<SEL_CC, WT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)kPhRecBytes));
+            EACB_CUDA((allow_max_dyn_smem(k_phase_csr<SEL_CC, WT>)));
             k_phase_csr<SEL_CC, WT><<<gr, kPhThreads, kPhRecBytes, st>>>(
                 first, deg, dest, weight, V, E, wbits, -1, 255, nullptr, 0, 1, nullptr, g.label, pk,
                 g.ea, (unsigned long long *)&g.cnt[C_CURSOR], (unsigned long long)g.Emax, g.best,

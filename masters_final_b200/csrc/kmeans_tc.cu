@@ -734,8 +734,7 @@ int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *
                              ? (size_t)(kExactThreads / 32) * kmax * sizeof(float) : 0;
     int es = EACB_OK;
     auto exact = [&](auto kern) {
-        if (esmem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                      (int)esmem) != cudaSuccess)
+        if (esmem > 48 * 1024 && allow_max_dyn_smem(kern) != cudaSuccess)
             es = EACB_ERR_CUDA;
         else
             kern<<<148 * 8, kExactThreads, esmem, st>>>(X, n, D, C, kk, kmax, P, amb, namb, s.err,
