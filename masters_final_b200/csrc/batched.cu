@@ -107,6 +107,35 @@ struct ArenaBlock {
     }
 };
 
+// The workers' streams, destroyed once every worker has left.
+class WorkerStreams {
+  public:
+    explicit WorkerStreams(int32_t n)
+    {
+        st_.reserve((size_t)n);
+        for (int32_t i = 0; i < n; ++i) {
+            cudaStream_t s = nullptr;
+            const cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+            if (e != cudaSuccess) {
+                note_cuda_error((int)e, __FILE__, __LINE__);
+                break;
+            }
+            st_.push_back(s);
+        }
+    }
+    ~WorkerStreams()
+    {
+        for (cudaStream_t s : st_) cudaStreamDestroy(s);
+    }
+    WorkerStreams(const WorkerStreams &) = delete;
+    WorkerStreams &operator=(const WorkerStreams &) = delete;
+    size_t size() const { return st_.size(); }
+    cudaStream_t operator[](size_t i) const { return st_[i]; }
+
+  private:
+    std::vector<cudaStream_t> st_;
+};
+
 struct Slice {
     int32_t *labels;       // P x n
     float *centroids;      // P x kmax x d
@@ -269,11 +298,16 @@ extern "C" int eacb_batched_eac(eacb_instance *inst, int32_t n_inst,
         inst[i].cuda_error = inst[i].cuda_line = 0;
     }
     std::atomic<int32_t> next(0);
-    const int32_t nw = std::min(n_workers, n_inst);
+    // Every worker's stream is made here, before any work is queued: making
+    // one while other streams are busy waits for their work (80 ms a worker
+    // in a 48-dataset batch, most of the call), on an idle device it is
+    // microseconds.  Fewer streams than asked: fewer workers.
+    WorkerStreams streams(std::min(n_workers, n_inst));
+    const int32_t nw = (int32_t)streams.size();
+    if (nw < 1) return EACB_ERR_CUDA;
     auto worker = [&](int w) {
         if (cudaSetDevice(dev) != cudaSuccess) return;
-        cudaStream_t st = nullptr;
-        if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return;
+        const cudaStream_t st = streams[w];
         // instances run side by side: each one's Boruvka rounds take one
         // block (a plain launch) instead of a cooperative grid over the GPU
         if (nw > 1) eacb::set_thread_round_team(1);
@@ -292,7 +326,6 @@ extern "C" int eacb_batched_eac(eacb_instance *inst, int32_t n_inst,
             if (I.status) cudaStreamSynchronize(st);   // nothing of it left in flight
         }
         eacb::set_thread_round_team(0);
-        cudaStreamDestroy(st);
     };
     std::vector<std::thread> pool;
     try {
