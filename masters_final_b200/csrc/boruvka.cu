@@ -2207,8 +2207,7 @@ struct Engine {
             return EACB_OK;
         }
         const int64_t ntiles = (n_in + kETile - 1) / kETile;
-        EACB_CUDA(cudaMemsetAsync(scan.status, 0, sizeof(uint64_t) * ntiles, st));
-        EACB_CUDA(cudaMemsetAsync(scan.counter, 0, sizeof(int), st));
+        EACB_CUDA(scan.clear(ntiles, false, st));
         k_edge_tile<MODE, Src><<<(unsigned)ntiles, kET, 0, st>>>(
             src, n_in, out, best, scan.status, scan.counter, &cnt[C_AUX0], err);
         EACB_CHECK_LAUNCH();

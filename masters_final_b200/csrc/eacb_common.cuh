@@ -255,43 +255,64 @@ __device__ __forceinline__ uint64_t status_load(const uint64_t *st)
     return v;
 }
 
+// Each tile's word has a 128-byte line of its own: every block in flight polls
+// its predecessors, and words that share lines make all of them meet on the
+// few lines around the newest tiles.
+//
 // Called by warp 0 of the block with the tile aggregate; returns (to every
-// lane of warp 0) the exclusive prefix of this tile.
+// lane of warp 0) the exclusive prefix of this tile.  The blocks in flight
+// have mostly published aggregates only, so a tile looks back over hundreds
+// of predecessors; a step covers kLookback x 32 of them with all loads in
+// flight together.
+constexpr int kStatusStride = 16;     // words
+constexpr int kLookback = 4;
+
 __device__ __forceinline__ int64_t lookback(uint64_t *status, int64_t tile, int64_t agg,
                                             int64_t init, int *err)
 {
     const int lane = threadIdx.x & 31;
     if (tile == 0) {
-        if (lane == 0) status_store(&status[0], kFlagInc | ((uint64_t)(init + agg) & kValMask));
+        if (lane == 0) status_store(status, kFlagInc | ((uint64_t)(init + agg) & kValMask));
         return init;
     }
-    if (lane == 0) status_store(&status[tile], kFlagAgg | ((uint64_t)agg & kValMask));
-    int64_t prefix = 0;
+    if (lane == 0) status_store(&status[tile * kStatusStride], kFlagAgg | ((uint64_t)agg & kValMask));
+    int64_t mine = 0;                 // this lane's share of the prefix
     int64_t pos = tile - 1;           // highest tile not yet folded in
     int spins = 0;
-    while (true) {
-        int64_t t = pos - lane;
-        uint64_t s = (t >= 0) ? status_load(&status[t]) : (kFlagInc);  // t<0 never happens before an inclusive
-        unsigned empty = __ballot_sync(0xffffffffu, (s >> 62) == 0);
-        if (empty) {
-            if (++spins > kSpinLimit) {
-                if (lane == 0) set_err(err, DEV_SPIN_LIMIT);
-                break;
-            }
-            continue;
-        }
-        unsigned inc = __ballot_sync(0xffffffffu, (s >> 62) == 2);
-        // fold lanes [0, first inclusive] (lane 0 = tile pos)
-        int stop = inc ? (__ffs(inc) - 1) : 31;
-        int64_t v = (lane <= stop) ? status_val(s) : 0;
+    bool found = false;
+    while (!found) {
+        uint64_t s[kLookback];
 #pragma unroll
-        for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-        prefix += v;
-        if (inc) break;
-        pos -= 32;
+        for (int k = 0; k < kLookback; ++k) {
+            const int64_t t = pos - 32 * k - lane;
+            s[k] = t >= 0 ? status_load(&status[t * kStatusStride]) : kFlagInc;   // past tile 0, which is inclusive
+        }
+        // fold the groups of 32 in order, up to the first one that is not
+        // complete (its rest is read again) or holds an inclusive prefix
+        int folded = 0;
+#pragma unroll
+        for (int k = 0; k < kLookback; ++k) {
+            if (found || folded != k) continue;
+            const unsigned empty = __ballot_sync(0xffffffffu, (s[k] >> 62) == 0);
+            const unsigned inc = __ballot_sync(0xffffffffu, (s[k] >> 62) == 2);
+            // tiles before the first inclusive one need not be there yet
+            const int stop = inc ? __ffs(inc) - 1 : 31;
+            if (empty & (0xffffffffu >> (31 - stop))) continue;
+            if (lane <= stop) mine += status_val(s[k]);
+            found = inc != 0u;
+            ++folded;
+        }
+        pos -= 32 * folded;
+        if (!found && folded == 0 && ++spins > kSpinLimit) {
+            if (lane == 0) set_err(err, DEV_SPIN_LIMIT);
+            break;
+        }
     }
+    int64_t prefix = mine;
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) prefix += __shfl_xor_sync(0xffffffffu, prefix, d);
     if (lane == 0)
-        status_store(&status[tile], kFlagInc | ((uint64_t)(prefix + agg) & kValMask));
+        status_store(&status[tile * kStatusStride], kFlagInc | ((uint64_t)(prefix + agg) & kValMask));
     return prefix;
 }
 

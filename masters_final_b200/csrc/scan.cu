@@ -3,11 +3,11 @@
 // Replaces MyML/MyML/utils/scan.py:144-249 (scan_gpu: a recursive Blelloch
 // scan with one launch per level plus a fix-up pass, int only) and the CPU
 // scans :42-72.  One launch: each CTA takes the next tile index from an
-// atomic counter, reduces 16 elements per thread loaded with 128-bit loads,
-// scans the thread sums across the CTA (warp shuffles + a Blelloch tree over
-// warp totals), obtains its tile prefix by looking back over its
+// atomic counter, loads 16 elements per thread with 128-bit loads that a warp
+// makes back to back, scans them with warp shuffles and the warps' totals
+// with one more, obtains its tile prefix by looking back over its
 // predecessors' published aggregates, and writes its outputs.  HBM traffic is
-// one read and one write of the stream.
+// one read and one write of the stream.  A short stream takes one CTA.
 #include "eacb_common.cuh"
 #include "scan_impl.cuh"
 
@@ -28,9 +28,8 @@ static int scan_entry(const TIn *in, TOut *out, int64_t n, int64_t init, int64_t
     Carver c(ws, ws_bytes);
     ScanScratch s = ScanScratch::carve(c, n);
     if (c.overflow) return EACB_ERR_WORKSPACE;
-    if (n > 0) EACB_CUDA(cudaMemsetAsync(s.err, 0, sizeof(int), as_stream(stream)));
     ProfScope ps(PROF_SCAN, as_stream(stream));
-    int st = scan_launch<TIn, TOut>(in, out, n, init, d_total, s, as_stream(stream));
+    int st = scan_launch<TIn, TOut>(in, out, n, init, d_total, s, as_stream(stream), true);
     ps.done((double)n * (sizeof(TIn) + sizeof(TOut)));
     return st;
 }

@@ -4,24 +4,55 @@
 
 namespace eacb {
 
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 24;
-constexpr int64_t kScanTile = (int64_t)kScanThreads * kScanItems;
+// Tile shape.  Bound by HBM (one read and one write of the stream), and
+// before that by the look-back: with the status words of neighbouring tiles
+// in one line, the polls of every block in flight met on a few lines and a
+// tile took 25-40 ns whatever its size (64 Mi int32: 186 us with 6,144
+// elements per tile, 1 word apart; 170 us with 16,384).  So each tile has a
+// line of its own (kStatusStride), and 128 bytes per thread keep the tiles
+// few and the loads many.  A warp owns consecutive elements and each of its
+// 16-byte loads and stores covers 512 consecutive bytes, so every line is
+// touched once.  64 Mi int32: 110 us (4.9 TB/s); 135 us with the wide tiles
+// alone, 118 with status words 32 bytes apart.
+constexpr int kScanThreads = 512;
+constexpr int kScanWarps = kScanThreads / 32;
+// elements per thread: 128 bytes of the wider type, or 64 while that leaves
+// SMs without a tile
+template <typename TIn, typename TOut>
+constexpr int kScanWide = 128 / (int)(sizeof(TIn) > sizeof(TOut) ? sizeof(TIn) : sizeof(TOut));
+template <typename TIn, typename TOut> constexpr int kScanNarrow = kScanWide<TIn, TOut> / 2;
+constexpr int64_t kScanWideMin = 148;     // wide tiles from one per SM
+constexpr int64_t scan_tile(int items) { return (int64_t)kScanThreads * items; }
+// up to this many elements one block scans the stream by itself
+constexpr int kScanSmallThreads = 1024;
+constexpr int kScanSmallItems = 16;
+constexpr int64_t kScanSmallStep = (int64_t)kScanSmallThreads * kScanSmallItems;
+constexpr int64_t kScanSmallMax = 2 * kScanSmallStep;
 
 struct ScanScratch {
-    uint64_t *status;
-    int *counter;
-    int *err;
+    uint64_t *status;      // kStatusStride words per tile, from the counter's line on
+    int *counter;          // tile counter
+    int *err;              // its own sits in the line before the counter's
     int64_t max_tiles;
+    // lines: [own error word] [counter] [tile 0] [tile 1] ...
     static ScanScratch carve(Carver &c, int64_t n, int *err = nullptr)
     {
         ScanScratch s;
-        s.err = err ? err : c.take<int>(1);
         // sized for the smallest tile any single-pass kernel uses (2048)
         s.max_tiles = (n + 2047) / 2048 + 1;
-        s.status = c.take<uint64_t>(s.max_tiles);
-        s.counter = c.take<int>(1);
+        uint64_t *w = c.take<uint64_t>((size_t)(s.max_tiles + 2) * kStatusStride);
+        s.err = err ? err : (int *)w;
+        s.counter = (int *)(w + kStatusStride);
+        s.status = w + 2 * kStatusStride;
         return s;
+    }
+    // zeroes the tile counter and `tiles` status lines (and, with_err, the
+    // scratch's own error word) in one memset
+    cudaError_t clear(int64_t tiles, bool with_err, cudaStream_t st) const
+    {
+        const size_t line = kStatusStride * sizeof(uint64_t);
+        char *p = (char *)counter - (with_err ? line : 0);
+        return cudaMemsetAsync(p, 0, (size_t)((char *)status - p) + (size_t)tiles * line, st);
     }
 };
 
@@ -29,112 +60,217 @@ template <typename T> struct Vec16;
 template <> struct Vec16<int32_t> { typedef int4 type; static constexpr int n = 4; };
 template <> struct Vec16<int64_t> { typedef longlong2 type; static constexpr int n = 2; };
 
-template <typename TOut>
-__device__ __forceinline__ TOut narrow(int64_t v) { return (TOut)v; }
-template <>
-__device__ __forceinline__ int32_t narrow<int32_t>(int64_t v) { return (int32_t)(uint32_t)(uint64_t)v; }
-
-template <typename TIn, typename TOut, bool VEC>
-__global__ void __launch_bounds__(kScanThreads)
-k_scan(const TIn *__restrict__ in, TOut *__restrict__ out, int64_t n, int64_t init,
-       uint64_t *status, int *counter, int64_t *total, int *err, const int64_t *d_n = nullptr)
+// a 16-byte input vector's outputs in one store: 16 bytes, or 32 where int32
+// widens to int64 (two 16-byte stores would each write half sectors)
+__device__ __forceinline__ void store_vec(int32_t *p, const int32_t (&o)[4])
 {
+    __stcs(reinterpret_cast<int4 *>(p), make_int4(o[0], o[1], o[2], o[3]));
+}
+__device__ __forceinline__ void store_vec(int64_t *p, const int64_t (&o)[2])
+{
+    __stcs(reinterpret_cast<longlong2 *>(p), make_longlong2(o[0], o[1]));
+}
+__device__ __forceinline__ void store_vec(int64_t *p, const int64_t (&o)[4])
+{
+    asm volatile("st.global.cs.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(o[0]), "l"(o[1]),
+                 "l"(o[2]), "l"(o[3])
+                 : "memory");
+}
+
+// Prefixes inside a tile: int32 outputs are stored modulo 2^32, so theirs are
+// scanned in 32 bits; totals and the tiles' prefixes are always 64-bit.
+template <typename TOut> struct ScanAcc { typedef int64_t type; };
+template <> struct ScanAcc<int32_t> { typedef uint32_t type; };
+
+__device__ __forceinline__ uint32_t warp_incl(uint32_t v)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += o;
+    }
+    return v;
+}
+__device__ __forceinline__ int64_t warp_incl(int64_t v) { return warp_incl_sum(v); }
+
+// exact warp sum of values below 2^47 in magnitude (two 32-bit reductions)
+__device__ __forceinline__ int64_t warp_sum_47(int64_t v)
+{
+    const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)(v & 0xffffff));
+    const int hi = __reduce_add_sync(0xffffffffu, (int)(v >> 24));
+    return ((int64_t)hi << 24) + (int64_t)lo;
+}
+
+// A thread's share of a step: ITEMS elements as ITEMS / VN groups of VN
+// consecutive ones (VN: elements of a 16-byte input vector), group j of lane
+// l at first + (j * 32 + l) * VN.
+template <typename TIn, typename TOut, bool VEC, int ITEMS>
+struct ScanItems {
+    typedef typename ScanAcc<TOut>::type Acc;
+    static constexpr int VN = Vec16<TIn>::n;
+    static constexpr int NG = ITEMS / VN;
+    static constexpr int64_t kWarpSpan = 32 * ITEMS;
+    TIn v[ITEMS];
+    Acc pre[NG];               // sum of the warp's elements before the group
+
+    // elements of [first, n); the rest read as zero
+    __device__ __forceinline__ void load(const TIn *in, int64_t first, int64_t n, bool full)
+    {
+        const int lane = threadIdx.x & 31;
+        if (VEC && full) {
+            typedef typename Vec16<TIn>::type V;
+            const V *p = reinterpret_cast<const V *>(in + first) + lane;
+#pragma unroll
+            for (int j = 0; j < NG; ++j) {
+                const V x = __ldcs(p + j * 32);
+                memcpy(&v[j * VN], &x, sizeof(V));
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) {
+                const int64_t e = first + (int64_t)((q / VN) * 32 + lane) * VN + q % VN;
+                v[q] = e < n ? in[e] : TIn(0);
+            }
+        }
+    }
+
+    // prefixes of the groups within the warp; returns the warp's exact total
+    __device__ __forceinline__ int64_t scan_warp()
+    {
+        Acc run = 0;
+        int64_t exact = 0;
+#pragma unroll
+        for (int j = 0; j < NG; ++j) {
+            int64_t s = 0;
+#pragma unroll
+            for (int e = 0; e < VN; ++e) s += (int64_t)v[j * VN + e];
+            exact += s;
+            const Acc inc = warp_incl((Acc)s);
+            pre[j] = run + inc - (Acc)s;
+            run += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        // a 64-bit running sum is the total already; a 32-bit one has lost
+        // the high part (a lane's 32 int32 values stay below 2^37)
+        if (sizeof(Acc) == 8) return (int64_t)run;
+        return warp_sum_47(exact);
+    }
+
+    __device__ __forceinline__ void store(TOut *out, int64_t first, int64_t n, bool full,
+                                          int64_t base) const
+    {
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int j = 0; j < NG; ++j) {
+            Acc run = (Acc)base + pre[j];
+            TOut o[VN];
+#pragma unroll
+            for (int e = 0; e < VN; ++e) {
+                o[e] = (TOut)run;
+                run += (Acc)v[j * VN + e];
+            }
+            const int64_t e0 = first + (int64_t)(j * 32 + lane) * VN;
+            if (VEC && full) {
+                store_vec(out + e0, o);
+            } else {
+#pragma unroll
+                for (int e = 0; e < VN; ++e)
+                    if (e0 + e < n) out[e0 + e] = o[e];
+            }
+        }
+    }
+};
+
+template <typename TIn, typename TOut, bool VEC, int ITEMS>
+__global__ void __launch_bounds__(kScanThreads, 2)
+k_scan(const TIn *__restrict__ in, TOut *__restrict__ out, int64_t n, int64_t init,
+       uint64_t *status, int *counter, int64_t *total, int *err)
+{
+    typedef ScanItems<TIn, TOut, VEC, ITEMS> Items;
+    constexpr int64_t kTile = scan_tile(ITEMS);
     __shared__ int s_tile;
-    __shared__ int64_t s_prefix;
-    // with d_n the length is read on the device and the grid is sized for
-    // the largest length: surplus blocks take tile ids past the end and leave
-    if (d_n) n = *d_n;
+    __shared__ int64_t s_warp[kScanWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1);
     __syncthreads();
     const int64_t tile = s_tile;
-    if (tile * kScanTile >= n && !(n == 0 && tile == 0)) return;
-    if (n == 0) {
-        if (threadIdx.x == 0 && total) *total = init;
-        return;
-    }
-    const int64_t base = tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
-    TIn v[kScanItems];
-    const bool full = base + kScanItems <= n;
-    if (VEC && full) {
-        typedef typename Vec16<TIn>::type V;
-        const V *p = reinterpret_cast<const V *>(in + base);
-#pragma unroll
-        for (int i = 0; i < kScanItems / Vec16<TIn>::n; ++i) {
-            V x = __ldcs(p + i);
-            memcpy(&v[i * Vec16<TIn>::n], &x, sizeof(V));
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < kScanItems; ++i) v[i] = (base + i < n) ? in[base + i] : TIn(0);
-    }
-    int64_t sum = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) sum += (int64_t)v[i];
-    int64_t agg;
-    int64_t excl = block_excl_sum<kScanThreads>(sum, agg);
-    if (threadIdx.x < 32) {
-        int64_t pre = lookback(status, tile, agg, init, err);
-        if (threadIdx.x == 0) s_prefix = pre;
+    const int64_t first = tile * kTile + (int64_t)warp * Items::kWarpSpan;
+    const bool full = (tile + 1) * kTile <= n;
+    Items it;
+    it.load(in, first, n, full);
+    const int64_t wt = it.scan_warp();
+    if (lane == 0) s_warp[warp] = wt;
+    __syncthreads();
+    if (warp == 0) {
+        // the warps' totals become their prefixes in the whole stream
+        const int64_t x = lane < kScanWarps ? s_warp[lane] : 0;
+        const int64_t inc = warp_incl_sum(x);
+        const int64_t agg = __shfl_sync(0xffffffffu, inc, 31);
+        const int64_t pre = lookback(status, tile, agg, init, err);
+        if (lane < kScanWarps) s_warp[lane] = pre + inc - x;
+        if (lane == 0 && (tile + 1) * kTile >= n && total) *total = pre + agg;
     }
     __syncthreads();
-    int64_t run = s_prefix + excl;
-    TOut o[kScanItems];
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        o[i] = narrow<TOut>(run);
-        run += (int64_t)v[i];
+    it.store(out, first, n, full, s_warp[warp]);
+}
+
+// A short stream on one block: no tile state to clear and no look-back.
+// clear_err: an error word to zero on the way (null: leave it).
+template <typename TIn, typename TOut, bool VEC>
+__global__ void __launch_bounds__(kScanSmallThreads)
+k_scan_small(const TIn *__restrict__ in, TOut *__restrict__ out, int64_t n, int64_t init,
+             int64_t *total, int *clear_err)
+{
+    typedef ScanItems<TIn, TOut, VEC, kScanSmallItems> Items;
+    __shared__ int64_t s_warp[2][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int64_t run = init;
+    int ph = 0;
+    for (int64_t base = 0; base < n; base += kScanSmallStep, ph ^= 1) {
+        const int64_t first = base + (int64_t)warp * Items::kWarpSpan;
+        const bool full = base + kScanSmallStep <= n;
+        Items it;
+        it.load(in, first, n, full);
+        const int64_t wt = it.scan_warp();
+        if (lane == 0) s_warp[ph][warp] = wt;      // the other half was read one barrier ago
+        __syncthreads();
+        const int64_t x = s_warp[ph][lane];
+        const int64_t inc = warp_incl_sum(x);
+        it.store(out, first, n, full, run + __shfl_sync(0xffffffffu, inc - x, warp));
+        run += __shfl_sync(0xffffffffu, inc, 31);
     }
-    if (VEC && full) {
-        typedef typename Vec16<TOut>::type V;
-        V *p = reinterpret_cast<V *>(out + base);
-#pragma unroll
-        for (int i = 0; i < kScanItems / Vec16<TOut>::n; ++i) {
-            V x;
-            memcpy(&x, &o[i * Vec16<TOut>::n], sizeof(V));
-            __stcs(p + i, x);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < kScanItems; ++i)
-            if (base + i < n) out[base + i] = o[i];
+    if (threadIdx.x == 0) {
+        if (total) *total = run;
+        if (clear_err) *clear_err = 0;
     }
-    const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    if (tile == ntiles - 1 && threadIdx.x == 0 && total) *total = s_prefix + agg;
 }
 
 __global__ void k_set_i64(int64_t *p, int64_t v);
 
-// Clears look-back state with a kernel (usable where memset nodes are not).
-__global__ void k_clear_status(uint64_t *status, int64_t n, int *counter);
-
-// Scan whose length is read on the device (*d_n <= max_n); no memset calls,
-// so it can be captured into a conditional graph body.  With clear = false
-// the caller's previous kernel has already zeroed the look-back state
-// (status words [0, ceil(max_n / kScanTile)) and the tile counter).
-template <typename TIn, typename TOut>
-inline int scan_launch_dev(const TIn *in, TOut *out, const int64_t *d_n, int64_t max_n,
-                           int64_t init, int64_t *d_total, const ScanScratch &s, cudaStream_t st,
-                           bool clear = true)
+template <typename TIn, typename TOut, int ITEMS>
+inline int scan_launch_tiles(const TIn *in, TOut *out, int64_t n, int64_t init, int64_t *d_total,
+                             const ScanScratch &s, cudaStream_t st, bool clear_err, bool vec)
 {
-    const int64_t ntiles = (max_n + kScanTile - 1) / kScanTile;
-    const int64_t grid = ntiles > 0 ? ntiles : 1;
-    if (clear) {
-        k_clear_status<<<grid_for(grid, 256, 148 * 4), 256, 0, st>>>(s.status, grid, s.counter);
-        EACB_CHECK_LAUNCH();
-    }
-    if (((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0))
-        k_scan<TIn, TOut, true><<<(unsigned)grid, kScanThreads, 0, st>>>(
-            in, out, max_n, init, s.status, s.counter, d_total, s.err, d_n);
+    const int64_t ntiles = (n + scan_tile(ITEMS) - 1) / scan_tile(ITEMS);
+    if (ntiles > (int64_t)0x7fffffff) return EACB_ERR_UNSUPPORTED;
+    EACB_CUDA(s.clear(ntiles, clear_err, st));
+    if (vec)
+        k_scan<TIn, TOut, true, ITEMS><<<(unsigned)ntiles, kScanThreads, 0, st>>>(
+            in, out, n, init, s.status, s.counter, d_total, s.err);
     else
-        k_scan<TIn, TOut, false><<<(unsigned)grid, kScanThreads, 0, st>>>(
-            in, out, max_n, init, s.status, s.counter, d_total, s.err, d_n);
+        k_scan<TIn, TOut, false, ITEMS><<<(unsigned)ntiles, kScanThreads, 0, st>>>(
+            in, out, n, init, s.status, s.counter, d_total, s.err);
     EACB_CHECK_LAUNCH();
     return EACB_OK;
 }
 
+// clear_err: also zero the scratch's own error word (the one in the line
+// before the counter).  Up to kScanSmallMax elements (two steps of one
+// block) the clearing memset and the look-back cost more than the one
+// block's second step does.
 template <typename TIn, typename TOut>
 inline int scan_launch(const TIn *in, TOut *out, int64_t n, int64_t init, int64_t *d_total,
-                       const ScanScratch &s, cudaStream_t st)
+                       const ScanScratch &s, cudaStream_t st, bool clear_err = false)
 {
     if (n == 0) {
         if (d_total) {
@@ -143,19 +279,25 @@ inline int scan_launch(const TIn *in, TOut *out, int64_t n, int64_t init, int64_
         }
         return EACB_OK;
     }
-    const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    if (ntiles > (int64_t)0x7fffffff) return EACB_ERR_UNSUPPORTED;
-    EACB_CUDA(cudaMemsetAsync(s.status, 0, sizeof(uint64_t) * ntiles, st));
-    EACB_CUDA(cudaMemsetAsync(s.counter, 0, sizeof(int), st));
-    const bool vec = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0);
-    if (vec)
-        k_scan<TIn, TOut, true><<<(unsigned)ntiles, kScanThreads, 0, st>>>(
-            in, out, n, init, s.status, s.counter, d_total, s.err);
-    else
-        k_scan<TIn, TOut, false><<<(unsigned)ntiles, kScanThreads, 0, st>>>(
-            in, out, n, init, s.status, s.counter, d_total, s.err);
-    EACB_CHECK_LAUNCH();
-    return EACB_OK;
+    // 16-byte input vectors, and as many outputs as one holds in one store
+    const bool vec = ((uintptr_t)in % 16 == 0) &&
+                     ((uintptr_t)out % (16 / sizeof(TIn) * sizeof(TOut)) == 0);
+    if (n <= kScanSmallMax) {
+        int *ce = clear_err ? s.err : nullptr;
+        if (vec)
+            k_scan_small<TIn, TOut, true><<<1, kScanSmallThreads, 0, st>>>(in, out, n, init,
+                                                                          d_total, ce);
+        else
+            k_scan_small<TIn, TOut, false><<<1, kScanSmallThreads, 0, st>>>(in, out, n, init,
+                                                                           d_total, ce);
+        EACB_CHECK_LAUNCH();
+        return EACB_OK;
+    }
+    constexpr int kWide = kScanWide<TIn, TOut>, kNarrow = kScanNarrow<TIn, TOut>;
+    if (n < kScanWideMin * scan_tile(kWide))
+        return scan_launch_tiles<TIn, TOut, kNarrow>(in, out, n, init, d_total, s, st, clear_err,
+                                                     vec);
+    return scan_launch_tiles<TIn, TOut, kWide>(in, out, n, init, d_total, s, st, clear_err, vec);
 }
 
 }  // namespace eacb

@@ -7,10 +7,10 @@
 // application and has no allocator to draw a workspace from.  Such callers
 // cannot provide the workspace that eacb_scan_excl_i32 asks for.
 //
-// How: the scan's look-back scratch (one status word per 4096-element tile,
-// a tile counter and an error word) lives in a fixed array in device memory,
+// How: the scan's look-back scratch (a status word per 16,384-element tile, a
+// tile counter and an error word, each in a 128-byte line) lives in a fixed array in device memory,
 // defined below.  It is part of the library's image: every GPU that loads
-// libeacb200 holds it (about 350 KiB) until the process exits.  The device
+// libeacb200 holds it (about 2 MiB) until the process exits.  The device
 // address of that array is looked up once per device with
 // cudaGetSymbolAddress (a lookup, not an allocation), on the first call made
 // while that device is current; make that first call before any stream
@@ -28,11 +28,13 @@
 
 namespace {
 
-// n up to 2^28 elements -> 43,691 tiles of 6,144
+// n up to 2^28 elements -> 16,385 tiles of 16,384; fewer but smaller tiles
+// below kScanWideMin of them
 constexpr int64_t kNoAllocMaxN = EACB_SCAN_NOALLOC_MAX_N;
-constexpr int64_t kNoAllocTiles = kNoAllocMaxN / eacb::kScanTile + 1;
-// layout: [0] error word, [8..16) tile counter, [256..) tile status words
-constexpr size_t kNoAllocBytes = 256 + (size_t)kNoAllocTiles * sizeof(uint64_t);
+constexpr int64_t kNoAllocTiles = kNoAllocMaxN / eacb::scan_tile(eacb::kScanWide<int32_t, int32_t>) + 1;
+constexpr size_t kLine = eacb::kStatusStride * sizeof(uint64_t);
+// lines: [0] error word, [1] tile counter, [2 ..] tile status words
+constexpr size_t kNoAllocBytes = (2 + (size_t)kNoAllocTiles) * kLine;
 
 static __device__ __align__(256) unsigned char g_scan_scratch[kNoAllocBytes];
 
@@ -68,15 +70,15 @@ extern "C" int eacb_scan_excl_i32_noalloc(const int32_t *in, int32_t *out, int64
     if (s) return s;
     eacb::ScanScratch sc;
     sc.err = (int *)base;
-    sc.counter = (int *)(base + 8);
-    sc.status = (uint64_t *)(base + 256);
+    sc.counter = (int *)(base + kLine);
+    sc.status = (uint64_t *)(base + 2 * kLine);
     sc.max_tiles = kNoAllocTiles;
     cudaStream_t st = (cudaStream_t)stream;
-    // the previous call's contents are still there: clear what starts at zero
-    // (scan_launch clears the tile counter and the status words it uses)
-    EACB_CUDA(cudaMemsetAsync(sc.err, 0, sizeof(int), st));
+    // the previous call's contents are still there: scan_launch clears what
+    // has to start at zero (error word, tile counter, the status words it uses)
+    if (n == 0) EACB_CUDA(cudaMemsetAsync(sc.err, 0, sizeof(int), st));
     eacb::ProfScope ps(eacb::PROF_SCAN, st);
-    s = eacb::scan_launch<int32_t, int32_t>(in, out, n, init, d_total, sc, st);
+    s = eacb::scan_launch<int32_t, int32_t>(in, out, n, init, d_total, sc, st, true);
     ps.done((double)n * 2.0 * sizeof(int32_t));
     if (s) return s;
     // report a device-side failure of this call (a look-back wait that gave

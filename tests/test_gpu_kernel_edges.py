@@ -1,0 +1,39 @@
+"""Kernels and dispatch branches at the sizes where they change: tile edges,
+remainders, the smallest and largest of a range.  Everything compared here is
+whole numbers or float32 results with a fixed order of operations, so every
+comparison is exact."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# the one-block scan's step and limit, the tile of the look-back scan
+SCAN_STEP, SCAN_SMALL_MAX, SCAN_TILE = 16384, 32768, 8192
+
+
+@pytest.mark.parametrize("types", ["i32_i32", "i32_i64", "i64_i64"])
+@pytest.mark.parametrize("n", [1, 3, 511, 513, SCAN_STEP - 1, SCAN_STEP, SCAN_STEP + 1,
+                               SCAN_SMALL_MAX - 5, SCAN_SMALL_MAX, SCAN_SMALL_MAX + 1,
+                               5 * SCAN_TILE, 5 * SCAN_TILE + 1, 40 * SCAN_TILE + 4099])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_scan_edges(types, n, offset):
+    """Both scans against numpy's running sum in 64 bits, aligned and one
+    element off the 16-byte boundary, negative values and an initial value."""
+    import torch
+    from masters_final_b200.utils.scan import exprefixsumNumba, exprefixsumNumbaSingle
+    ti, to = {"i32_i32": (np.int32, np.int32), "i32_i64": (np.int32, np.int64),
+              "i64_i64": (np.int64, np.int64)}[types]
+    rng = np.random.default_rng(n + offset)
+    hi = 1 << 31 if ti == np.int32 else 1 << 40
+    x = rng.integers(-hi, hi, size=n).astype(ti)
+    c = np.cumsum(x.astype(np.int64)) + 7
+    want = np.concatenate([[7], c[:-1]]).astype(np.int64).astype(to)
+    xd = torch.empty(n + offset, dtype=getattr(torch, np.dtype(ti).name), device="cuda")[offset:]
+    od = torch.empty(n + offset, dtype=getattr(torch, np.dtype(to).name), device="cuda")[offset:]
+    xd.copy_(torch.from_numpy(x))
+    assert exprefixsumNumba(xd, od, 7) == int(c[-1])
+    assert np.array_equal(od.cpu().numpy(), want)
+    assert np.array_equal(xd.cpu().numpy(), x)
+    if ti == to:                                       # in place
+        assert exprefixsumNumbaSingle(xd, 7) == int(c[-1])
+        assert np.array_equal(xd.cpu().numpy(), want)
