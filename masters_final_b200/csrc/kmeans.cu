@@ -26,6 +26,8 @@
 #include "members.cuh"
 #include "kmeans_common.cuh"
 
+#include <cooperative_groups.h>
+
 #include <type_traits>
 
 namespace eacb {
@@ -316,75 +318,95 @@ __global__ void k_centroids(const float *__restrict__ X, int32_t n, int32_t D,
 
 // Empty clusters take the points arg_k_select returns for their number
 // (KMeans.py:727-750, MyML/MyML/utils/sorting.py:9-47): the reference's
-// quickselect on (distance, index) pairs, one block per partition, with the
-// distances permuted in place (key[r] is the reference's a[args[r]]; the
-// distances are not needed again before the next label pass).
+// quickselect on (distance, index) pairs, one thread-block cluster per
+// partition, with the distances permuted in place (key[r] is the reference's
+// a[args[r]]; the distances are not needed again before the next label pass).
 //
 // One partition step of the reference on [lo, hi] with pivot mid moves the
 // element at r to the back (swapping in the element at w) when it is >= mid,
-// and otherwise advances r.  Its result has a closed form that a block can
-// compute in parallel.  Read the range from the front (F[t] = position
-// lo + t) and from the back (B[u] = position hi - u); "big" means >= mid.
-// The step examines F up to its m-th big a_m, then B up to its m-th small
-// b_m, then F again, and so on, until hi - lo + 1 elements are examined; the
-// last one examined stays at r.  Every other examined element lands at:
-//   a front small F[t]       -> position of F[t] (it stays),
-//   the m-th front big       -> position of B[b_{m-1} + 1]   (b_0 = -1),
-//   the m-th back small      -> position of F[a_m],
-//   a back big B[u]          -> position of B[u + 1],
-// and r = lo + (number of smalls that landed).  Ranges up to kFillSeqMax
-// elements finish with the reference's loop on one thread: its dependent
-// loads cost about as much per element as a parallel step costs per range,
-// so the handover is at a few hundred elements.
+// and otherwise advances r.  Its result has a closed form that a cluster can
+// compute in parallel.  Count positions t from lo; "big" means >= mid, NS is
+// the number of the others ("small").  The step reads the range from the
+// front and from the back, and the two readings meet behind position x: x is
+// NS - 1 when the element at position NS is small (or there is none), else
+// NS.  The element read last is the one at x (read from the front) when that
+// completes the reading, else the one at x + 1:
+//   x = NS - 1: at x when it is small, else at x + 1;
+//   x = NS:     at x when x is the end or the element at x + 1 is small,
+//               else at x + 1.
+// It stays at r.  With A the bigs at positions <= x (from the front) and B
+// the smalls behind x (from the back), every other element lands at:
+//   a front small           -> its own position,
+//   the m-th front big      -> one before B's (m-1)-th position (the end for m = 1),
+//   the m-th back small     -> A's m-th position,
+//   a back big              -> one position further front,
+// and r = lo + NS, less one if the last element is small.
+//
+// The reference goes on in [lo, r] when its target k is at most r, and only
+// those positions are read again: then the step is just "B's m-th element
+// replaces A's m-th" (k is the number of empty clusters, so nearly every step
+// is one).  Otherwise all elements move.
+//
+// Bound by the passes over the range (two reads of the keys and one of the
+// lists, halving from step to step) and a cluster barrier between them: with
+// one block per partition and all elements moved in each step a 2,000,000
+// point partition took 18.4 ms, all of it one SM; eight blocks take 0.77 ms.
+// Ranges up to kFillSeqMax elements finish with the reference's loop on one
+// thread in shared memory.
 constexpr int kFillThreads = 1024;
 constexpr int kFillItems = 8;
-constexpr int64_t kFillSeqMax = 256;
-constexpr int64_t kFillInf = (int64_t)1 << 62;
+constexpr int kFillTile = kFillThreads * kFillItems;
+constexpr int kFillSeqMax = 256;
+constexpr int kFillRounds = 1 << 15;     // steps shrink the range; equal keys take one per cluster
+// blocks per partition: a cluster from this many points on (below, one
+// block's passes cost no more than the cluster's barriers)
+constexpr int kFillCluster = 8;
+constexpr int kFillClusterMin = 16384;
 
-// Walks [lo, hi] in ascending order, calling f(p, big, bigs_before) for every
-// position (bigs_before = # bigs in [lo, p)); returns the number of bigs.
-// Called by the whole block.
+// Walks [t0, t1) in ascending tiles, calling f(t, big, before) for every
+// position; before packs the front bigs (high half) and back smalls (low
+// half) of the walk before t, on top of `base`.  x splits front and back.
 template <typename F>
-__device__ int64_t fill_scan_bigs(const float *key, int64_t lo, int64_t hi, float mid, F f)
+__device__ __forceinline__ void fill_walk(const float *key, int t0, int t1, float mid, int x,
+                                          int64_t base, F f)
 {
-    int64_t base = 0;
-    for (int64_t t0 = lo; t0 <= hi; t0 += (int64_t)kFillThreads * kFillItems) {
-        const int64_t p0 = t0 + (int64_t)threadIdx.x * kFillItems;
+    for (int64_t b = t0; b < t1; b += kFillTile) {
+        const int64_t p0 = b + (int64_t)threadIdx.x * kFillItems;
         unsigned mask = 0;
-        int c = 0;
+        int64_t c = 0;
 #pragma unroll
         for (int q = 0; q < kFillItems; ++q) {
-            const int64_t p = p0 + q;
-            if (p <= hi && key[p] >= mid) {
-                mask |= 1u << q;
-                ++c;
+            const int64_t t = p0 + q;
+            if (t < t1) {
+                const bool big = key[t] >= mid;
+                mask |= (big ? 1u : 0u) << q;
+                c += big ? (t <= x ? (1ll << 32) : 0ll) : (t > x ? 1ll : 0ll);
             }
         }
         int64_t tot;
-        int64_t before = base + block_excl_sum<kFillThreads>(c, tot);
+        int64_t before = base + block_excl_sum_shfl<kFillThreads>(c, tot);
 #pragma unroll
         for (int q = 0; q < kFillItems; ++q) {
-            const int64_t p = p0 + q;
-            if (p <= hi) {
+            const int64_t t = p0 + q;
+            if (t < t1) {
                 const bool big = (mask >> q) & 1u;
-                f(p, big, before);
-                before += big;
+                f((int)t, big, before);
+                before += big ? (t <= x ? (1ll << 32) : 0ll) : (t > x ? 1ll : 0ll);
             }
         }
         base += tot;
     }
-    return base;
 }
 
-// number of entries <= v in the ascending array a[0, len)
-__device__ __forceinline__ int64_t count_le(const int32_t *a, int64_t len, int64_t v)
+// smalls among [t0, t1), summed over the block
+__device__ __forceinline__ int fill_smalls(const float *key, int t0, int t1, float mid)
 {
-    int64_t lo = 0, hi = len;
-    while (lo < hi) {
-        const int64_t m = (lo + hi) >> 1;
-        if (a[m] <= v) lo = m + 1; else hi = m;
-    }
-    return lo;
+    int c = 0;
+#pragma unroll 8
+    for (int64_t t = (int64_t)t0 + threadIdx.x; t < t1; t += kFillThreads) c += !(key[t] >= mid);
+    int64_t tot;
+    block_excl_sum_shfl<kFillThreads>(c, tot);
+    return (int)tot;
 }
 
 __global__ void __launch_bounds__(kFillThreads, 1)
@@ -393,146 +415,194 @@ k_fill_empty(const float *X, int32_t n, int32_t D, float *dists, const int64_t *
              const int32_t *nempty, int32_t *args_all, int32_t *sel_all, float *okey_all,
              int32_t *oarg_all, float *C, int *err)
 {
-    __shared__ int64_t s_v[5];
-    const int p = blockIdx.x;
-    if (!active[p] || nempty[p] == 0) return;          // uniform across the block
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cl = cg::this_cluster();
+    const int CL = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    __shared__ int s_small[2], s_fb[2], s_bs[2];       // this block's counts, by step parity
+    __shared__ float s_key[kFillSeqMax];
+    __shared__ int32_t s_arg[kFillSeqMax];
+    const int p = (int)blockIdx.x / CL;
+    if (!active[p] || nempty[p] == 0) return;          // uniform across the cluster
     const int k = nempty[p];
-    float *key = dists + (int64_t)p * n;
-    int32_t *args = args_all + (int64_t)p * n;
-    int32_t *sel = sel_all + (int64_t)p * n;           // front-big and back-small indices
-    float *okey = okey_all + (int64_t)p * n;
-    int32_t *oarg = oarg_all + (int64_t)p * n;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) args[i] = (int32_t)i;
-    __syncthreads();
-    int64_t lo = 0, hi = n - 1;
-    int rounds = 0;
-    while (hi - lo + 1 > kFillSeqMax) {
-        if (++rounds > 4096) {                         // cannot happen: every step shrinks the range
-            if (threadIdx.x == 0) set_err(err, DEV_CHASE_LIMIT);
+    float *key0 = dists + (int64_t)p * n;
+    int32_t *args0 = args_all + (int64_t)p * n;
+    int32_t *sel = sel_all + (int64_t)p * n;           // positions of A, then of B
+    const int gt = rank * kFillThreads + (int)threadIdx.x, gs = CL * kFillThreads;
+    for (int64_t i = gt; i < n; i += gs) args0[i] = (int32_t)i;
+    cl.sync();
+    int lo = 0, hi = n - 1;
+    for (int step = 0; hi - lo + 1 > kFillSeqMax; ++step) {
+        if (step > kFillRounds) {                      // a NaN pivot does not shrink the range
+            if (gt == 0) set_err(err, DEV_CHASE_LIMIT);
             return;
         }
-        const int64_t L = hi - lo + 1;
-        const float mid = key[(lo + hi) / 2];
-        // count the bigs, then list front bigs (sel[0, NB)) and back smalls
-        // (sel[NB, L)) by rank
-        int64_t nbig;
-        {
-            int64_t c = 0;
-            for (int64_t q = lo + threadIdx.x; q <= hi; q += blockDim.x) c += key[q] >= mid;
-            nbig = 0;
-            block_excl_sum<kFillThreads>(c, nbig);
+        const int L = hi - lo + 1, ph = step & 1;
+        float *key = key0 + lo;
+        int32_t *args = args0 + lo;
+        const float mid = key[(int)(((int64_t)lo + hi) / 2 - lo)];
+        const int cs = (L + CL - 1) / CL;
+        const int c0 = (int)min((int64_t)L, (int64_t)rank * cs);
+        const int c1 = (int)min((int64_t)L, (int64_t)c0 + cs);
+        // the smalls of the range
+        const int mine = fill_smalls(key, c0, c1, mid);
+        if (threadIdx.x == 0) s_small[ph] = mine;
+        cl.sync();
+        int NS = 0;
+        for (int q = 0; q < CL; ++q) NS += *cl.map_shared_rank(&s_small[ph], q);
+        // where the two readings meet and which element is read last
+        const bool has = NS < L && key[NS] >= mid;     // a big at position NS
+        const int x = NS == L ? L - 1 : (has ? NS : NS - 1);
+        bool at_x;
+        if (NS == L) at_x = true;
+        else if (!has) at_x = x >= 0 && !(key[x] >= mid);
+        else at_x = x == L - 1 || !(key[x + 1] >= mid);
+        const int last = at_x ? x : x + 1;
+        const float klast = key[last];
+        const int32_t alast = args[last];
+        const int Sm = NS - (klast >= mid ? 0 : 1);
+        const int r = lo + Sm - (klast > mid ? 1 : 0);
+        // front bigs and back smalls before each block's share
+        int fb = 0, bs = 0;
+        if (c1 <= x + 1) {
+            fb = (c1 - c0) - mine;
+        } else if (c0 > x) {
+            bs = mine;
+        } else {
+            const int sf = fill_smalls(key, c0, x + 1, mid);
+            fb = (x + 1 - c0) - sf;
+            bs = mine - sf;
         }
-        const int64_t NB = nbig, NS = L - NB;
-        fill_scan_bigs(key, lo, hi, mid, [&](int64_t q, bool big, int64_t before) {
-            const int64_t t = q - lo;
-            if (big) sel[before] = (int32_t)t;
-            else sel[NB + NS - 1 - (t - before)] = (int32_t)(hi - q);   // rank from the back
-        });
-        __syncthreads();
         if (threadIdx.x == 0) {
-            const int32_t *A = sel, *Bs = sel + NB;
-            auto a_of = [&](int64_t m) -> int64_t { return m <= NB ? A[m - 1] : kFillInf; };
-            auto b_of = [&](int64_t m) -> int64_t {
-                return m == 0 ? -1 : (m <= NS ? Bs[m - 1] : kFillInf);
-            };
-            // the segment m1 in which the examination ends: first m with
-            // (a_m + 1) + (b_m + 1) >= L
-            int64_t ml = 1, mh = (NB < NS ? NB : NS) + 1;
-            while (ml < mh) {
-                const int64_t m = (ml + mh) >> 1;
-                const int64_t am = a_of(m), bm = b_of(m);
-                const bool reach = am >= kFillInf || bm >= kFillInf || am + bm + 2 >= L;
-                if (reach) mh = m; else ml = m + 1;
-            }
-            const int64_t m1 = ml, am1 = a_of(m1), bprev = b_of(m1 - 1);
-            int64_t x, y, last_front;
-            if (am1 >= kFillInf || am1 + 1 + bprev + 1 >= L) {   // ends in the front run
-                y = bprev;
-                x = L - 2 - y;
-                last_front = 1;
-            } else {                                              // ends in the back run
-                x = am1;
-                y = L - 2 - x;
-                last_front = 0;
-            }
-            const int64_t front_smalls = (x + 1) - count_le(A, NB, x);
-            const int64_t back_smalls = count_le(Bs, NS, y);
-            const int64_t lp = last_front ? lo + x : hi - y;
-            const int64_t settled_smalls = front_smalls + back_smalls - (key[lp] < mid ? 1 : 0);
-            s_v[0] = x;
-            s_v[1] = y;
-            s_v[2] = last_front;
-            s_v[3] = settled_smalls;
+            s_fb[ph] = fb;
+            s_bs[ph] = bs;
         }
-        __syncthreads();
-        const int64_t x = s_v[0], y = s_v[1], last_front = s_v[2], Sm = s_v[3];
-        fill_scan_bigs(key, lo, hi, mid, [&](int64_t q, bool big, int64_t before) {
-            const int64_t t = q - lo, u = hi - q;
-            const bool front = t <= x;
-            int64_t dst;
-            if ((front && last_front && t == x) || (!front && !last_front && u == y)) {
-                dst = Sm;
-            } else if (front) {
-                if (!big) {
-                    dst = t;
-                } else {                       // the m-th front big, m = before + 1
-                    const int64_t bm = before == 0 ? -1 : sel[NB + before - 1];
-                    dst = (L - 1) - (bm + 1);
-                }
-            } else {
-                if (!big) {                    // back small of rank (from the back)
-                    const int64_t rank = NS - 1 - (t - before);
-                    dst = sel[rank];
-                } else {
-                    dst = (L - 1) - (u + 1);
-                }
+        cl.sync();
+        int64_t base = 0;
+        int nA = 0, M = 0;
+        for (int q = 0; q < CL; ++q) {
+            const int f = *cl.map_shared_rank(&s_fb[ph], q), b = *cl.map_shared_rank(&s_bs[ph], q);
+            if (q < rank) base += ((int64_t)f << 32) + b;
+            nA += f;
+            M += b;
+        }
+        fill_walk(key, c0, c1, mid, x, base, [&](int t, bool big, int64_t before) {
+            if (t <= x) {
+                if (big) sel[before >> 32] = t;
+            } else if (!big) {
+                sel[nA + M - 1 - (int)(before & 0xffffffffll)] = t;
             }
-            okey[lo + dst] = key[q];
-            oarg[lo + dst] = args[q];
         });
-        __syncthreads();
-        for (int64_t q = lo + threadIdx.x; q <= hi; q += blockDim.x) {
-            key[q] = okey[q];
-            args[q] = oarg[q];
-        }
-        __syncthreads();
-        int64_t r = lo + Sm;
-        if (key[r] > mid) r--;
-        if (k <= r) hi = r; else lo = r + 1;
-    }
-    if (threadIdx.x != 0) return;
-    int64_t guard = 0;
-    const int64_t limit = 64 * (int64_t)n + 4096;
-    while (lo < hi) {
-        int64_t r = lo, w = hi;
-        const float mid = key[(r + w) / 2];
-        float kr = key[r];
-        while (r < w) {
-            if (kr >= mid) {
-                const float kw = key[w];
-                const int32_t t = args[w];
-                key[w] = kr;
-                args[w] = args[r];
-                key[r] = kw;
-                args[r] = t;
-                kr = kw;
-                w--;
-            } else {
-                kr = key[++r];
+        cl.sync();
+        if (k <= r) {
+            for (int64_t m = gt; m < M; m += gs) {
+                const int a = sel[m], b = sel[nA + m];
+                key[a] = key[b];
+                args[a] = args[b];
             }
-            ++guard;
+            if (gt == 0 && r == lo + NS && !at_x) {    // it equals mid and comes from x + 1
+                key[NS] = klast;
+                args[NS] = alast;
+            }
+            hi = r;
+        } else {
+            float *okey = okey_all + (int64_t)p * n + lo;
+            int32_t *oarg = oarg_all + (int64_t)p * n + lo;
+            fill_walk(key, c0, c1, mid, x, base, [&](int t, bool big, int64_t before) {
+                int dst;
+                if (t == last) dst = Sm;
+                else if (t <= x) {
+                    const int m = (int)(before >> 32);           // front bigs before
+                    dst = !big ? t : (m == 0 ? L : sel[nA + m - 1]) - 1;
+                } else {
+                    dst = big ? t - 1 : sel[M - 1 - (int)(before & 0xffffffffll)];
+                }
+                okey[dst] = key[t];
+                oarg[dst] = args[t];
+            });
+            cl.sync();
+            for (int64_t t = gt; t < L; t += gs) {
+                key[t] = okey[t];
+                args[t] = oarg[t];
+            }
+            lo = r + 1;
         }
-        if (key[r] > mid) r--;
-        if (k <= r) hi = r; else lo = r + 1;
-        if (++guard > limit) { set_err(err, DEV_CHASE_LIMIT); return; }
+        cl.sync();
     }
+    if (rank != 0) return;
+    const int L = hi - lo + 1;
+    for (int t = (int)threadIdx.x; t < L; t += kFillThreads) {
+        s_key[t] = key0[lo + t];
+        s_arg[t] = args0[lo + t];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int a = 0, b = L - 1, steps = 0;
+        while (a < b) {
+            if (++steps > kFillSeqMax) {               // a NaN pivot does not shrink the range
+                set_err(err, DEV_CHASE_LIMIT);
+                break;
+            }
+            int r = a, w = b;
+            const float mid = s_key[(int)((2 * (int64_t)lo + a + b) / 2 - lo)];
+            float kr = s_key[r];
+            while (r < w) {
+                if (kr >= mid) {
+                    const float kw = s_key[w];
+                    const int32_t t = s_arg[w];
+                    s_key[w] = kr;
+                    s_arg[w] = s_arg[r];
+                    s_key[r] = kw;
+                    s_arg[r] = t;
+                    kr = kw;
+                    w--;
+                } else {
+                    kr = s_key[++r];
+                }
+            }
+            if (s_key[r] > mid) r--;
+            if (k <= lo + r) b = r; else a = r + 1;
+        }
+    }
+    __syncthreads();
+    for (int t = (int)threadIdx.x; t < L; t += kFillThreads) args0[lo + t] = s_arg[t];
+    __syncthreads();
+    // the empty clusters, in order, take the points of args[0, k)
     const int Kp = kk[p];
     int e = 0;
-    for (int c = 0; c < Kp; ++c) {
-        if (S[((int64_t)p * K + c + 1) * ntiles] != S[((int64_t)p * K + c) * ntiles]) continue;
-        const int32_t src = args[e++];
-        for (int d = 0; d < D; ++d) C[((int64_t)p * kmax + c) * D + d] = X[(int64_t)src * D + d];
+    for (int b = 0; b < Kp; b += kFillThreads) {
+        const int c = b + (int)threadIdx.x;
+        const bool empty = c < Kp && S[((int64_t)p * K + c + 1) * ntiles] == S[((int64_t)p * K + c) * ntiles];
+        int64_t tot;
+        const int at = e + (int)block_excl_sum_shfl<kFillThreads>(empty, tot);
+        if (empty) {
+            const int32_t src = args0[at];
+            for (int d = 0; d < D; ++d) C[((int64_t)p * kmax + c) * D + d] = X[(int64_t)src * D + d];
+        }
+        e += (int)tot;
     }
+}
+
+static int launch_fill_empty(cudaStream_t st, const float *X, int32_t n, int32_t D, int32_t P,
+                             float *dists, const int64_t *S, int32_t K, int64_t ntiles,
+                             const int32_t *kk, int32_t kmax, const int32_t *active,
+                             const int32_t *nempty, int32_t *args, int32_t *sel, float *okey,
+                             int32_t *oarg, float *C, int *err)
+{
+    const unsigned cl = n >= kFillClusterMin ? kFillCluster : 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)P * cl);
+    cfg.blockDim = dim3(kFillThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = cl;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    EACB_CUDA(cudaLaunchKernelEx(&cfg, k_fill_empty, X, n, D, dists, S, K, ntiles, kk, kmax, active,
+                                 nempty, args, sel, okey, oarg, C, err));
+    EACB_CHECK_LAUNCH();
+    return EACB_OK;
 }
 
 __global__ void k_init_centroids(const float *X, int32_t D, const int32_t *init, const int32_t *kk,
@@ -701,10 +771,10 @@ extern "C" int eacb_kmeans_ensemble(const float *X, int32_t n, int32_t d, int32_
         EACB_CHECK_LAUNCH();
         // amb, mypos and members are free here (the centroids are done) and
         // serve as the quickselect's scratch
-        k_fill_empty<<<P, kFillThreads, 0, st>>>(X, n, d, w.dists, w.S, kmax, nt, k, kmax,
-                                                 w.active, w.nempty, w.args, w.amb,
-                                                 (float *)w.mypos, w.members, centroids, w.err);
-        EACB_CHECK_LAUNCH();
+        if ((s = launch_fill_empty(st, X, n, d, P, w.dists, w.S, kmax, nt, k, kmax, w.active,
+                                   w.nempty, w.args, w.amb, (float *)w.mypos, w.members,
+                                   centroids, w.err)))
+            return s;
     }
     if (dists_out)
         EACB_CUDA(cudaMemcpyAsync(dists_out, w.dists, sizeof(float) * (size_t)P * n,
@@ -851,9 +921,9 @@ extern "C" int eacb_kmeans_centroids(const float *X, int32_t n, int32_t d, const
     EACB_CHECK_LAUNCH();
     // the quickselect permutes its keys: it works on a copy of the distances
     EACB_CUDA(cudaMemcpyAsync(w.key, dists, sizeof(float) * (size_t)n, cudaMemcpyDeviceToDevice, st));
-    k_fill_empty<<<1, kFillThreads, 0, st>>>(X, n, d, w.key, w.S, k, nt, w.kk, k, w.active,
-                                             w.nempty, w.args, w.sel, w.okey, w.oarg, C, w.err);
-    EACB_CHECK_LAUNCH();
+    if ((s = launch_fill_empty(st, X, n, d, 1, w.key, w.S, k, nt, w.kk, k, w.active, w.nempty,
+                               w.args, w.sel, w.okey, w.oarg, C, w.err)))
+        return s;
     int e = 0;
     EACB_CUDA(cudaMemcpyAsync(&e, w.err, sizeof(int), cudaMemcpyDeviceToHost, st));
     EACB_CUDA(cudaStreamSynchronize(st));

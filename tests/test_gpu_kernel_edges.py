@@ -37,3 +37,27 @@ def test_scan_edges(types, n, offset):
     if ti == to:                                       # in place
         assert exprefixsumNumbaSingle(xd, 7) == int(c[-1])
         assert np.array_equal(xd.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("kind", ["random", "equal", "few", "ascending", "descending"])
+@pytest.mark.parametrize("n,empty", [(40, 3), (256, 1), (257, 5), (2000, 300), (16383, 2),
+                                     (16384, 2), (70001, 1), (70001, 300), (300001, 7)])
+def test_empty_cluster_selection(kind, n, empty):
+    """The points the empty clusters take, one block and a cluster of blocks,
+    against the oracle's quickselect: pivots that keep the lower part and
+    (equal, descending keys) ones that settle it and go on above."""
+    import torch
+    import oracle
+    from masters_final_b200.cluster.KMeans import kmeans_centroids
+    rng = np.random.default_rng(n + empty)
+    x = rng.standard_normal((n, 2)).astype(np.float32)
+    full = 5
+    k = full + empty
+    ids = np.sort(rng.choice(k, full, replace=False)).astype(np.int32)
+    labels = ids[rng.integers(0, full, n)]
+    labels[:full] = ids
+    dist = {"random": rng.random(n), "equal": np.ones(n), "few": rng.integers(0, 3, n),
+            "ascending": np.arange(n) / n, "descending": np.arange(n, 0, -1) / n}[kind].astype(np.float32)
+    got = kmeans_centroids(x, labels, dist, k).cpu().numpy()
+    want = oracle.kmeans_centroids(x, labels, dist, k)
+    assert np.array_equal(got, want)
