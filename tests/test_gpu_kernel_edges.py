@@ -61,3 +61,19 @@ def test_empty_cluster_selection(kind, n, empty):
     got = kmeans_centroids(x, labels, dist, k).cpu().numpy()
     want = oracle.kmeans_centroids(x, labels, dist, k)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 128, 129, 255, 257, 1023, 2049, 4111, 16385, 131073, 262207,
+                               1000003])
+def test_inertia_order(n):
+    """The inertia is numpy's pairwise float32 sum of the distances, bit for
+    bit, at the sizes where its split tree changes depth."""
+    from masters_final_b200.cluster.KMeans import kmeans_ensemble
+    rng = np.random.default_rng(n)
+    x = (rng.standard_normal((n, 3)) * 10).astype(np.float32)
+    ks = [1, min(2, n)]
+    inits = [[0], list(range(ks[1]))]
+    _, _, dists, _, inertia = kmeans_ensemble(x, ks, inits, max_iter=1)
+    d = dists.cpu().numpy()
+    for p in range(2):
+        assert inertia[p].item() == np.add.reduce(d[p])
