@@ -285,61 +285,142 @@ static int launch_inertia(cudaStream_t st, const float *dists, int32_t n, int32_
     return EACB_OK;
 }
 
-// float32 (reference) or float64 sums of each cluster's members in point order
-constexpr int kCentDepth = 16;       // members in flight per lane
+// float32 (reference) or float64 sums of each cluster's members in point
+// order, one warp per cluster.  The sums are sequential in member order (the
+// reference's order), so a cluster's sum is a chain as long as the cluster
+// and the largest cluster sets the kernel's time.  All lanes copy the
+// members' rows ahead into a ring of staging buffers (cp.async; three
+// batches of rows in flight, the batches' member ids further ahead in a ring
+// of their own), and lane d adds dimension d from shared memory, where the
+// chain is the additions alone.  A pass, against a lane per (cluster,
+// dimension) with 16 loads in flight: 2,000,000 x 8, 10 x 1,000 clusters 720
+// -> 380 us; 500,000 x 16, 20 x 530 clusters 485 -> 330; 1,000,000 x 2, 1,024
+// clusters 165 -> 33.
+constexpr int kCentWarps = 4;                     // warps per block
+constexpr int kCentRing = 4;                      // row buffers per warp
+constexpr int kCentIds = 2 * kCentRing;           // id buffers per warp
+constexpr int kCentFloats = 1024;                 // floats per row buffer
+constexpr int kCentBatch = 128;                   // members per buffer at most
+struct CentStage {
+    float row[kCentRing][kCentFloats];
+    int32_t id[kCentIds][kCentBatch];
+};
+constexpr size_t kCentSmem = kCentWarps * sizeof(CentStage);
 
-template <bool F64>
-__global__ void k_centroids(const float *__restrict__ X, int32_t n, int32_t D,
-                            const int32_t *__restrict__ members, const int64_t *__restrict__ S,
-                            int32_t K, int64_t ntiles, const int32_t *__restrict__ kk, int32_t kmax,
-                            const int32_t *__restrict__ active, float *C, int32_t *nempty)
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *dst, const void *src)
 {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES)
+                     : "memory");
+}
+
+// CH: floats per copy (4, 2 or 1: the largest that divides D and that X's
+// alignment allows)
+template <bool F64, int CH>
+__global__ void __launch_bounds__(kCentWarps * 32)
+k_centroids(const float *__restrict__ X, int32_t D, const int32_t *__restrict__ members,
+            const int64_t *__restrict__ S, int32_t K, int64_t ntiles,
+            const int32_t *__restrict__ kk, int32_t kmax, const int32_t *__restrict__ active,
+            float *C, int32_t *nempty)
+{
+    extern __shared__ __align__(16) uint8_t cent_smem[];
     const int p = blockIdx.y;
     if (!active[p]) return;
-    const int Kp = kk[p];
-    const int lane = threadIdx.x & 31;
-    const int G = 32 / D;                       // clusters per warp
-    const int g = lane / D, d = lane - g * D;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int c = warp * G + g;
-    if (g >= G || c >= Kp) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = blockIdx.x * kCentWarps + warp;
+    if (c >= kk[p]) return;
+    CentStage &st = reinterpret_cast<CentStage *>(cent_smem)[warp];
     const int64_t s0 = S[((int64_t)p * K + c) * ntiles], s1 = S[((int64_t)p * K + c + 1) * ntiles];
-    const int64_t cnt = s1 - s0;
-    float *out = C + ((int64_t)p * kmax + c) * D + d;
+    const int cnt = (int)(s1 - s0);
     if (cnt == 0) {
-        if (d == 0) atomicAdd(&nempty[p], 1);
+        if (lane == 0) atomicAdd(&nempty[p], 1);
         return;
     }
-    // The sums are sequential in member order (the reference's order), so a
-    // cluster's sum is a chain as long as the cluster; the largest cluster
-    // sets the kernel's time.  Members go kCentDepth at a time: the next
-    // batch's ids load while this batch's coordinates do, and the adds follow
-    // in order, so a batch costs one memory latency.
+    const int batch = min(kCentBatch, kCentFloats / D);
+    const int nb = (cnt + batch - 1) / batch;
+    const int32_t *mem = members + s0;
+    // a row is `per` copies: lane l takes copy l % per of members l / per, ...
+    const int per = D / CH, mstep = 32 / per, m_of = lane / per, ch = (lane - m_of * per) * CH;
+    auto ids = [&](int b) {
+        if (b >= nb) return;
+        const int nm = min(batch, cnt - b * batch);
+        for (int m = lane; m < nm; m += 32)
+            cp_async<4>(&st.id[b % kCentIds][m], mem + (int64_t)b * batch + m);
+    };
+    auto rows = [&](int b) {
+        if (b >= nb || m_of >= mstep) return;
+        const int nm = min(batch, cnt - b * batch);
+        const int32_t *id = st.id[b % kCentIds];
+        float *buf = st.row[b % kCentRing] + ch;
+#pragma unroll 4
+        for (int m = m_of; m < nm; m += mstep)
+            cp_async<4 * CH>(buf + m * D, X + (int64_t)id[m] * D + ch);
+    };
+    auto commit = []() { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    for (int b = 0; b < kCentRing; ++b) ids(b);
+    commit();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    // group b: the rows of batch b and the ids of batch b + kCentRing
+    for (int b = 0; b < kCentRing - 1; ++b) {
+        rows(b);
+        ids(b + kCentRing);
+        commit();
+    }
     using Acc = typename std::conditional<F64, double, float>::type;
     Acc acc = 0;
-    auto add = [&](float v) {
-        if (F64) acc += (double)v;
-        else acc = (Acc)__fadd_rn((float)acc, v);
-    };
-    int64_t m = s0;
-    if (m + kCentDepth <= s1) {
-        int32_t id[kCentDepth];
-#pragma unroll
-        for (int q = 0; q < kCentDepth; ++q) id[q] = members[m + q];
-        for (; m + kCentDepth <= s1; m += kCentDepth) {
-            float v[kCentDepth];
-#pragma unroll
-            for (int q = 0; q < kCentDepth; ++q) v[q] = X[(int64_t)id[q] * D + d];
-            const bool more = m + 2 * kCentDepth <= s1;
-#pragma unroll
-            for (int q = 0; q < kCentDepth; ++q) id[q] = more ? members[m + kCentDepth + q] : 0;
-#pragma unroll
-            for (int q = 0; q < kCentDepth; ++q) add(v[q]);
+    for (int b = 0; b < nb; ++b) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kCentRing - 2) : "memory");
+        __syncwarp();                             // batch b is there; batch b - 1 is summed
+        rows(b + kCentRing - 1);
+        ids(b + 2 * kCentRing - 1);
+        commit();
+        const int nm = min(batch, cnt - b * batch);
+        if (lane < D) {
+            const float *v = st.row[b % kCentRing] + lane;
+#pragma unroll 8
+            for (int m = 0; m < nm; ++m, v += D) {
+                if (F64) acc += (double)*v;
+                else acc = (Acc)__fadd_rn((float)acc, *v);
+            }
         }
     }
-    for (; m < s1; ++m) add(X[(int64_t)members[m] * D + d]);
+    if (lane >= D) return;
+    float *out = C + ((int64_t)p * kmax + c) * D + lane;
     if (F64) *out = __double2float_rn((double)acc / (double)cnt);
     else *out = __double2float_rn(__ddiv_rn((double)acc, (double)cnt));
+}
+
+static int launch_centroids(cudaStream_t st, bool f64, const float *X, int32_t D, int32_t P,
+                            const int32_t *members, const int64_t *S, int32_t K, int64_t ntiles,
+                            const int32_t *kk, int32_t kmax, const int32_t *active, float *C,
+                            int32_t *nempty)
+{
+    const dim3 grid((unsigned)((kmax + kCentWarps - 1) / kCentWarps), (unsigned)P);
+    cudaError_t e = cudaSuccess;
+    auto go = [&](auto kern) {
+        if ((e = allow_max_dyn_smem(kern)) != cudaSuccess) return;
+        kern<<<grid, kCentWarps * 32, kCentSmem, st>>>(X, D, members, S, K, ntiles, kk, kmax,
+                                                       active, C, nempty);
+    };
+    const int ch = D % 4 == 0 && (uintptr_t)X % 16 == 0 ? 4
+                   : D % 2 == 0 && (uintptr_t)X % 8 == 0 ? 2 : 1;
+    if (f64) {
+        if (ch == 4) go(k_centroids<true, 4>);
+        else if (ch == 2) go(k_centroids<true, 2>);
+        else go(k_centroids<true, 1>);
+    } else {
+        if (ch == 4) go(k_centroids<false, 4>);
+        else if (ch == 2) go(k_centroids<false, 2>);
+        else go(k_centroids<false, 1>);
+    }
+    EACB_CUDA(e);
+    EACB_CHECK_LAUNCH();
+    return EACB_OK;
 }
 
 // Empty clusters take the points arg_k_select returns for their number
@@ -786,16 +867,9 @@ extern "C" int eacb_kmeans_ensemble(const float *X, int32_t n, int32_t d, int32_
                                                                w.mypos);
         EACB_CHECK_LAUNCH();
         EACB_CUDA(cudaMemsetAsync(w.nempty, 0, sizeof(int32_t) * P, st));
-        const int G = 32 / d;
-        const int warps = (kmax + G - 1) / G;
-        dim3 cg((unsigned)((warps * 32 + 255) / 256), (unsigned)P);
-        if (centroid_mode == 1)
-            k_centroids<true><<<cg, 256, 0, st>>>(X, n, d, w.members, w.S, kmax, nt, k, kmax,
-                                                  w.active, centroids, w.nempty);
-        else
-            k_centroids<false><<<cg, 256, 0, st>>>(X, n, d, w.members, w.S, kmax, nt, k, kmax,
-                                                   w.active, centroids, w.nempty);
-        EACB_CHECK_LAUNCH();
+        if ((s = launch_centroids(st, centroid_mode == 1, X, d, P, w.members, w.S, kmax, nt, k, kmax,
+                                  w.active, centroids, w.nempty)))
+            return s;
         // amb, mypos and members are free here (the centroids are done) and
         // serve as the quickselect's scratch
         if ((s = launch_fill_empty(st, X, n, d, P, w.dists, w.S, kmax, nt, k, kmax, w.active,
@@ -936,16 +1010,9 @@ extern "C" int eacb_kmeans_centroids(const float *X, int32_t n, int32_t d, const
     if (place_smem > 48 * 1024) EACB_CUDA(allow_max_dyn_smem(k_ml_place));
     k_ml_place<<<(unsigned)nt, 32, place_smem, st>>>(labels, n, k, nt, w.S, w.members, w.mypos);
     EACB_CHECK_LAUNCH();
-    const int G = 32 / d;
-    const int warps = (k + G - 1) / G;
-    dim3 cg((unsigned)((warps * 32 + 255) / 256), 1u);
-    if (centroid_mode == 1)
-        k_centroids<true><<<cg, 256, 0, st>>>(X, n, d, w.members, w.S, k, nt, w.kk, k, w.active, C,
-                                              w.nempty);
-    else
-        k_centroids<false><<<cg, 256, 0, st>>>(X, n, d, w.members, w.S, k, nt, w.kk, k, w.active, C,
-                                               w.nempty);
-    EACB_CHECK_LAUNCH();
+    if ((s = launch_centroids(st, centroid_mode == 1, X, d, 1, w.members, w.S, k, nt, w.kk, k,
+                              w.active, C, w.nempty)))
+        return s;
     // the quickselect permutes its keys: it works on a copy of the distances
     EACB_CUDA(cudaMemcpyAsync(w.key, dists, sizeof(float) * (size_t)n, cudaMemcpyDeviceToDevice, st));
     if ((s = launch_fill_empty(st, X, n, d, 1, w.key, w.S, k, nt, w.kk, k, w.active, w.nempty,

@@ -77,3 +77,25 @@ def test_inertia_order(n):
     d = dists.cpu().numpy()
     for p in range(2):
         assert inertia[p].item() == np.add.reduce(d[p])
+
+
+@pytest.mark.parametrize("d", [1, 2, 3, 4, 6, 8, 17, 32])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("f64", [False, True])
+def test_centroid_batches(d, offset, f64):
+    """Centroid sums at cluster sizes around the staging batch (1 to a few
+    thousand members), rows on and off the 16-byte boundary."""
+    import torch
+    import oracle
+    from masters_final_b200.cluster.KMeans import kmeans_centroids
+    rng = np.random.default_rng(d)
+    b = min(256, 1024 // d)
+    sizes = [1, 2, b - 1, b, b + 1, 2 * b, 2 * b + 1, 3 * b + 7, 5000]
+    labels = rng.permutation(np.repeat(np.arange(len(sizes)), sizes)).astype(np.int32)
+    x = (rng.standard_normal((labels.size, d)) * 100).astype(np.float32)
+    buf = torch.empty(x.size + offset, device="cuda")[offset:]
+    buf.copy_(torch.from_numpy(x.reshape(-1)))
+    dist = np.zeros(labels.size, dtype=np.float32)
+    got = kmeans_centroids(buf.view(-1, d), labels, dist, len(sizes),
+                           centroid_mode="f64" if f64 else "numba")
+    assert np.array_equal(got.cpu().numpy(), oracle.kmeans_centroids(x, labels, dist, len(sizes), f64=f64))
