@@ -11,12 +11,11 @@
 // centroids are float32(float64(float32 sequential sum) / count), the
 // inertia is numpy's float32 pairwise sum of the distances and a partition
 // stops early when it changes by at most tol.  The float32 label pass below
-// screens all centroids with an FMA-accumulated float32 distance and keeps
-// the best two; when the runner-up is outside the screening error bound of
-// the winner (|screen - exact| <= (D+3) 2^-23 |exact|), only the winner's
-// exact distance is computed, otherwise the point is re-labelled by the
-// exact reference loop.  The labels are therefore identical to the
-// reference's for any input.
+// screens all centroids and keeps the best two; when the runner-up is outside
+// the screening error bound of the winner only the winner's exact distance
+// is computed, otherwise the point is re-labelled in the reference's
+// arithmetic.  The labels are therefore identical to the reference's for any
+// input.
 //
 // Batching: all P partitions of an ensemble (each with its own k) advance
 // together; every kernel takes the partition from its grid and partitions
@@ -32,111 +31,233 @@
 
 namespace eacb {
 
-constexpr int kLT = 128;         // label threads per block
-constexpr int kLPPT = 2;         // points per thread
-constexpr int kLCH = 128;        // centroids per shared-memory chunk
-
-template <int DM>
-__global__ void __launch_bounds__(kLT)
-k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__restrict__ C,
-            const int32_t *__restrict__ kk, int32_t kmax, const int32_t *__restrict__ active,
-            double ratio, int32_t *__restrict__ labels, float *__restrict__ dists,
-            int32_t *__restrict__ amb, int *__restrict__ namb)
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *dst, const void *src)
 {
-    __shared__ float cs[kLCH * DM];
-    const int p = blockIdx.y;
-    if (!active[p]) return;
-    const int K = kk[p];
-    const float *Cp = C + (int64_t)p * kmax * D;
-    float x[kLPPT][DM];
-    float b1[kLPPT], b2[kLPPT];
-    int i1[kLPPT];
-    int64_t idx[kLPPT];
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES)
+                     : "memory");
+}
+
+// ------------------------------------------------- float32 label pass --
+// The screen works on data centred at its mean, where |x - c|^2 = |x|^2 +
+// 2 (|c|^2 / 2 - x.c): a centroid's score is its half norm less the dot
+// product, one fused multiply-add per dimension in the centroid's row order,
+// two points at a time (fma.rn.f32x2).  A thread holds 2 NP points in
+// registers and reads each centroid row (values doubled for the packed
+// operand, negated, then the half norm) from shared memory as a broadcast.
+// The best two scores and the winner's group of four centroids are kept per
+// point with 12 min/max/select operations per group: three per centroid,
+// where an index per centroid took five.
+//
+// Error: with S = |x|^2 + |c|^2 (centred, u = 2^-24), centring both sides
+// moves the distance by at most 4 u S, the half norm and the chain of D
+// products by (3 D + 1) u S, and the reference's own float32 squares by 6 u S:
+// a screened distance is within e(c) = (3 D + 12) u S of the reference's.  A
+// point whose runner-up is not certainly behind its winner goes to the exact
+// re-check; the winner of every other point is settled inside its group by
+// the direct float32 distances (their error is below e).
+//
+// Bound by the FMA and ALU pipes.  One pass, 500,000 x 16 points, 20
+// partitions of 530: TIMES
+constexpr int kLT = 128;               // label threads per block
+
+template <int DM> struct LabelRow {
+    static constexpr int RF = 2 * DM + 4;                // floats of a staged centroid
+    static constexpr int CH = DM <= 8 ? 128 : 64;        // centroids per staging buffer
+};
+
+__device__ __forceinline__ uint64_t pack2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+    return fminf(fminf(a, b), c);
+}
+
+// staged centroid rows: -c doubled, the half norm doubled; rows past k get
+// an infinite half norm and never win
+template <int DM>
+__global__ void k_prep_label_f32(const float *__restrict__ C, const int32_t *__restrict__ kk,
+                                 int32_t kmax, int32_t kpad, int32_t P, int32_t D,
+                                 const float *__restrict__ mu, const int32_t *__restrict__ active,
+                                 float *__restrict__ rows, float *cmax2)
+{
+    constexpr int RF = LabelRow<DM>::RF;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)P * kpad; e += stride) {
+        const int p = (int)(e / kpad), c = (int)(e % kpad);
+        if (!active[p]) continue;
+        const bool real = c < kk[p];
+        float *row = rows + e * RF;
+        float nrm = 0.f;
 #pragma unroll
-    for (int q = 0; q < kLPPT; ++q) {
-        idx[q] = ((int64_t)blockIdx.x * kLPPT + q) * kLT + threadIdx.x;
-#pragma unroll
-        for (int d = 0; d < DM; ++d) x[q][d] = (idx[q] < n && d < D) ? X[idx[q] * D + d] : 0.f;
-        b1[q] = b2[q] = __int_as_float(0x7f800000);
-        i1[q] = 0;
-    }
-    for (int c0 = 0; c0 < K; c0 += kLCH) {
-        const int cn = min(kLCH, K - c0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < cn * D; e += kLT) {
-            const int c = e / D, d = e - c * D;
-            cs[c * DM + d] = Cp[(int64_t)(c0 + c) * D + d];
+        for (int d = 0; d < DM; ++d) {
+            const float v = real && d < D ? __fsub_rn(C[((int64_t)p * kmax + c) * D + d], mu[d]) : 0.f;
+            nrm = fmaf(v, v, nrm);
+            row[2 * d] = row[2 * d + 1] = -v;
         }
-        __syncthreads();
-        for (int c = 0; c < cn; ++c) {
-            float s[kLPPT];
-#pragma unroll
-            for (int q = 0; q < kLPPT; ++q) s[q] = 0.f;
-#pragma unroll
-            for (int d = 0; d < DM; ++d) {
-                if (d < D) {
-                    const float cv = cs[c * DM + d];
-#pragma unroll
-                    for (int q = 0; q < kLPPT; ++q) {
-                        const float t = x[q][d] - cv;
-                        s[q] = fmaf(t, t, s[q]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < kLPPT; ++q) {
-                if (s[q] < b1[q]) {
-                    b2[q] = b1[q];
-                    b1[q] = s[q];
-                    i1[q] = c0 + c;
-                } else if (s[q] < b2[q]) {
-                    b2[q] = s[q];
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < kLPPT; ++q) {
-        if (idx[q] >= n) continue;
-        const int64_t o = (int64_t)p * n + idx[q];
-        if ((double)b2[q] > (double)b1[q] * ratio) {
-            labels[o] = i1[q];
-            dists[o] = (float)exact_dist<DM>(x[q], Cp + (int64_t)i1[q] * D, D);
-        } else {
-            const int slot = atomicAdd(namb, 1);
-            amb[slot] = (int32_t)o;      // resolved by k_label_exact
-        }
+        row[2 * DM] = row[2 * DM + 1] = real ? 0.5f * nrm : __int_as_float(0x7f800000);
+        // a NaN norm (which no screen may judge) counts only at centroid 0:
+        // there the reference keeps it, elsewhere it never compares as smaller
+        if (real && (nrm == nrm || c == 0))
+            atomicMax(reinterpret_cast<int *>(&cmax2[p]),
+                      nrm == nrm ? __float_as_int(nrm) : 0x7fffffff);
     }
 }
 
-// reference loop for the points the screen could not separate
-__global__ void k_label_exact(const float *__restrict__ X, int32_t n, int32_t D,
-                              const float *__restrict__ C, const int32_t *__restrict__ kk,
-                              int32_t kmax, const int32_t *__restrict__ amb,
-                              const int *__restrict__ namb, int32_t *labels, float *dists)
+template <int DM, int NP>
+__global__ void __launch_bounds__(kLT)
+k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__restrict__ C,
+            const float *__restrict__ rows, const int32_t *__restrict__ kk, int32_t kmax,
+            int32_t kpad, const int32_t *__restrict__ active, const float *__restrict__ mu,
+            const float *__restrict__ cmax2, float E, int32_t *__restrict__ labels,
+            float *__restrict__ dists, int32_t *__restrict__ amb, int *__restrict__ namb)
 {
-    const int m = *namb;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
-        const int64_t o = amb[t];
-        const int64_t p = o / n, i = o - p * n;
-        const int K = kk[p];
-        const float *x = X + i * D;
-        const float *Cp = C + p * kmax * D;
-        double best = 0.0;
-        int bl = 0;
-        for (int k = 0; k < K; ++k) {
-            double dist = 0.0;
-            for (int d = 0; d < D; ++d) {
-                const float diff = __fsub_rn(x[d], Cp[(int64_t)k * D + d]);
-                dist = __dadd_rn(dist, (double)__fmul_rn(diff, diff));
+    constexpr int RF = LabelRow<DM>::RF, CH = LabelRow<DM>::CH, Q = 2 * NP;
+    __shared__ __align__(16) float cs[2][CH * RF];
+    const int p = blockIdx.y;
+    if (!active[p]) return;
+    const int K = kk[p];
+    const float inf = __int_as_float(0x7f800000), cmax = cmax2[p];
+    uint64_t x[DM][NP];
+    float xn[Q], b1[Q], b2[Q];
+    int i1[Q];
+    const int64_t i0 = (int64_t)blockIdx.x * (Q * kLT) + threadIdx.x;    // point q: i0 + q kLT
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        xn[q] = 0.f;
+        b1[q] = b2[q] = inf;
+        i1[q] = 0;
+    }
+#pragma unroll
+    for (int d = 0; d < DM; ++d) {
+        const float m = d < D ? mu[d] : 0.f;
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            float v[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int64_t i = i0 + (2 * j + h) * kLT;
+                v[h] = i < n && d < D ? __fsub_rn(X[i * D + d], m) : 0.f;
+                xn[2 * j + h] = fmaf(v[h], v[h], xn[2 * j + h]);
             }
-            if (k == 0 || dist < best) {
-                best = dist;
-                bl = k;
+            x[d][j] = pack2(v[0], v[1]);
+        }
+    }
+    const float *src = rows + (int64_t)p * kpad * RF;
+    auto stage = [&](int c0, int buf) {          // kpad is a multiple of CH
+        for (int e = threadIdx.x; e < CH * RF / 4; e += kLT)
+            cp_async<16>(&cs[buf][4 * e], src + (int64_t)c0 * RF + 4 * e);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    stage(0, 0);
+    int buf = 0;
+    for (int c0 = 0; c0 < K; c0 += CH, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                         // this buffer is there, the other one is free
+        if (c0 + CH < K) stage(c0 + CH, buf ^ 1);
+        const int g1 = min(CH, K - c0 + 3) >> 2;
+        for (int g = 0; g < g1; ++g) {
+            const float *row = &cs[buf][4 * g * RF];
+            uint64_t acc[4][NP];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const uint64_t h = *reinterpret_cast<const uint64_t *>(row + c * RF + 2 * DM);
+#pragma unroll
+                for (int j = 0; j < NP; ++j) acc[c][j] = h;
+            }
+#pragma unroll
+            for (int d = 0; d < DM; d += 2) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(row + c * RF + 2 * d);
+#pragma unroll
+                    for (int j = 0; j < NP; ++j) acc[c][j] = ffma2(x[d][j], v.x, acc[c][j]);
+#pragma unroll
+                    for (int j = 0; j < NP; ++j) acc[c][j] = ffma2(x[d + 1][j], v.y, acc[c][j]);
+                }
+            }
+            const int id = (c0 >> 2) + g;
+#pragma unroll
+            for (int j = 0; j < NP; ++j) {
+                float s[4][2];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) unpack2(acc[c][j], s[c][0], s[c][1]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int q = 2 * j + h;
+                    const float l0 = fminf(s[0][h], s[1][h]), h0 = fmaxf(s[0][h], s[1][h]);
+                    const float l1 = fminf(s[2][h], s[3][h]), h1 = fmaxf(s[2][h], s[3][h]);
+                    const float m1 = fminf(l0, l1), m2 = min3(fmaxf(l0, l1), h0, h1);
+                    i1[q] = m1 < b1[q] ? id : i1[q];
+                    b2[q] = min3(b2[q], m2, fmaxf(b1[q], m1));
+                    b1[q] = fminf(b1[q], m1);
+                }
             }
         }
-        labels[o] = bl;
-        dists[o] = (float)best;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int64_t i = i0 + q * kLT;
+        if (i >= n) continue;
+        const int64_t o = (int64_t)p * n + i;
+        float xv[DM];
+#pragma unroll
+        for (int d = 0; d < DM; ++d) xv[d] = d < D ? X[i * D + d] : 0.f;
+        // the winner inside its group, by direct float32 distances
+        const float *Cg = C + ((int64_t)p * kmax + 4 * i1[q]) * D;
+        float bd = inf;
+        int bi = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (4 * i1[q] + c < K) {
+                float s = 0.f;
+#pragma unroll
+                for (int d = 0; d < DM; ++d)
+                    if (d < D) {
+                        const float t = __fsub_rn(xv[d], Cg[c * D + d]);
+                        s = fmaf(t, t, s);
+                    }
+                if (s < bd) {
+                    bd = s;
+                    bi = c;
+                }
+            }
+        }
+        const int w = 4 * i1[q] + bi;
+        // Only a centroid within |x| + sqrt(winner's distance and error) of
+        // the origin can be the reference's choice instead of the winner, so
+        // its norm -- and with it its error -- is bounded through the
+        // winner's distance (capped by the partition's largest norm).  The
+        // bound is 1% wide for this arithmetic's rounding, with an absolute
+        // part for products that underflow.
+        const float ncw = 2.f * rows[((int64_t)p * kpad + w) * RF + 2 * DM];
+        const float ew = E * (xn[q] + ncw);
+        const float rc = sqrtf(xn[q]) + sqrtf(fmaxf(0.f, xn[q] + 2.f * b1[q] + ew));
+        const float bound = 1.01f * (ew + E * (xn[q] + fminf(rc * rc, cmax))) + 1e-36f;
+        if (2.f * (b2[q] - b1[q]) > bound && bd < inf && cmax == cmax) {
+            labels[o] = w;
+            dists[o] = (float)exact_dist<DM>(xv, Cg + bi * D, D);
+        } else {
+            amb[atomicAdd(namb, 1)] = (int32_t)o;
+        }
     }
 }
 
@@ -306,17 +427,6 @@ struct CentStage {
     int32_t id[kCentIds][kCentBatch];
 };
 constexpr size_t kCentSmem = kCentWarps * sizeof(CentStage);
-
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void *dst, const void *src)
-{
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    if (BYTES == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES)
-                     : "memory");
-}
 
 // CH: floats per copy (4, 2 or 1: the largest that divides D and that X's
 // alignment allows)
@@ -775,35 +885,57 @@ struct KMWS {
     }
 };
 
-template <int DM>
-static void launch_label(dim3 grid, cudaStream_t st, const float *X, int32_t n, int32_t D,
-                         const float *C, const int32_t *kk, int32_t kmax, const int32_t *active,
-                         double ratio, int32_t *labels, float *dists, int32_t *amb, int *namb)
+template <int DM, int NP>
+static int launch_label(cudaStream_t st, const float *X, int32_t n, int32_t D, int32_t P,
+                        const float *C, const int32_t *kk, int32_t kmax, const int32_t *active,
+                        int32_t *labels, float *dists, int32_t *amb, int *namb, const TcScratch &s)
 {
-    k_label_f32<DM><<<grid, kLT, 0, st>>>(X, n, D, C, kk, kmax, active, ratio, labels, dists, amb,
-                                          namb);
+    static_assert(kTcCentPad % LabelRow<DM>::CH == 0, "whole staging buffers of rows");
+    const int32_t kpad = (int32_t)s.kt_max * kTcCentPad;
+    if (LabelRow<DM>::RF * sizeof(float) > (size_t)2 * s.Kp) return EACB_ERR_INTERNAL;
+    float *rows = reinterpret_cast<float *>(s.B);
+    k_prep_label_f32<DM><<<grid_for((int64_t)P * kpad, 128), 128, 0, st>>>(
+        C, kk, kmax, kpad, P, D, s.mu, active, rows, s.cmax2);
+    EACB_CHECK_LAUNCH();
+    const float E = (float)((3 * D + 12) * ldexp(1.0, -24));
+    const dim3 grid((unsigned)((n + 2 * NP * kLT - 1) / (2 * NP * kLT)), (unsigned)P);
+    ProfScope ps(PROF_KMEANS, st);
+    k_label_f32<DM, NP><<<grid, kLT, 0, st>>>(X, n, D, C, rows, kk, kmax, kpad, active, s.mu, s.cmax2,
+                                              E, labels, dists, amb, namb);
+    EACB_CHECK_LAUNCH();
+    ps.done(0.0);
+    return EACB_OK;
 }
 
 int label_pass_f32(const float *X, int32_t n, int32_t D, int32_t P, const float *C,
                    const int32_t *kk, int32_t kmax, const int32_t *active, int32_t *labels,
-                   float *dists, int32_t *amb, int *namb, cudaStream_t st)
+                   float *dists, int32_t *amb, int *namb, TcScratch &s, cudaStream_t st)
 {
-    // |screen - exact| <= (D + 3) 2^-23 exact, so the winner is certain when
-    // the runner-up's screened distance exceeds ratio * the winner's
-    const double eps = (double)(D + 3) * ldexp(1.0, -23);
-    const double ratio = (1.0 + eps) / (1.0 - eps);
+    int r = data_mean(X, n, D, s, st);
+    if (r) return r;
+    EACB_CUDA(cudaMemsetAsync(s.cmax2, 0, sizeof(float) * P, st));
     EACB_CUDA(cudaMemsetAsync(namb, 0, sizeof(int), st));
-    dim3 grid((unsigned)((n + kLT * kLPPT - 1) / (kLT * kLPPT)), (unsigned)P);
-    ProfScope ps(PROF_KMEANS, st);
-    if (D <= 4) launch_label<4>(grid, st, X, n, D, C, kk, kmax, active, ratio, labels, dists, amb, namb);
-    else if (D <= 8) launch_label<8>(grid, st, X, n, D, C, kk, kmax, active, ratio, labels, dists, amb, namb);
-    else if (D <= 16) launch_label<16>(grid, st, X, n, D, C, kk, kmax, active, ratio, labels, dists, amb, namb);
-    else launch_label<32>(grid, st, X, n, D, C, kk, kmax, active, ratio, labels, dists, amb, namb);
-    EACB_CHECK_LAUNCH();
-    ps.done(0.0);
-    k_label_exact<<<148 * 4, 128, 0, st>>>(X, n, D, C, kk, kmax, amb, namb, labels, dists);
-    EACB_CHECK_LAUNCH();
-    return EACB_OK;
+    // more points per thread (fewer reads of the staged rows per distance)
+    // while that leaves every SM four blocks
+    auto many = [&](int np) {
+        return ((int64_t)n + 2 * np * kLT - 1) / (2 * np * kLT) * P >= 148 * 4;
+    };
+#define EACB_LABEL(DM, NPW)                                                                    \
+    (many(NPW) ? launch_label<DM, NPW>(st, X, n, D, P, C, kk, kmax, active, labels, dists, amb, \
+                                       namb, s)                                                \
+               : launch_label<DM, 1>(st, X, n, D, P, C, kk, kmax, active, labels, dists, amb,  \
+                                     namb, s))
+    if (D <= 2) r = EACB_LABEL(2, 4);
+    else if (D <= 4) r = EACB_LABEL(4, 4);
+    else if (D <= 6) r = EACB_LABEL(6, 2);
+    else if (D <= 8) r = EACB_LABEL(8, 2);
+    else if (D <= 12) r = EACB_LABEL(12, 2);
+    else if (D <= 16) r = EACB_LABEL(16, 2);
+    else if (D <= 24) r = EACB_LABEL(24, 1);
+    else r = EACB_LABEL(32, 1);
+#undef EACB_LABEL
+    if (r) return r;
+    return label_exact_points(X, n, D, P, C, kk, kmax, labels, dists, amb, namb, nullptr, st);
 }
 
 }  // namespace eacb
@@ -848,7 +980,7 @@ extern "C" int eacb_kmeans_ensemble(const float *X, int32_t n, int32_t d, int32_
                               w.namb, w.tc, st);
         else
             s = label_pass_f32(X, n, d, P, centroids, k, kmax, w.active, labels, w.dists, w.amb,
-                               w.namb, st);
+                               w.namb, w.tc, st);
         if (s) return s;
         // the member scratch is free here: at most n / 32 node sums per partition
         if ((s = launch_inertia(st, w.dists, n, P, (float *)w.args, w.active, w.inertia, w.iters,
@@ -914,7 +1046,7 @@ extern "C" int eacb_kmeans_label(const float *X, int32_t n, int32_t d, const flo
     EACB_CHECK_LAUNCH();
     if (label_mode == 1)
         return label_pass_tc(X, n, d, 1, C, kk, k, active, labels, dists, amb, namb, tc, st);
-    return label_pass_f32(X, n, d, 1, C, kk, k, active, labels, dists, amb, namb, st);
+    return label_pass_f32(X, n, d, 1, C, kk, k, active, labels, dists, amb, namb, tc, st);
 }
 
 extern "C" size_t eacb_kmeans_label_workspace_size(int32_t n, int32_t d, int32_t k)

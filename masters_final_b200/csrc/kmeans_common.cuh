@@ -26,20 +26,24 @@ static __global__ void k_set2(int32_t *a, int32_t *b, int32_t va, int32_t vb)
     *b = vb;
 }
 
-// Scratch of the tensor-core label pass: operands in the UMMA layout.
+// Scratch of the label passes.  Tensor cores: operands in the UMMA layout.
+// Float32: B holds the staged centroid rows (a row's 8 D + 16 bytes, D
+// rounded up to the kernel's, fit the 2 Kp >= 12 D of a tile row).
+constexpr int kTcCentPad = 128;      // centroid rows are padded to tiles of this many
 struct TcScratch {
-    int Kp;              // 3d rounded up to a multiple of 16
+    int Kp;              // 6d rounded up to a multiple of 16
     int64_t n_pad;       // points rounded up to the 128-point tile
-    int kt_max;          // 256-centroid tiles per partition
-    uint8_t *A;          // point tiles (BF16 [hi, hi, lo])
+    int kt_max;          // kTcCentPad-centroid tiles per partition
+    uint8_t *A;          // point tiles
     float *nx;           // |x - mu|^2
-    uint8_t *B;          // centroid tiles (BF16 [hi, lo, hi])
+    uint8_t *B;          // centroid tiles
     float *nc;           // |c - mu|^2 (+inf for padding)
     float *cmax2;        // per partition max |c - mu|^2
     float *mu;           // data mean
     double *part;        // column-sum partials
     int *err;
-    bool points_ready;   // A / nx / mu depend on X only
+    bool points_ready;   // A / nx depend on X only
+    bool mean_ready;     // and so do part / mu
     static TcScratch carve(Carver &c, int32_t n, int32_t D, int32_t P, int32_t kmax);
 };
 
@@ -49,5 +53,16 @@ struct TcScratch {
 int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *C,
                   const int32_t *kk, int32_t kmax, const int32_t *active, int32_t *labels,
                   float *dists, int32_t *amb, int *namb, TcScratch &s, cudaStream_t st);
+
+// About the data's mean (of a strided sample), once per scratch: the label
+// passes centre on it, which keeps their error bounds small; their results
+// do not depend on it.
+int data_mean(const float *X, int32_t n, int32_t D, TcScratch &s, cudaStream_t st);
+
+// The reference's label and distance for the *namb listed (partition, point)
+// pairs; err (may be null): nonzero means they are done already.
+int label_exact_points(const float *X, int32_t n, int32_t D, int32_t P, const float *C,
+                       const int32_t *kk, int32_t kmax, int32_t *labels, float *dists,
+                       const int32_t *amb, const int *namb, const int *err, cudaStream_t st);
 
 }  // namespace eacb

@@ -30,7 +30,7 @@
 namespace eacb {
 
 constexpr int kTM = 128;           // points per CTA tile
-constexpr int kTN = 128;           // centroids per MMA tile
+constexpr int kTN = kTcCentPad;    // centroids per MMA tile
 constexpr int kTThreads = 256;     // 8 warps: 4 TMEM lane quarters x 2 column halves
 constexpr int kTColGroups = kTThreads / kTM;
 constexpr int kTColsPer = kTN / kTColGroups;
@@ -153,31 +153,54 @@ __host__ __device__ __forceinline__ uint32_t core_off(int row, int k, int Kp)
 }
 
 // ------------------------------------------------------------ preparation --
-// data mean, float64 partials per block then a fixed-order final sum
-__global__ void k_colsum(const float *X, int32_t n, int32_t D, double *part)
+// Mean of at most kMeanRows rows, evenly spread: float64 partials per block
+// (one thread per dimension and row lane, consecutive addresses), then a
+// fixed-order final sum.  Reading all of 2,000,000 x 8 took 383 us.
+constexpr int kMeanRows = 65536;
+constexpr int kMeanBlocks = 296;
+__global__ void __launch_bounds__(256)
+k_colsum(const float *X, int32_t n, int32_t D, int32_t m, double *part)
 {
-    __shared__ double s[32][33];
-    const int d = threadIdx.x & 31, r = threadIdx.x >> 5;   // 256 threads: 8 row lanes
+    __shared__ double s[256];
+    const int per = 256 / D;                           // row lanes
+    const int d = threadIdx.x % D, r = threadIdx.x / D;
     double acc = 0.0;
-    if (d < D)
-        for (int64_t i = (int64_t)blockIdx.x * 8 + r; i < n; i += (int64_t)gridDim.x * 8)
-            acc += (double)X[i * D + d];
-    s[r][d] = acc;
+    if (r < per)
+        for (int64_t j = (int64_t)blockIdx.x * per + r; j < m; j += (int64_t)gridDim.x * per)
+            acc += (double)X[j * n / m * D + d];
+    s[threadIdx.x] = acc;
     __syncthreads();
-    if (r == 0 && d < D) {
+    if (r == 0) {
         double t = 0.0;
-        for (int q = 0; q < 8; ++q) t += s[q][d];
+        for (int q = 0; q < per; ++q) t += s[q * D + d];
         part[(int64_t)blockIdx.x * 32 + d] = t;
     }
 }
 
-__global__ void k_mean(const double *part, int nblocks, int32_t n, int32_t D, float *mu)
+// (a sum that is not finite centres on 0 instead, so that finite points keep
+// finite scores)
+__global__ void k_mean(const double *part, int nblocks, int32_t m, int32_t D, float *mu)
 {
-    const int d = threadIdx.x;
+    const int lane = threadIdx.x & 31, d = threadIdx.x >> 5;
     if (d >= D) return;
     double t = 0.0;
-    for (int b = 0; b < nblocks; ++b) t += part[(int64_t)b * 32 + d];
-    mu[d] = (float)(t / (double)n);
+    for (int b = lane; b < nblocks; b += 32) t += part[(int64_t)b * 32 + d];
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    const float v = (float)(t / (double)m);
+    if (lane == 0) mu[d] = fabsf(v) <= 3.4e38f ? v : 0.f;
+}
+
+int data_mean(const float *X, int32_t n, int32_t D, TcScratch &s, cudaStream_t st)
+{
+    if (s.mean_ready) return EACB_OK;
+    const int32_t m = std::min(n, kMeanRows);
+    k_colsum<<<kMeanBlocks, 256, 0, st>>>(X, n, D, m, s.part);
+    EACB_CHECK_LAUNCH();
+    k_mean<<<1, 1024, 0, st>>>(s.part, kMeanBlocks, m, D, s.mu);
+    EACB_CHECK_LAUNCH();
+    s.mean_ready = true;
+    return EACB_OK;
 }
 
 // Rows of one operand, centred and split into three BF16 parts
@@ -586,7 +609,7 @@ k_label_exact_tc(const float *__restrict__ X, int32_t n, int32_t D, const float 
                  const int *__restrict__ err, int32_t *labels, float *dists)
 {
     extern __shared__ float s_sum[];
-    if (*err != 0) return;                      // k_exact_all did every point
+    if (err && *err != 0) return;               // k_exact_all did every point
     const int64_t cap = (int64_t)P * n;
     const int m = (int)min((int64_t)*namb, cap);
     const float grow = 1.f + 4.f * (float)(D + 2) * 5.9604645e-8f;     // 2^-24
@@ -612,7 +635,7 @@ k_label_exact_tc(const float *__restrict__ X, int32_t n, int32_t D, const float 
         for (int off = 16; off >= 1; off >>= 1) mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, off));
         const float thr = __fadd_ru(__fmul_ru(mn, grow), 1e-38f);
         double best = 0.0;
-        int bl = 0x7fffffff;
+        int bl = 0x7fffffff, nan0 = 0;
         for (int k = lane; k < K; k += 32) {
             float d32;
             if (cached) {
@@ -624,6 +647,12 @@ k_label_exact_tc(const float *__restrict__ X, int32_t n, int32_t D, const float 
             if (d32 > thr) continue;
             load_row<DM, VEC>(Cp + (int64_t)k * D, D, cv);
             const double dist = exact_dist_reg<DM>(xv, cv, D);
+            // a NaN never compares as smaller, so the reference keeps one
+            // only from centroid 0, and then to the end
+            if (dist != dist) {
+                if (k == 0) nan0 = 1;
+                continue;
+            }
             if (bl == 0x7fffffff || dist < best) {
                 best = dist;
                 bl = k;
@@ -633,14 +662,14 @@ k_label_exact_tc(const float *__restrict__ X, int32_t n, int32_t D, const float 
         for (int off = 16; off >= 1; off >>= 1) {
             const double ob = __shfl_xor_sync(0xffffffffu, best, off);
             const int ok = __shfl_xor_sync(0xffffffffu, bl, off);
-            if (ok != 0x7fffffff && (bl == 0x7fffffff || ob < best || (!(best < ob) && ok < bl))) {
+            if (ok != 0x7fffffff && (bl == 0x7fffffff || ob < best || (ob == best && ok < bl))) {
                 best = ob;
                 bl = ok;
             }
         }
         if (lane == 0) {
-            labels[o] = bl;
-            dists[o] = (float)best;
+            labels[o] = nan0 ? 0 : bl;
+            dists[o] = nan0 ? __int_as_float(0x7fffffff) : (float)best;
         }
         __syncwarp();                           // the sums are rewritten by the next point
     }
@@ -665,10 +694,39 @@ TcScratch TcScratch::carve(Carver &c, int32_t n, int32_t D, int32_t P, int32_t k
     s.nc = c.take<float>((size_t)P * s.kt_max * kTN);
     s.cmax2 = c.take<float>((size_t)P);
     s.mu = c.take<float>(32);
-    s.part = c.take<double>((size_t)32 * 296);
+    s.part = c.take<double>((size_t)32 * kMeanBlocks);
     s.err = c.take<int>(1);
-    s.points_ready = false;
+    s.points_ready = s.mean_ready = false;
     return s;
+}
+
+int label_exact_points(const float *X, int32_t n, int32_t D, int32_t P, const float *C,
+                       const int32_t *kk, int32_t kmax, int32_t *labels, float *dists,
+                       const int32_t *amb, const int *namb, const int *err, cudaStream_t st)
+{
+    const size_t esmem = kmax <= kExactCacheK
+                             ? (size_t)(kExactThreads / 32) * kmax * sizeof(float) : 0;
+    int es = EACB_OK;
+    auto exact = [&](auto kern) {
+        if (esmem > 48 * 1024 && allow_max_dyn_smem(kern) != cudaSuccess)
+            es = EACB_ERR_CUDA;
+        else
+            kern<<<148 * 8, kExactThreads, esmem, st>>>(X, n, D, C, kk, kmax, P, amb, namb, err,
+                                                        labels, dists);
+    };
+    // 16-byte row loads when every row is exactly DM floats on a 16-byte boundary
+    const bool al = ((uintptr_t)X % 16 == 0) && ((uintptr_t)C % 16 == 0);
+    if (D == 4 && al) exact(k_label_exact_tc<4, true>);
+    else if (D <= 4) exact(k_label_exact_tc<4, false>);
+    else if (D == 8 && al) exact(k_label_exact_tc<8, true>);
+    else if (D <= 8) exact(k_label_exact_tc<8, false>);
+    else if (D == 16 && al) exact(k_label_exact_tc<16, true>);
+    else if (D <= 16) exact(k_label_exact_tc<16, false>);
+    else if (D == 32 && al) exact(k_label_exact_tc<32, true>);
+    else exact(k_label_exact_tc<32, false>);
+    if (es) return es;
+    EACB_CHECK_LAUNCH();
+    return EACB_OK;
 }
 
 int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *C,
@@ -676,10 +734,8 @@ int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *
                   float *dists, int32_t *amb, int *namb, TcScratch &s, cudaStream_t st)
 {
     if (!s.points_ready) {
-        k_colsum<<<296, 256, 0, st>>>(X, n, D, s.part);
-        EACB_CHECK_LAUNCH();
-        k_mean<<<1, 32, 0, st>>>(s.part, 296, n, D, s.mu);
-        EACB_CHECK_LAUNCH();
+        int r = data_mean(X, n, D, s, st);
+        if (r) return r;
         k_prep_points<<<grid_for(s.n_pad, 128), 128, 0, st>>>(X, n, D, s.Kp, s.mu, s.A, s.nx,
                                                               s.n_pad);
         EACB_CHECK_LAUNCH();
@@ -730,29 +786,7 @@ int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *
     ps.done(0.0);
     k_exact_all<<<296, 256, 0, st>>>(X, n, D, C, kk, kmax, P, active, s.err, labels, dists);
     EACB_CHECK_LAUNCH();
-    const size_t esmem = kmax <= kExactCacheK
-                             ? (size_t)(kExactThreads / 32) * kmax * sizeof(float) : 0;
-    int es = EACB_OK;
-    auto exact = [&](auto kern) {
-        if (esmem > 48 * 1024 && allow_max_dyn_smem(kern) != cudaSuccess)
-            es = EACB_ERR_CUDA;
-        else
-            kern<<<148 * 8, kExactThreads, esmem, st>>>(X, n, D, C, kk, kmax, P, amb, namb, s.err,
-                                                        labels, dists);
-    };
-    // 16-byte row loads when every row is exactly DM floats on a 16-byte boundary
-    const bool al = ((uintptr_t)X % 16 == 0) && ((uintptr_t)C % 16 == 0);
-    if (D == 4 && al) exact(k_label_exact_tc<4, true>);
-    else if (D <= 4) exact(k_label_exact_tc<4, false>);
-    else if (D == 8 && al) exact(k_label_exact_tc<8, true>);
-    else if (D <= 8) exact(k_label_exact_tc<8, false>);
-    else if (D == 16 && al) exact(k_label_exact_tc<16, true>);
-    else if (D <= 16) exact(k_label_exact_tc<16, false>);
-    else if (D == 32 && al) exact(k_label_exact_tc<32, true>);
-    else exact(k_label_exact_tc<32, false>);
-    if (es) return es;
-    EACB_CHECK_LAUNCH();
-    return EACB_OK;
+    return label_exact_points(X, n, D, P, C, kk, kmax, labels, dists, amb, namb, s.err, st);
 }
 
 }  // namespace eacb

@@ -99,3 +99,49 @@ def test_centroid_batches(d, offset, f64):
     got = kmeans_centroids(buf.view(-1, d), labels, dist, len(sizes),
                            centroid_mode="f64" if f64 else "numba")
     assert np.array_equal(got.cpu().numpy(), oracle.kmeans_centroids(x, labels, dist, len(sizes), f64=f64))
+
+
+@pytest.mark.parametrize("d", [1, 2, 3, 5, 7, 9, 13, 16, 17, 25, 32])
+@pytest.mark.parametrize("k", [1, 3, 5, 127, 130, 515])
+def test_label_f32_shapes(d, k):
+    """The float32 label pass against the reference's loop: every padded
+    dimension, ragged groups of four centroids and staging buffers, both
+    points-per-thread variants, a far-off mean, ties, points on centroids."""
+    import oracle
+    from masters_final_b200.cluster.KMeans import kmeans_label
+    rng = np.random.default_rng(100 * d + k)
+    for n in (700, 310_003 if k == 130 and d in (2, 8, 16) else 3001):
+        x = (rng.standard_normal((n, d)) + 300.0 * rng.standard_normal(d)).astype(np.float32)
+        c = x[rng.choice(n, k, replace=False)].copy()
+        if k > 2:
+            c[k - 1] = c[0]                       # exact tie between distant ids
+        x[:40] = c[rng.integers(0, k, 40)]
+        lab, dist = kmeans_label(x, c, label_mode="cuda")
+        want = oracle.kmeans_label(x, c)
+        assert np.array_equal(lab.cpu().numpy(), want[0])
+        assert np.array_equal(dist.cpu().numpy(), want[1])
+
+
+@pytest.mark.parametrize("bad", [None, 0, 1, 2, 6])
+def test_label_f32_special_values(bad):
+    """Infinities, NaN points, huge and tiny values, and a NaN centroid: the
+    reference never takes a NaN distance except from centroid 0."""
+    import oracle
+    from masters_final_b200.cluster.KMeans import kmeans_label
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((4000, 3)).astype(np.float32)
+    c = x[:7].copy()
+    x[100:110] *= np.float32(1e25)
+    x[110:140] *= np.float32(1e-30)
+    x[200, 1] = np.inf
+    x[201, 0] = -np.inf
+    x[202] = np.nan
+    c[4] = 0
+    if bad is not None:
+        c[bad, 1] = np.nan
+        c[(bad + 3) % 7, 0] = np.inf
+    with np.errstate(all="ignore"):
+        want = oracle.kmeans_label(x, c)
+    lab, dist = kmeans_label(x, c, label_mode="cuda")
+    assert np.array_equal(lab.cpu().numpy(), want[0])
+    assert np.array_equal(dist.cpu().numpy(), want[1], equal_nan=True)
