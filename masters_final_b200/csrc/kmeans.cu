@@ -47,8 +47,8 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src)
 // 2 (|c|^2 / 2 - x.c): a centroid's score is its half norm less the dot
 // product, one fused multiply-add per dimension in the centroid's row order,
 // two points at a time (fma.rn.f32x2).  A thread holds 2 NP points in
-// registers and reads each centroid row (values doubled for the packed
-// operand, negated, then the half norm) from shared memory as a broadcast.
+// registers and reads each centroid row (the half norm, then the values
+// negated) from shared memory as a broadcast, a vector ahead of its use.
 // The best two scores and the winner's group of four centroids are kept per
 // point with 12 min/max/select operations per group: three per centroid,
 // where an index per centroid took five.
@@ -58,16 +58,20 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src)
 // products by (3 D + 1) u S, and the reference's own float32 squares by 6 u S:
 // a screened distance is within e(c) = (3 D + 12) u S of the reference's.  A
 // point whose runner-up is not certainly behind its winner goes to the exact
-// re-check; the winner of every other point is settled inside its group by
-// the direct float32 distances (their error is below e).
+// re-check.
 //
-// Bound by the FMA and ALU pipes.  One pass, 500,000 x 16 points, 20
-// partitions of 530: TIMES
+// Bound by the FMA pipe (half of its cycles) and the shared-memory reads.
+// One pass: 500,000 x 16 points, 20 partitions of 530: 20.5 ms with a
+// subtract and a multiply-add per dimension and an index per centroid; 6.4
+// with scalar row loads and re-reads of the winner's group at the end (a
+// lane per row: D loads of 32 sectors each); 3.7 with vector loads.  32
+// dimensions, 10 partitions: 6.3 -> 4.0.  1,000,000 x 2, k 1,024: 0.90 ->
+// 0.25 ms.
 constexpr int kLT = 128;               // label threads per block
 
 template <int DM> struct LabelRow {
-    static constexpr int RF = 2 * DM + 4;                // floats of a staged centroid
-    static constexpr int CH = DM <= 8 ? 128 : 64;        // centroids per staging buffer
+    static constexpr int RF = (DM + 4) & ~3;             // floats of a staged centroid
+    static constexpr int CH = 128;                       // centroids per staging buffer
 };
 
 __device__ __forceinline__ uint64_t pack2(float a, float b)
@@ -80,6 +84,7 @@ __device__ __forceinline__ void unpack2(uint64_t v, float &a, float &b)
 {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
+__device__ __forceinline__ uint64_t twice(float a) { return pack2(a, a); }
 __device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c)
 {
     uint64_t d;
@@ -91,8 +96,8 @@ __device__ __forceinline__ float min3(float a, float b, float c)
     return fminf(fminf(a, b), c);
 }
 
-// staged centroid rows: -c doubled, the half norm doubled; rows past k get
-// an infinite half norm and never win
+// staged centroid rows: the half norm, then -c; rows past k get an infinite
+// half norm and never win
 template <int DM>
 __global__ void k_prep_label_f32(const float *__restrict__ C, const int32_t *__restrict__ kk,
                                  int32_t kmax, int32_t kpad, int32_t P, int32_t D,
@@ -111,9 +116,9 @@ __global__ void k_prep_label_f32(const float *__restrict__ C, const int32_t *__r
         for (int d = 0; d < DM; ++d) {
             const float v = real && d < D ? __fsub_rn(C[((int64_t)p * kmax + c) * D + d], mu[d]) : 0.f;
             nrm = fmaf(v, v, nrm);
-            row[2 * d] = row[2 * d + 1] = -v;
+            row[1 + d] = -v;
         }
-        row[2 * DM] = row[2 * DM + 1] = real ? 0.5f * nrm : __int_as_float(0x7f800000);
+        row[0] = real ? 0.5f * nrm : __int_as_float(0x7f800000);
         // a NaN norm (which no screen may judge) counts only at centroid 0:
         // there the reference keeps it, elsewhere it never compares as smaller
         if (real && (nrm == nrm || c == 0))
@@ -122,8 +127,9 @@ __global__ void k_prep_label_f32(const float *__restrict__ C, const int32_t *__r
     }
 }
 
-template <int DM, int NP>
-__global__ void __launch_bounds__(kLT)
+// VEC: D equals DM and the rows of X and C can be read as vectors
+template <int DM, int NP, bool VEC>
+__global__ void __launch_bounds__(kLT, 4)
 k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__restrict__ C,
             const float *__restrict__ rows, const int32_t *__restrict__ kk, int32_t kmax,
             int32_t kpad, const int32_t *__restrict__ active, const float *__restrict__ mu,
@@ -131,7 +137,7 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
             float *__restrict__ dists, int32_t *__restrict__ amb, int *__restrict__ namb)
 {
     constexpr int RF = LabelRow<DM>::RF, CH = LabelRow<DM>::CH, Q = 2 * NP;
-    __shared__ __align__(16) float cs[2][CH * RF];
+    __shared__ __align__(16) float cs[2][(CH + 4) * RF];
     const int p = blockIdx.y;
     if (!active[p]) return;
     const int K = kk[p];
@@ -147,18 +153,23 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
         i1[q] = 0;
     }
 #pragma unroll
-    for (int d = 0; d < DM; ++d) {
-        const float m = d < D ? mu[d] : 0.f;
+    for (int j = 0; j < NP; ++j) {
+        float v[2][DM];
 #pragma unroll
-        for (int j = 0; j < NP; ++j) {
-            float v[2];
+        for (int h = 0; h < 2; ++h) {
+            // past the last point: its row again, never written
+            const int64_t i = min((int64_t)n - 1, i0 + (2 * j + h) * kLT);
+            load_row<DM, VEC>(X + i * D, D, v[h]);
+        }
+#pragma unroll
+        for (int d = 0; d < DM; ++d) {
+            const float m = VEC || d < D ? mu[d] : 0.f;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int64_t i = i0 + (2 * j + h) * kLT;
-                v[h] = i < n && d < D ? __fsub_rn(X[i * D + d], m) : 0.f;
-                xn[2 * j + h] = fmaf(v[h], v[h], xn[2 * j + h]);
+                v[h][d] = __fsub_rn(v[h][d], m);
+                xn[2 * j + h] = fmaf(v[h][d], v[h][d], xn[2 * j + h]);
             }
-            x[d][j] = pack2(v[0], v[1]);
+            x[d][j] = pack2(v[0][d], v[1][d]);
         }
     }
     const float *src = rows + (int64_t)p * kpad * RF;
@@ -174,25 +185,36 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
         __syncthreads();                         // this buffer is there, the other one is free
         if (c0 + CH < K) stage(c0 + CH, buf ^ 1);
         const int g1 = min(CH, K - c0 + 3) >> 2;
-        for (int g = 0; g < g1; ++g) {
-            const float *row = &cs[buf][4 * g * RF];
+        // the four rows' next 16-byte vectors are read while the current ones
+        // are used (past the last group they are read and dropped)
+        const float *row = cs[buf];
+        float4 f[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) f[c] = *reinterpret_cast<const float4 *>(row + c * RF);
+        for (int g = 0; g < g1; ++g, row += 4 * RF) {
             uint64_t acc[4][NP];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const uint64_t h = *reinterpret_cast<const uint64_t *>(row + c * RF + 2 * DM);
+            for (int v = 0; v < RF / 4; ++v) {
+                float4 nx[4];
 #pragma unroll
-                for (int j = 0; j < NP; ++j) acc[c][j] = h;
-            }
+                for (int c = 0; c < 4; ++c)
+                    nx[c] = *reinterpret_cast<const float4 *>(
+                        row + (4 * v + 4 < RF ? c * RF + 4 * v + 4 : (4 + c) * RF));
 #pragma unroll
-            for (int d = 0; d < DM; d += 2) {
+                for (int k = 0; k < 4; ++k) {
+                    const int d = 4 * v + k - 1;
+                    if (d >= DM) continue;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(row + c * RF + 2 * d);
+                    for (int c = 0; c < 4; ++c) {
+                        const float e = k == 0 ? f[c].x : k == 1 ? f[c].y : k == 2 ? f[c].z : f[c].w;
+                        const uint64_t w = twice(e);
 #pragma unroll
-                    for (int j = 0; j < NP; ++j) acc[c][j] = ffma2(x[d][j], v.x, acc[c][j]);
-#pragma unroll
-                    for (int j = 0; j < NP; ++j) acc[c][j] = ffma2(x[d + 1][j], v.y, acc[c][j]);
+                        for (int j = 0; j < NP; ++j)
+                            acc[c][j] = d < 0 ? w : ffma2(x[d < 0 ? 0 : d][j], w, acc[c][j]);
+                    }
                 }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) f[c] = nx[c];
             }
             const int id = (c0 >> 2) + g;
 #pragma unroll
@@ -218,27 +240,24 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
         const int64_t i = i0 + q * kLT;
         if (i >= n) continue;
         const int64_t o = (int64_t)p * n + i;
-        float xv[DM];
+        // the winner inside its group: the one with the same score again
+        const float *rg = rows + ((int64_t)p * kpad + 4 * i1[q]) * RF;
+        int bi = -1;
+        float ncw = 0.f;
 #pragma unroll
-        for (int d = 0; d < DM; ++d) xv[d] = d < D ? X[i * D + d] : 0.f;
-        // the winner inside its group, by direct float32 distances
-        const float *Cg = C + ((int64_t)p * kmax + 4 * i1[q]) * D;
-        float bd = inf;
-        int bi = 0;
+        for (int c = 3; c >= 0; --c) {
+            float e[RF];
+            load_row<RF, true>(rg + c * RF, RF, e);
+            float s = e[0];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (4 * i1[q] + c < K) {
-                float s = 0.f;
-#pragma unroll
-                for (int d = 0; d < DM; ++d)
-                    if (d < D) {
-                        const float t = __fsub_rn(xv[d], Cg[c * D + d]);
-                        s = fmaf(t, t, s);
-                    }
-                if (s < bd) {
-                    bd = s;
-                    bi = c;
-                }
+            for (int d = 0; d < DM; ++d) {
+                float v[2];
+                unpack2(x[d][q / 2], v[0], v[1]);
+                s = fmaf(v[q & 1], e[1 + d], s);
+            }
+            if (s == b1[q]) {
+                bi = c;
+                ncw = 2.f * e[0];
             }
         }
         const int w = 4 * i1[q] + bi;
@@ -248,13 +267,15 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
         // winner's distance (capped by the partition's largest norm).  The
         // bound is 1% wide for this arithmetic's rounding, with an absolute
         // part for products that underflow.
-        const float ncw = 2.f * rows[((int64_t)p * kpad + w) * RF + 2 * DM];
         const float ew = E * (xn[q] + ncw);
         const float rc = sqrtf(xn[q]) + sqrtf(fmaxf(0.f, xn[q] + 2.f * b1[q] + ew));
         const float bound = 1.01f * (ew + E * (xn[q] + fminf(rc * rc, cmax))) + 1e-36f;
-        if (2.f * (b2[q] - b1[q]) > bound && bd < inf && cmax == cmax) {
+        if (2.f * (b2[q] - b1[q]) > bound && bi >= 0 && b1[q] < inf && cmax == cmax) {
+            float xv[DM], cv[DM];
+            load_row<DM, VEC>(X + i * D, D, xv);
+            load_row<DM, VEC>(C + ((int64_t)p * kmax + w) * D, D, cv);
             labels[o] = w;
-            dists[o] = (float)exact_dist<DM>(xv, Cg + bi * D, D);
+            dists[o] = (float)exact_dist<DM>(xv, cv, D);
         } else {
             amb[atomicAdd(namb, 1)] = (int32_t)o;
         }
@@ -900,8 +921,14 @@ static int launch_label(cudaStream_t st, const float *X, int32_t n, int32_t D, i
     const float E = (float)((3 * D + 12) * ldexp(1.0, -24));
     const dim3 grid((unsigned)((n + 2 * NP * kLT - 1) / (2 * NP * kLT)), (unsigned)P);
     ProfScope ps(PROF_KMEANS, st);
-    k_label_f32<DM, NP><<<grid, kLT, 0, st>>>(X, n, D, C, rows, kk, kmax, kpad, active, s.mu, s.cmax2,
-                                              E, labels, dists, amb, namb);
+    // rows as vectors where their length and place allow it
+    const uintptr_t at = (uintptr_t)X | (uintptr_t)C;
+    if (D == DM && at % (DM % 4 == 0 ? 16 : 8) == 0)
+        k_label_f32<DM, NP, true><<<grid, kLT, 0, st>>>(X, n, D, C, rows, kk, kmax, kpad, active,
+                                                        s.mu, s.cmax2, E, labels, dists, amb, namb);
+    else
+        k_label_f32<DM, NP, false><<<grid, kLT, 0, st>>>(X, n, D, C, rows, kk, kmax, kpad, active,
+                                                         s.mu, s.cmax2, E, labels, dists, amb, namb);
     EACB_CHECK_LAUNCH();
     ps.done(0.0);
     return EACB_OK;
@@ -927,8 +954,8 @@ int label_pass_f32(const float *X, int32_t n, int32_t D, int32_t P, const float 
                                      namb, s))
     if (D <= 2) r = EACB_LABEL(2, 4);
     else if (D <= 4) r = EACB_LABEL(4, 4);
-    else if (D <= 6) r = EACB_LABEL(6, 2);
-    else if (D <= 8) r = EACB_LABEL(8, 2);
+    else if (D <= 6) r = EACB_LABEL(6, 4);
+    else if (D <= 8) r = EACB_LABEL(8, 4);
     else if (D <= 12) r = EACB_LABEL(12, 2);
     else if (D <= 16) r = EACB_LABEL(16, 2);
     else if (D <= 24) r = EACB_LABEL(24, 1);

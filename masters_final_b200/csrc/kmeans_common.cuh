@@ -20,6 +20,34 @@ __device__ __forceinline__ double exact_dist(const float *x, const float *c, int
     return dist;
 }
 
+// a row of D floats into registers (zeros past D): with VEC -- D equals DM
+// and rows start on 16-byte (DM a multiple of four) or 8-byte boundaries --
+// four or two floats at a time
+template <int DM, bool VEC>
+__device__ __forceinline__ void load_row(const float *c, int D, float (&v)[DM])
+{
+    if (VEC && DM % 4 == 0) {
+#pragma unroll
+        for (int d = 0; d + 3 < DM; d += 4) {
+            const float4 f = __ldg(reinterpret_cast<const float4 *>(c + d));
+            v[d] = f.x;
+            v[d + 1] = f.y;
+            v[d + 2] = f.z;
+            v[d + 3] = f.w;
+        }
+    } else if (VEC) {
+#pragma unroll
+        for (int d = 0; d + 1 < DM; d += 2) {
+            const float2 f = __ldg(reinterpret_cast<const float2 *>(c + d));
+            v[d] = f.x;
+            v[d + 1] = f.y;
+        }
+    } else {
+#pragma unroll
+        for (int d = 0; d < DM; ++d) v[d] = d < D ? __ldg(c + d) : 0.f;
+    }
+}
+
 static __global__ void k_set2(int32_t *a, int32_t *b, int32_t va, int32_t vb)
 {
     *a = va;

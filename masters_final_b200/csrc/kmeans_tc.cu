@@ -546,26 +546,6 @@ __global__ void k_exact_all(const float *__restrict__ X, int32_t n, int32_t D,
 // every centroid that can hold the reference's minimum -- and every one tied
 // with it -- has an FP32 sum within (1 + 4 (D + 2) 2^-24) of the smallest
 // FP32 sum, with a factor 2 to spare.
-// a centroid row into registers: four floats at a time when D is a
-// multiple of four (rows then start on 16-byte boundaries)
-template <int DM, bool VEC>
-__device__ __forceinline__ void load_row(const float *c, int D, float (&v)[DM])
-{
-    if (VEC) {
-#pragma unroll
-        for (int d = 0; d < DM; d += 4) {
-            const float4 f = __ldg(reinterpret_cast<const float4 *>(c + d));
-            v[d] = f.x;
-            v[d + 1] = f.y;
-            v[d + 2] = f.z;
-            v[d + 3] = f.w;
-        }
-    } else {
-#pragma unroll
-        for (int d = 0; d < DM; ++d) v[d] = d < D ? __ldg(c + d) : 0.f;
-    }
-}
-
 template <int DM>
 __device__ __forceinline__ float screen_dist(const float (&x)[DM], const float (&c)[DM], int D)
 {
