@@ -49,9 +49,9 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src)
 // two points at a time (fma.rn.f32x2).  A thread holds 2 NP points in
 // registers and reads each centroid row (the half norm, then the values
 // negated) from shared memory as a broadcast, a vector ahead of its use.
-// The best two scores and the winner's group of four centroids are kept per
-// point with 12 min/max/select operations per group: three per centroid,
-// where an index per centroid took five.
+// Per point the best two chunk minima and the winner's chunk are kept (chunks
+// of four or eight centroids); the runner-up inside that chunk is found at
+// the end from the same scores.
 //
 // Error: with S = |x|^2 + |c|^2 (centred, u = 2^-24), centring both sides
 // moves the distance by at most 4 u S, the half norm and the chain of D
@@ -64,37 +64,15 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src)
 // One pass: 500,000 x 16 points, 20 partitions of 530: 20.5 ms with a
 // subtract and a multiply-add per dimension and an index per centroid; 6.4
 // with scalar row loads and re-reads of the winner's group at the end (a
-// lane per row: D loads of 32 sectors each); 3.7 with vector loads.  32
-// dimensions, 10 partitions: 6.3 -> 4.0.  1,000,000 x 2, k 1,024: 0.90 ->
-// 0.25 ms.
+// lane per row: D loads of 32 sectors each); 3.7 with vector loads, 3.5 with
+// chunk minima.  32 dimensions, 10 partitions: 6.3 -> 3.9.  1,000,000 x 2,
+// k 1,024: 0.90 -> 0.15 ms.
 constexpr int kLT = 128;               // label threads per block
 
 template <int DM> struct LabelRow {
     static constexpr int RF = (DM + 4) & ~3;             // floats of a staged centroid
     static constexpr int CH = 128;                       // centroids per staging buffer
 };
-
-__device__ __forceinline__ uint64_t pack2(float a, float b)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float &a, float &b)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t twice(float a) { return pack2(a, a); }
-__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ float min3(float a, float b, float c)
-{
-    return fminf(fminf(a, b), c);
-}
 
 // staged centroid rows: the half norm, then -c; rows past k get an infinite
 // half norm and never win
@@ -127,8 +105,9 @@ __global__ void k_prep_label_f32(const float *__restrict__ C, const int32_t *__r
     }
 }
 
-// VEC: D equals DM and the rows of X and C can be read as vectors
-template <int DM, int NP, bool VEC>
+// CK: centroids per chunk; VEC: D equals DM and the rows of X and C can be
+// read as vectors
+template <int DM, int NP, int CK, bool VEC>
 __global__ void __launch_bounds__(kLT, 4)
 k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__restrict__ C,
             const float *__restrict__ rows, const int32_t *__restrict__ kk, int32_t kmax,
@@ -138,6 +117,7 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
 {
     constexpr int RF = LabelRow<DM>::RF, CH = LabelRow<DM>::CH, Q = 2 * NP;
     __shared__ __align__(16) float cs[2][(CH + 4) * RF];
+    static_assert(CH % CK == 0 && kTcCentPad % CK == 0, "whole chunks");
     const int p = blockIdx.y;
     if (!active[p]) return;
     const int K = kk[p];
@@ -184,7 +164,8 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                         // this buffer is there, the other one is free
         if (c0 + CH < K) stage(c0 + CH, buf ^ 1);
-        const int g1 = min(CH, K - c0 + 3) >> 2;
+        const int g1 = min(CH, (K - c0 + CK - 1) / CK * CK) >> 2;    // groups of four
+        float cmin[Q];                           // the chunk's least scores
         // the four rows' next 16-byte vectors are read while the current ones
         // are used (past the last group they are read and dropped)
         const float *row = cs[buf];
@@ -216,7 +197,8 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
 #pragma unroll
                 for (int c = 0; c < 4; ++c) f[c] = nx[c];
             }
-            const int id = (c0 >> 2) + g;
+            const bool first = CK == 4 || (g & 1) == 0, ends = CK == 4 || (g & 1) == 1;
+            const int id = (c0 + 4 * g) / CK;
 #pragma unroll
             for (int j = 0; j < NP; ++j) {
                 float s[4][2];
@@ -225,12 +207,9 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int q = 2 * j + h;
-                    const float l0 = fminf(s[0][h], s[1][h]), h0 = fmaxf(s[0][h], s[1][h]);
-                    const float l1 = fminf(s[2][h], s[3][h]), h1 = fmaxf(s[2][h], s[3][h]);
-                    const float m1 = fminf(l0, l1), m2 = min3(fmaxf(l0, l1), h0, h1);
-                    i1[q] = m1 < b1[q] ? id : i1[q];
-                    b2[q] = min3(b2[q], m2, fmaxf(b1[q], m1));
-                    b1[q] = fminf(b1[q], m1);
+                    const float m = min4(s[0][h], s[1][h], s[2][h], s[3][h]);
+                    cmin[q] = first ? m : fminf(cmin[q], m);
+                    if (ends) top2_chunks(cmin[q], id, b1[q], b2[q], i1[q]);
                 }
             }
         }
@@ -240,12 +219,12 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
         const int64_t i = i0 + q * kLT;
         if (i >= n) continue;
         const int64_t o = (int64_t)p * n + i;
-        // the winner inside its group: the one with the same score again
-        const float *rg = rows + ((int64_t)p * kpad + 4 * i1[q]) * RF;
+        // the winner and the runner-up inside its chunk, by the same scores
+        const float *rg = rows + ((int64_t)p * kpad + CK * i1[q]) * RF;
         int bi = -1;
-        float ncw = 0.f;
+        float ncw = 0.f, best = inf;
 #pragma unroll
-        for (int c = 3; c >= 0; --c) {
+        for (int c = 0; c < CK; ++c) {
             float e[RF];
             load_row<RF, true>(rg + c * RF, RF, e);
             float s = e[0];
@@ -255,12 +234,14 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
                 unpack2(x[d][q / 2], v[0], v[1]);
                 s = fmaf(v[q & 1], e[1 + d], s);
             }
-            if (s == b1[q]) {
+            if (s < best) {
                 bi = c;
                 ncw = 2.f * e[0];
             }
+            b2[q] = fminf(b2[q], fmaxf(best, s));
+            best = fminf(best, s);
         }
-        const int w = 4 * i1[q] + bi;
+        const int w = CK * i1[q] + bi;
         // Only a centroid within |x| + sqrt(winner's distance and error) of
         // the origin can be the reference's choice instead of the winner, so
         // its norm -- and with it its error -- is bounded through the
@@ -906,7 +887,7 @@ struct KMWS {
     }
 };
 
-template <int DM, int NP>
+template <int DM, int NP, int CK>
 static int launch_label(cudaStream_t st, const float *X, int32_t n, int32_t D, int32_t P,
                         const float *C, const int32_t *kk, int32_t kmax, const int32_t *active,
                         int32_t *labels, float *dists, int32_t *amb, int *namb, const TcScratch &s)
@@ -924,10 +905,10 @@ static int launch_label(cudaStream_t st, const float *X, int32_t n, int32_t D, i
     // rows as vectors where their length and place allow it
     const uintptr_t at = (uintptr_t)X | (uintptr_t)C;
     if (D == DM && at % (DM % 4 == 0 ? 16 : 8) == 0)
-        k_label_f32<DM, NP, true><<<grid, kLT, 0, st>>>(X, n, D, C, rows, kk, kmax, kpad, active,
+        k_label_f32<DM, NP, CK, true><<<grid, kLT, 0, st>>>(X, n, D, C, rows, kk, kmax, kpad, active,
                                                         s.mu, s.cmax2, E, labels, dists, amb, namb);
     else
-        k_label_f32<DM, NP, false><<<grid, kLT, 0, st>>>(X, n, D, C, rows, kk, kmax, kpad, active,
+        k_label_f32<DM, NP, CK, false><<<grid, kLT, 0, st>>>(X, n, D, C, rows, kk, kmax, kpad, active,
                                                          s.mu, s.cmax2, E, labels, dists, amb, namb);
     EACB_CHECK_LAUNCH();
     ps.done(0.0);
@@ -947,19 +928,26 @@ int label_pass_f32(const float *X, int32_t n, int32_t D, int32_t P, const float 
     auto many = [&](int np) {
         return ((int64_t)n + 2 * np * kLT - 1) / (2 * np * kLT) * P >= 148 * 4;
     };
-#define EACB_LABEL(DM, NPW)                                                                    \
-    (many(NPW) ? launch_label<DM, NPW>(st, X, n, D, P, C, kk, kmax, active, labels, dists, amb, \
-                                       namb, s)                                                \
-               : launch_label<DM, 1>(st, X, n, D, P, C, kk, kmax, active, labels, dists, amb,  \
-                                     namb, s))
-    if (D <= 2) r = EACB_LABEL(2, 4);
-    else if (D <= 4) r = EACB_LABEL(4, 4);
-    else if (D <= 6) r = EACB_LABEL(6, 4);
-    else if (D <= 8) r = EACB_LABEL(8, 4);
-    else if (D <= 12) r = EACB_LABEL(12, 2);
-    else if (D <= 16) r = EACB_LABEL(16, 2);
-    else if (D <= 24) r = EACB_LABEL(24, 1);
-    else r = EACB_LABEL(32, 1);
+    // chunks of eight for few dimensions and many centroids, where the min
+    // operations cost more than the eight rows compared at the end (2
+    // dimensions, 1,000,000 points, k 1,024: 153 us, 250 with the runner-up
+    // tracked throughout; 100 x 10,000, k 75: 39 us against 26 with four)
+    const bool wide = kmax >= 256;
+#define EACB_LABEL(DM, NPW, CKW)                                                                 \
+    (!many(NPW) ? launch_label<DM, 1, 4>(st, X, n, D, P, C, kk, kmax, active, labels, dists, amb, \
+                                         namb, s)                                                 \
+     : wide     ? launch_label<DM, NPW, CKW>(st, X, n, D, P, C, kk, kmax, active, labels, dists,  \
+                                             amb, namb, s)                                        \
+                : launch_label<DM, NPW, 4>(st, X, n, D, P, C, kk, kmax, active, labels, dists,    \
+                                           amb, namb, s))
+    if (D <= 2) r = EACB_LABEL(2, 4, 8);
+    else if (D <= 4) r = EACB_LABEL(4, 4, 8);
+    else if (D <= 6) r = EACB_LABEL(6, 4, 4);
+    else if (D <= 8) r = EACB_LABEL(8, 4, 4);
+    else if (D <= 12) r = EACB_LABEL(12, 2, 4);
+    else if (D <= 16) r = EACB_LABEL(16, 2, 4);
+    else if (D <= 24) r = EACB_LABEL(24, 1, 4);
+    else r = EACB_LABEL(32, 1, 4);
 #undef EACB_LABEL
     if (r) return r;
     return label_exact_points(X, n, D, P, C, kk, kmax, labels, dists, amb, namb, nullptr, st);

@@ -20,6 +20,47 @@ __device__ __forceinline__ double exact_dist(const float *x, const float *c, int
     return dist;
 }
 
+__device__ __forceinline__ uint64_t pack2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t twice(float a) { return pack2(a, a); }
+__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// Folds the least score of a chunk of centroids into the best two chunk
+// minima and the winner's chunk.  The runner-up inside the winner's chunk is
+// looked for once, at the end: per centroid this takes 1.6 (chunks of four)
+// or 1.1 (eight) operations of the half-rate ALU pipe that bounds the label
+// passes, where keeping the best two of all centroids took 3.5 and an index
+// per centroid 5.
+__device__ __forceinline__ void top2_chunks(float m, int id, float &b1, float &b2, int &i1)
+{
+    i1 = m < b1 ? id : i1;
+    b2 = fminf(b2, fmaxf(b1, m));
+    b1 = fminf(b1, m);
+}
+__device__ __forceinline__ float min4(float a, float b, float c, float d)
+{
+    return fminf(min3(a, b, c), d);
+}
+
 // a row of D floats into registers (zeros past D): with VEC -- D equals DM
 // and rows start on 16-byte (DM a multiple of four) or 8-byte boundaries --
 // four or two floats at a time

@@ -6,13 +6,15 @@
 // significant bits) and the K dimension holds the six products that matter
 // (see put_row), the large h*h group last.  The epilogue (8 warps, one point
 // row per thread, half the columns per warp) reads the accumulator tile
-// from TMEM with tcgen05.ld, forms the screened distance and keeps the best
-// two per point.  A point whose runner-up lies within the proven error bound
-// E (|x|^2 + max|c|^2) of its winner (E from the split, the accumulation
-// order and the epilogue arithmetic, times 2) is re-labelled by the
-// reference's exact loop; every other point gets its winner's exact
-// reference distance.  Labels therefore equal the reference's
-// (MyML/MyML/cluster/KMeans.py:453-490) for any input.
+// from TMEM with tcgen05.ld, forms the screened distances and keeps the best
+// two of the minima of four columns per point, with the winner's four.  A
+// point whose best columns outside the winner's four, or whose distances
+// inside it, are not apart by more than the proven error bound is
+// re-labelled in the reference's arithmetic; every other point gets its
+// winner's exact reference distance.  Labels therefore equal the reference's
+// (MyML/MyML/cluster/KMeans.py:453-490) for any input.  2,000,000 x 8, ten
+// partitions of about 1,000: 7.8 ms a pass with an index and a runner-up per
+// column (six instructions), 6.3 now (two and a half).
 //
 // Shapes: M = 128 points per CTA, N <= 128 centroids per MMA tile, K = 6d
 // padded to a multiple of 16 (<= 192).  Operands are pre-arranged in global
@@ -273,7 +275,41 @@ __global__ void k_prep_centroids(const float *C, const int32_t *kk, int32_t kmax
     }
 }
 
+template <int DM>
+__device__ __forceinline__ float screen_dist(const float (&x)[DM], const float (&c)[DM], int D)
+{
+    float acc = 0.f;
+#pragma unroll
+    for (int d = 0; d < DM; ++d)
+        if (d < D) {
+            const float diff = __fsub_rn(x[d], c[d]);
+            acc = __fmaf_rn(diff, diff, acc);
+        }
+    return acc;
+}
+
+template <int DM>
+__device__ __forceinline__ double exact_dist_reg(const float (&x)[DM], const float (&c)[DM], int D)
+{
+    double dist = 0.0;
+#pragma unroll
+    for (int d = 0; d < DM; ++d)
+        if (d < D) {
+            const float diff = __fsub_rn(x[d], c[d]);
+            dist = __dadd_rn(dist, (double)__fmul_rn(diff, diff));
+        }
+    return dist;
+}
+
 // ---------------------------------------------------------------- labels --
+// columns of which only the least score is kept: the winner's chunk is
+// compared again at the end, a row of D floats per column (with eight columns
+// the rows cost more than the scores saved)
+constexpr int kTcChunk = 4;
+
+// DM: D rounded up to 4, 8, 16 or 32; VEC: D equals DM and the rows of X and C
+// can be read as 16-byte vectors
+template <int DM, bool VEC>
 __global__ void __launch_bounds__(kTThreads, 4)
 k_label_tc(const float *__restrict__ X, int32_t n, int32_t D, int32_t Kp, const float *__restrict__ C,
            const int32_t *__restrict__ kk, int32_t kmax, int32_t kt_max, int32_t P, int32_t ppc,
@@ -422,13 +458,18 @@ k_label_tc(const float *__restrict__ X, int32_t n, int32_t D, int32_t Kp, const 
             // the screened distance less the row's |x|^2 (the same for every
             // column, so the order and the gaps are those of the distance):
             // one rounding, where adding |x|^2 first would take two
-            const int cb = t * kTN + c0;
+            constexpr int CK = kTcChunk;
+            const int gb = (t * kTN + c0) / CK;
+            const uint64_t m2 = pack2(-2.f, -2.f);
 #pragma unroll
-            for (int jj = 0; jj < 32; ++jj) {
-                const float sv = fmaf(-2.f, v[jj], ncv[jj]);      // ncp[c] = +inf past K
-                i1 = sv < b1 ? cb + jj : i1;
-                b2 = fminf(b2, fmaxf(b1, sv));
-                b1 = fminf(b1, sv);
+            for (int g = 0; g < 32 / CK; ++g) {
+                float sc[CK];
+#pragma unroll
+                for (int h = 0; h < CK; h += 2)      // ncp[c] = +inf past K
+                    unpack2(ffma2(m2, pack2(v[CK * g + h], v[CK * g + h + 1]),
+                                  pack2(ncv[CK * g + h], ncv[CK * g + h + 1])),
+                            sc[h], sc[h + 1]);
+                top2_chunks(min4(sc[0], sc[1], sc[2], sc[3]), gb + g, b1, b2, i1);
             }
         }
         tc_fence_before();
@@ -461,22 +502,42 @@ k_label_tc(const float *__restrict__ X, int32_t n, int32_t D, int32_t Kp, const 
                 }
                 // Column c's screened distance is within e(c) = E/2 (|x|^2 +
                 // |c|^2) of the exact one.  A column c* that the exact
-                // arithmetic could rank at or before the winner w has
-                // |x - c*|^2 <= |x - c_w|^2 <= w1 + |x|^2 + e(w), so |c*| <=
-                // |x| + sqrt(w1 + |x|^2 + e(w)) (capped by the largest norm).
-                // The winner is certain when the runner-up is more than e(w) +
-                // e(c*) above it (the bound taken 1% wide for the rounding of
-                // this arithmetic).
-                const float ew = 0.5f * E * (xn + nc[((int64_t)p * kt_max) * kTN + wi]);
-                const float rc = sqrtf(xn) + sqrtf(fmaxf(0.f, w1 + xn + ew));
-                const float cstar2 = fminf(rc * rc, cmax2[p]);
-                const float bound = 1.01f * (ew + 0.5f * E * (xn + cstar2));
+                // arithmetic could rank at or before the least screened one,
+                // w, has |x - c*|^2 <= |x - c_w|^2 <= w1 + |x|^2 + e(w), so
+                // |c*| and |c_w| are at most |x| + sqrt(w1 + |x|^2 + e(w))
+                // and at most the partition's largest norm (which bounds the
+                // e(w) under the root).  No column outside w's chunk comes
+                // before w when the least of them is more than e(w) + e(c*)
+                // above it (the bound taken 1% wide for the rounding of this
+                // arithmetic).
+                const float cm2 = cmax2[p];
+                const float rc = sqrtf(xn) + sqrtf(fmaxf(0.f, w1 + xn + 0.5f * E * (xn + cm2)));
+                const float bound = 1.01f * E * (xn + fminf(rc * rc, cm2));
+                // inside the chunk: direct float32 distances, within (D + 2)
+                // 2^-24 of the reference's (relative), so the least is
+                // certain when the next is beyond four times that
+                const int64_t row0 = (int64_t)p * kmax;
+                constexpr int CK = kTcChunk;
+                float xv[DM], cv[DM];
+                load_row<DM, VEC>(X + i * D, D, xv);
+                float bd = __int_as_float(0x7f800000), bd2 = bd;
+                int w = -1;
+#pragma unroll
+                for (int c = 0; c < CK; ++c) {
+                    if (CK * wi + c >= kk[p]) break;
+                    load_row<DM, VEC>(C + (row0 + CK * wi + c) * D, D, cv);
+                    const float d32 = screen_dist<DM>(xv, cv, DM);
+                    w = d32 < bd ? CK * wi + c : w;
+                    bd2 = fminf(bd2, fmaxf(bd, d32));
+                    bd = fminf(bd, d32);
+                }
+                const float thr = __fadd_ru(__fmul_ru(bd, 1.f + 4.f * (float)(D + 2) * 5.9604645e-8f),
+                                            1e-38f);
                 const int64_t o = (int64_t)p * n + i;
-                if (w2 - w1 > bound) {
-                    float xv[32];
-                    for (int d = 0; d < D; ++d) xv[d] = X[i * D + d];
-                    labels[o] = wi;
-                    dists[o] = (float)exact_dist<32>(xv, C + ((int64_t)p * kmax + wi) * D, D);
+                if (w2 - w1 > bound && bd2 > thr && w >= 0) {
+                    load_row<DM, VEC>(C + (row0 + w) * D, D, cv);
+                    labels[o] = w;
+                    dists[o] = (float)exact_dist_reg<DM>(xv, cv, D);
                 } else {
                     amb[atomicAdd(namb, 1)] = (int32_t)o;
                 }
@@ -546,32 +607,6 @@ __global__ void k_exact_all(const float *__restrict__ X, int32_t n, int32_t D,
 // every centroid that can hold the reference's minimum -- and every one tied
 // with it -- has an FP32 sum within (1 + 4 (D + 2) 2^-24) of the smallest
 // FP32 sum, with a factor 2 to spare.
-template <int DM>
-__device__ __forceinline__ float screen_dist(const float (&x)[DM], const float (&c)[DM], int D)
-{
-    float acc = 0.f;
-#pragma unroll
-    for (int d = 0; d < DM; ++d)
-        if (d < D) {
-            const float diff = __fsub_rn(x[d], c[d]);
-            acc = __fmaf_rn(diff, diff, acc);
-        }
-    return acc;
-}
-
-template <int DM>
-__device__ __forceinline__ double exact_dist_reg(const float (&x)[DM], const float (&c)[DM], int D)
-{
-    double dist = 0.0;
-#pragma unroll
-    for (int d = 0; d < DM; ++d)
-        if (d < D) {
-            const float diff = __fsub_rn(x[d], c[d]);
-            dist = __dadd_rn(dist, (double)__fmul_rn(diff, diff));
-        }
-    return dist;
-}
-
 constexpr int kExactThreads = 256;
 constexpr int kExactCacheK = 2048;     // FP32 sums kept in shared memory up to this k
 
@@ -749,7 +784,6 @@ int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *
     // a floor on the request so that no more CTAs than asked share an SM
     const size_t floor_bytes = (size_t)(228 / (ctas + 1) + 2) * 1024;
     const size_t smem_req = smem < floor_bytes ? floor_bytes : smem;
-    EACB_CUDA(allow_max_dyn_smem(k_label_tc));
     // one CTA per 128-point tile and share of the partitions: all partitions
     // (the tile's operands load once) unless that leaves fewer than two
     // CTAs per SM slot in flight
@@ -759,9 +793,23 @@ int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *
     const int ppc = (P + groups - 1) / groups;
     dim3 grid((unsigned)ptiles, (unsigned)((P + ppc - 1) / ppc));
     ProfScope ps(PROF_KMEANS, st);
-    k_label_tc<<<grid, kTThreads, smem_req, st>>>(X, n, D, s.Kp, C, kk, kmax, s.kt_max, P, ppc, active,
-                                                  s.A, s.nx, s.B, s.nc, s.cmax2, E, nbuf, labels, dists,
-                                                  amb, namb, s.err);
+    cudaError_t ce = cudaSuccess;
+    auto go = [&](auto kern) {
+        if ((ce = allow_max_dyn_smem(kern)) != cudaSuccess) return;
+        kern<<<grid, kTThreads, smem_req, st>>>(X, n, D, s.Kp, C, kk, kmax, s.kt_max, P, ppc, active,
+                                                s.A, s.nx, s.B, s.nc, s.cmax2, E, nbuf, labels, dists,
+                                                amb, namb, s.err);
+    };
+    const bool al = ((uintptr_t)X % 16 == 0) && ((uintptr_t)C % 16 == 0);
+    if (D == 4 && al) go(k_label_tc<4, true>);
+    else if (D <= 4) go(k_label_tc<4, false>);
+    else if (D == 8 && al) go(k_label_tc<8, true>);
+    else if (D <= 8) go(k_label_tc<8, false>);
+    else if (D == 16 && al) go(k_label_tc<16, true>);
+    else if (D <= 16) go(k_label_tc<16, false>);
+    else if (D == 32 && al) go(k_label_tc<32, true>);
+    else go(k_label_tc<32, false>);
+    EACB_CUDA(ce);
     EACB_CHECK_LAUNCH();
     ps.done(0.0);
     k_exact_all<<<296, 256, 0, st>>>(X, n, D, C, kk, kmax, P, active, s.err, labels, dists);
