@@ -145,3 +145,20 @@ def test_label_f32_special_values(bad):
     lab, dist = kmeans_label(x, c, label_mode="cuda")
     assert np.array_equal(lab.cpu().numpy(), want[0])
     assert np.array_equal(dist.cpu().numpy(), want[1], equal_nan=True)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 15])
+@pytest.mark.parametrize("n", [1, 14, 16, 17, 31, 64, 4096 + 5, 1 << 20, (1 << 22) + 13])
+def test_diassoc_edges(n, offset):
+    """top - count on spans that start and end off the 16-byte boundary; the
+    bytes around the span stay as they are."""
+    import torch
+    from masters_final_b200 import _lib
+    rng = np.random.default_rng(n)
+    host = rng.integers(0, 256, n + 40, dtype=np.uint8)
+    d = torch.from_numpy(host.copy()).cuda()
+    span = d[offset:offset + n]
+    _lib.check(_lib.load().eacb_make_diassoc(_lib.ptr(span), n, 101, _lib.stream_handle()), "diassoc")
+    want = host.copy()
+    want[offset:offset + n] = (101 - want[offset:offset + n].astype(np.int64)).astype(np.uint8)
+    assert np.array_equal(d.cpu().numpy(), want)
