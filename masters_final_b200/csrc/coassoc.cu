@@ -1141,12 +1141,7 @@ extern "C" int eacb_coassoc_prepare(const int32_t *labels, int32_t n, int32_t P,
     k_ml_count<<<(unsigned)(P * nt), 256, K * sizeof(int), st>>>(labels, n, K, nt, w.cnt, w.err);
     EACB_CHECK_LAUNCH();
     if ((s = scan_launch<int32_t, int64_t>(w.cnt, w.S, m, 0, &w.S[m], w.scan, st))) return s;
-    const size_t place_smem = (size_t)K * (sizeof(int64_t) + sizeof(int32_t));
-    if (place_smem > 48 * 1024)
-        EACB_CUDA(allow_max_dyn_smem(k_ml_place));
-    k_ml_place<<<(unsigned)(P * nt), 32, place_smem, st>>>(labels, n, K, nt, w.S, w.members,
-                                                           w.mypos);
-    EACB_CHECK_LAUNCH();
+    if ((s = launch_ml_place(st, labels, n, P, K, nt, w.S, w.members, w.mypos))) return s;
     EACB_CUDA(cudaMemsetAsync(w.maxcnt, 0, sizeof(int), st));
     k_ncl<<<P, 256, 0, st>>>(w.S, K, nt, w.ncl, w.maxcnt);
     EACB_CHECK_LAUNCH();

@@ -1007,12 +1007,7 @@ extern "C" int eacb_kmeans_ensemble(const float *X, int32_t n, int32_t d, int32_
                                                                         w.err);
         EACB_CHECK_LAUNCH();
         if ((s = scan_launch<int32_t, int64_t>(w.cnt, w.S, m, 0, &w.S[m], w.scan, st))) return s;
-        const size_t place_smem = (size_t)kmax * (sizeof(int64_t) + sizeof(int32_t));
-        if (place_smem > 48 * 1024)
-            EACB_CUDA(allow_max_dyn_smem(k_ml_place));
-        k_ml_place<<<(unsigned)(P * nt), 32, place_smem, st>>>(labels, n, kmax, nt, w.S, w.members,
-                                                               w.mypos);
-        EACB_CHECK_LAUNCH();
+        if ((s = launch_ml_place(st, labels, n, P, kmax, nt, w.S, w.members, w.mypos))) return s;
         EACB_CUDA(cudaMemsetAsync(w.nempty, 0, sizeof(int32_t) * P, st));
         if ((s = launch_centroids(st, centroid_mode == 1, X, d, P, w.members, w.S, kmax, nt, k, kmax,
                                   w.active, centroids, w.nempty)))
@@ -1153,10 +1148,7 @@ extern "C" int eacb_kmeans_centroids(const float *X, int32_t n, int32_t d, const
     EACB_CHECK_LAUNCH();
     int s = scan_launch<int32_t, int64_t>(w.cnt, w.S, m, 0, &w.S[m], w.scan, st);
     if (s) return s;
-    const size_t place_smem = (size_t)k * (sizeof(int64_t) + sizeof(int32_t));
-    if (place_smem > 48 * 1024) EACB_CUDA(allow_max_dyn_smem(k_ml_place));
-    k_ml_place<<<(unsigned)nt, 32, place_smem, st>>>(labels, n, k, nt, w.S, w.members, w.mypos);
-    EACB_CHECK_LAUNCH();
+    if ((s = launch_ml_place(st, labels, n, 1, k, nt, w.S, w.members, w.mypos))) return s;
     if ((s = launch_centroids(st, centroid_mode == 1, X, d, 1, w.members, w.S, k, nt, w.kk, k,
                               w.active, C, w.nempty)))
         return s;

@@ -162,3 +162,22 @@ def test_diassoc_edges(n, offset):
     want = host.copy()
     want[offset:offset + n] = (101 - want[offset:offset + n].astype(np.int64)).astype(np.uint8)
     assert np.array_equal(d.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("k", [1, 2, 700, 8192])
+@pytest.mark.parametrize("n", [1, 31, 512, 4095, 4096, 4097, 12801])
+def test_member_lists(n, k):
+    """The stable counting sort behind the centroid sums at tile and warp
+    edges, with one, few and the most clusters: float32 sums in point order
+    tell every misplaced member."""
+    import oracle
+    from masters_final_b200.cluster.KMeans import kmeans_centroids
+    rng = np.random.default_rng(n * 7 + k)
+    labels = rng.integers(0, k, n).astype(np.int32)
+    labels[n // 2:] = np.sort(labels[n // 2:])
+    x = (rng.standard_normal((n, 2)) * 10.0 ** rng.integers(-3, 4, (n, 1))).astype(np.float32)
+    dist = rng.random(n).astype(np.float32)
+    if k - np.unique(labels).size >= n:
+        pytest.skip("more empty clusters than points")
+    got = kmeans_centroids(x, labels, dist, k).cpu().numpy()
+    assert np.array_equal(got, oracle.kmeans_centroids(x, labels, dist, k))
