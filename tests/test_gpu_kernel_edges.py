@@ -181,3 +181,28 @@ def test_member_lists(n, k):
         pytest.skip("more empty clusters than points")
     got = kmeans_centroids(x, labels, dist, k).cpu().numpy()
     assert np.array_equal(got, oracle.kmeans_centroids(x, labels, dist, k))
+
+
+@pytest.mark.parametrize("n,P,K,cap", [(300, 5, 3, 110), (4000, 9, 6, 900), (42_000, 5, 12, 4100),
+                                       (41_100, 255, 9, 5000)])
+def test_capped_rows(n, P, K, cap):
+    """Rows over their capacity against the row restatement: spans below and
+    above the rank chunk, many partitions, quotas inside a rank."""
+    import torch
+    import oracle
+    from masters_final_b200.EAC.sparse import CoassocBuilder, capacity_indptr
+    rng = np.random.default_rng(n + P)
+    L = rng.integers(0, K, (P, n)).astype(np.int32)
+    L[rng.random((P, n)) < 0.02] = -1
+    b = CoassocBuilder(L, n)
+    caps = capacity_indptr(n, cap, "constant")
+    ip, ind, dat, nnz, disc, mx = b.build(caps)
+    ip = ip.cpu().numpy()
+    assert disc > 0
+    rows = np.unique(np.concatenate([[0, 1, 2, n // 2, n - 2, n - 1], rng.integers(0, n, 40),
+                                     rng.integers(0, max(1, n - 40_000), 8)]))
+    want = oracle.coassoc_rows(L, caps.cpu().numpy(), rows)
+    for i, (cols, counts) in zip(rows, want):
+        a, e = ip[i], ip[i + 1]
+        assert np.array_equal(ind[a:e].cpu().numpy(), cols), i
+        assert np.array_equal(dat[a:e].cpu().numpy(), counts), i
