@@ -31,6 +31,7 @@
 #include "scan_impl.cuh"
 
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 namespace eacb {
@@ -1180,6 +1181,7 @@ enum : int {
     C_AUX1 = 9,
     C_SYM_LT = 10,    // CSR entries u -> v with u < v (symmetry check)
     C_SYM_GT = 11,    // ... with u > v
+    C_PLAN = 12,      // the final clustering's CutPlan (four words)
     C_COUNT = 16
 };
 
@@ -1837,12 +1839,13 @@ __global__ void k_engine_reset(int *err, int64_t *cnt, unsigned long long *hist,
     }
 }
 
-// Sizes of a round-kernel run started from the host, and its barrier at zero.
+// Sizes of a round-kernel run started from the host (E < 0: the edge words a
+// filter kept, cnt[C_AUX0]), and its barrier at zero.
 __global__ void k_set_sizes(int64_t *cnt, int64_t V, int64_t E, GridBarrier *bar)
 {
     if (threadIdx.x == 0) {
         cnt[C_V] = V;
-        cnt[C_E] = E;
+        cnt[C_E] = E < 0 ? cnt[C_AUX0] : E;
         bar->count = 0;
     }
 }
@@ -1916,11 +1919,15 @@ static int round_team(int64_t V0, int64_t E, int kind, int *team)
 // with the loads of a step in flight together: graph rows are short, and a
 // thread per key keeps every key's dependent loads (key -> row extent ->
 // entries) overlapping with all the others.
+// The number of keys is read on the device (cnt[C_NMST]); after an error of
+// an earlier kernel the keys are not complete and none is looked up.
 template <typename WT>
-__global__ void k_key2eid(const uint64_t *keys, int64_t n_keys, const int32_t *first,
+__global__ void k_key2eid(const uint64_t *keys, const int64_t *cnt, const int32_t *first,
                           const int32_t *deg, const int32_t *dest, const WT *weight, Pack pk,
                           int32_t *out, int *err)
 {
+    if (*(volatile int *)err) return;
+    const int64_t n_keys = cnt[C_NMST];
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n_keys;
          q += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t s = keys[q];
@@ -1986,8 +1993,9 @@ struct Engine {
     static Engine carve(Carver &c, int32_t V0, int64_t Emax)
     {
         Engine g;
-        g.err = c.take<int>(1);
-        g.cnt = c.take<int64_t>(C_COUNT);
+        // the error word and the counts, read by the host in one copy
+        g.err = (int *)c.take<int64_t>(1 + C_COUNT);
+        g.cnt = (int64_t *)g.err + 1;
         g.hist = c.take<unsigned long long>(256);
         g.lohi = c.take<int>(2 * kPhaseSlots);
         g.giant = c.take<int32_t>(1);
@@ -2014,10 +2022,12 @@ struct Engine {
 
     int read_counts(cudaStream_t st, int64_t h[C_COUNT])
     {
-        int e = 0;
-        EACB_CUDA(cudaMemcpyAsync(h, cnt, C_COUNT * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-        EACB_CUDA(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        int64_t both[1 + C_COUNT];
+        EACB_CUDA(cudaMemcpyAsync(both, err, sizeof(both), cudaMemcpyDeviceToHost, st));
         EACB_CUDA(cudaStreamSynchronize(st));
+        std::copy(both + 1, both + 1 + C_COUNT, h);
+        int e;
+        memcpy(&e, both, sizeof(e));
         return dev_err_to_status(e);
     }
 
@@ -2109,11 +2119,10 @@ struct Engine {
     // edges to ea through cnt[C_CURSOR] with their selection in best; the
     // round kernel takes its edge count from the cursor, and the flattening
     // after it clears the slots, the cursor and the barrier for the next
-    // phase.  One read at the end gives the forest size, the component count
-    // and any error.
+    // phase.  Nothing is read: the forest size and any error stay on the
+    // device.
     template <typename Build>
-    int run_phased(Pack pk, const std::vector<Phase> &plan, Build build, cudaStream_t st,
-                   int64_t *n_mst_out, int64_t *n_comp_out)
+    int run_phased(Pack pk, const std::vector<Phase> &plan, Build build, cudaStream_t st)
     {
         for (size_t q = 0; q < plan.size(); ++q) {
             Phase ph = plan[q];
@@ -2123,11 +2132,6 @@ struct Engine {
             if ((s = rounds<SEL_MST>(pk, st, Emax, 1, q == 0 ? 1 : 0, q + 1 < plan.size())))
                 return s;
         }
-        int64_t h[C_COUNT];
-        int s = read_counts(st, h);
-        if (s) return s;
-        *n_mst_out = h[C_NMST];
-        *n_comp_out = plan.empty() ? V0 : h[C_V];
         return EACB_OK;
     }
 
@@ -2137,7 +2141,7 @@ struct Engine {
     // split() cuts from the build's per-weight kept counts, in order.
     template <typename Build, typename Split>
     int run_phased_retry(Pack pk, std::vector<Phase> plan, Build build, Split split,
-                         cudaStream_t st, int64_t *n_mst_out, int64_t *n_comp_out)
+                         cudaStream_t st)
     {
         int64_t V = V0, n_mst = 0;
         size_t q = 0;
@@ -2150,13 +2154,10 @@ struct Engine {
             EACB_CUDA(cudaMemsetAsync(hist, 0, 256 * sizeof(unsigned long long), st));
             int s = build(ph);
             if (s) return s;
-            int64_t Ep = 0;
-            int e = 0;
-            EACB_CUDA(cudaMemcpyAsync(&Ep, &cnt[C_CURSOR], sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                      st));
-            EACB_CUDA(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-            EACB_CUDA(cudaStreamSynchronize(st));
-            if (e == DEV_CAPACITY) {
+            int64_t h[C_COUNT];
+            const int e = read_counts(st, h);
+            const int64_t Ep = h[C_CURSOR];
+            if (e == dev_err_to_status(DEV_CAPACITY)) {
                 // the build still counted every kept entry, per weight, in
                 // hist: the pieces are cut from those counts
                 unsigned long long kh[256];
@@ -2169,7 +2170,7 @@ struct Engine {
                 plan.insert(plan.begin() + (ptrdiff_t)q, pieces.begin(), pieces.end());
                 continue;
             }
-            if (e) return dev_err_to_status(e);
+            if (e) return e;
             if (Ep > Emax) return EACB_ERR_INTERNAL;
             if (prof().enabled) prof().bytes[PROF_PHASE] += 8.0 * (double)Ep;   // words written
             int64_t nc = 0;
@@ -2194,8 +2195,6 @@ struct Engine {
                 }
             }
         }
-        *n_mst_out = n_mst;
-        *n_comp_out = V;
         return EACB_OK;
     }
 
@@ -2249,7 +2248,6 @@ static int csr_graph_run(int mode, const int32_t *dest, const WT *weight, int wb
     if (c.overflow) return EACB_ERR_WORKSPACE;
     if ((s = g.reset(st))) return s;
     int64_t h[C_COUNT];
-    int64_t n_mst = 0, n_comp = 0;
     const unsigned gr = grid_for((int64_t)V * 32, 256);
     const unsigned gph = grid_for(V, kPhThreads, 148 * 4);   // phase builds: grid-stride rows
     if (mode == SEL_MST) {
@@ -2297,7 +2295,15 @@ static int csr_graph_run(int mode, const int32_t *dest, const WT *weight, int wb
             ps.done(12.0 * V + (4.0 + sizeof(WT)) * (double)E);
             return EACB_OK;
         };
-        if ((s = g.run_phased(pk, plan, build, st, &n_mst, &n_comp))) return s;
+        if ((s = g.run_phased(pk, plan, build, st))) return s;
+        if (V > 1) {
+            k_key2eid<WT><<<grid_for(V - 1, 256), 256, 0, st>>>(g.mst, g.cnt, first, deg, dest,
+                                                                  weight, pk, mst_out, g.err);
+            EACB_CHECK_LAUNCH();
+        }
+        if ((s = g.read_counts(st, h))) return s;
+        if (h[C_SYM_LT] != h[C_SYM_GT]) return EACB_ERR_BAD_INPUT;   // not symmetric
+        *host_n_mst = h[C_NMST];
     } else {
         // every entry with identity labels: one word per undirected edge and
         // each vertex's first selection (the reference's round one)
@@ -2309,20 +2315,9 @@ static int csr_graph_run(int mode, const int32_t *dest, const WT *weight, int wb
                 (unsigned long long *)&g.cnt[C_SYM_LT], g.err);
             EACB_CHECK_LAUNCH();
         }
-        if ((s = g.read_counts(st, h))) return s;
-        if (h[C_SYM_LT] != h[C_SYM_GT]) return EACB_ERR_BAD_INPUT;   // not symmetric
-        if ((s = g.run<SEL_CC>(pk, h[C_CURSOR], V, st, &n_mst, &n_comp))) return s;
-    }
-    if (mode == SEL_MST) {
-        if (n_mst > 0) {
-            k_key2eid<WT><<<grid_for(n_mst, 256), 256, 0, st>>>(g.mst, n_mst, first, deg, dest,
-                                                                  weight, pk, mst_out, g.err);
-            EACB_CHECK_LAUNCH();
-        }
-        if ((s = g.read_counts(st, h))) return s;
-        if (h[C_SYM_LT] != h[C_SYM_GT]) return EACB_ERR_BAD_INPUT;   // not symmetric
-        *host_n_mst = n_mst;
-    } else {
+        // the rounds take the words' count from the build's cursor (one word
+        // per undirected edge); everything is queued up to one read
+        if ((s = g.rounds<SEL_CC>(pk, st, E / 2, 1, 1))) return s;
         // the reference's component numbers: ranks of the root ids
         const unsigned gv = grid_for(V, 256);
         k_root_flags<<<gv, 256, 0, st>>>(g.label, V, g.flag);
@@ -2332,8 +2327,10 @@ static int csr_graph_run(int mode, const int32_t *dest, const WT *weight, int wb
         k_rank_roots<<<gv, 256, 0, st>>>(g.label, g.pos, V, labels_out);
         EACB_CHECK_LAUNCH();
         if ((s = g.read_counts(st, h))) return s;
-        if (h[C_AUX1] != n_comp) return EACB_ERR_INTERNAL;
-        *host_n_comp = n_comp;
+        if (h[C_SYM_LT] != h[C_SYM_GT]) return EACB_ERR_BAD_INPUT;   // not symmetric
+        if (h[C_DONE] != 1) return EACB_ERR_NOT_CONVERGED;
+        if (h[C_AUX1] != h[C_V]) return EACB_ERR_INTERNAL;
+        *host_n_comp = h[C_V];
     }
     return EACB_OK;
 }
@@ -2371,8 +2368,9 @@ static int csr_dispatch(int mode, const int32_t *dest, const void *weight, int d
 // ---------------------------------------------------------------------------
 // Final clustering helpers
 // ---------------------------------------------------------------------------
-__global__ void k_weight_hist(const uint64_t *keys, int64_t n, Pack pk, int64_t *hist)
+__global__ void k_weight_hist(const uint64_t *keys, const int64_t *cnt, Pack pk, int64_t *hist)
 {
+    const int64_t n = cnt[C_NMST];
     __shared__ int64_t h[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) h[i] = 0;
     __syncthreads();
@@ -2394,10 +2392,12 @@ struct CutPlan {
 // The lifetime rule of MyML/MyML/EAC/eac.py:366-391 and the cut decision of
 // :220-265, evaluated on the 256-bin histogram of the uint8 MST weights
 // (sorted weights are the bins expanded in order).
-__global__ void k_cut_plan(const int64_t *hist, int64_t n_mst, int32_t n, int32_t max_dist,
-                           int32_t n_clusters, CutPlan *plan)
+// (d_n_mst: the number of weights on the device, or null: n_mst)
+__global__ void k_cut_plan(const int64_t *hist, int64_t n_mst, const int64_t *d_n_mst, int32_t n,
+                           int32_t max_dist, int32_t n_clusters, CutPlan *plan)
 {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    if (d_n_mst) n_mst = *d_n_mst;
     CutPlan p{0, 0, 255, 0};
     const int64_t n_disc = (int64_t)n - n_mst;
     int64_t nc;
@@ -2623,11 +2623,10 @@ static int split_final_phase(const Phase &ph, const unsigned long long kh[256], 
 }
 
 static void carve_final(Carver &c, int32_t n, int64_t nnz, Engine *g, int64_t **hist,
-                        CutPlan **plan, int32_t **cmin)
+                        int32_t **cmin)
 {
     *g = Engine::carve(c, n, final_edge_cap(n, nnz));
     *hist = c.take<int64_t>(256);
-    *plan = c.take<CutPlan>(1);
     *cmin = c.take<int32_t>(n);
 }
 
@@ -2636,9 +2635,8 @@ extern "C" size_t eacb_final_clustering_workspace_size(int32_t n, int64_t nnz)
     Carver c(nullptr, 0);
     Engine g;
     int64_t *h;
-    CutPlan *p;
     int32_t *m;
-    carve_final(c, n, nnz, &g, &h, &p, &m);
+    carve_final(c, n, nnz, &g, &h, &m);
     return c.off;
 }
 
@@ -2658,9 +2656,8 @@ extern "C" int eacb_final_clustering(const int64_t *indptr, const int32_t *indic
     Carver c(ws, ws_bytes);
     Engine g;
     int64_t *hist;
-    CutPlan *plan;
     int32_t *cmin;
-    carve_final(c, n, nnz, &g, &hist, &plan, &cmin);
+    carve_final(c, n, nnz, &g, &hist, &cmin);
     if (c.overflow) return EACB_ERR_WORKSPACE;
     g.kind = 1;
     if ((s = g.reset(st))) return s;
@@ -2669,7 +2666,6 @@ extern "C" int eacb_final_clustering(const int64_t *indptr, const int32_t *indic
     if (nnz > 0) {
         if ((s = launch_whist_u8(diassoc, nnz, g.hist, st))) return s;
     }
-    int64_t n_mst = 0, n_comp = 0;
     unsigned long long wh[256];
     if ((s = g.read_hist(st, wh))) return s;
     std::vector<Phase> phases;
@@ -2704,21 +2700,23 @@ extern "C" int eacb_final_clustering(const int64_t *indptr, const int32_t *indic
         return split_final_phase(ph, kh, g.Emax, indptr, n, hip, st, out);
     };
     if (g.Emax >= nnz) {
-        if ((s = g.run_phased(pk, phases, build, st, &n_mst, &n_comp))) return s;
+        if ((s = g.run_phased(pk, phases, build, st))) return s;
     } else {
-        if ((s = g.run_phased_retry(pk, phases, build, split, st, &n_mst, &n_comp))) return s;
+        if ((s = g.run_phased_retry(pk, phases, build, split, st))) return s;
     }
     // 2. lifetime rule on the weight histogram
+    static_assert(sizeof(CutPlan) == (C_COUNT - C_PLAN) * sizeof(int64_t), "the plan is read with the counts");
     EACB_CUDA(cudaMemsetAsync(hist, 0, 256 * sizeof(int64_t), st));
-    if (n_mst > 0) {
-        k_weight_hist<<<grid_for(n_mst, 256, 148 * 4), 256, 0, st>>>(g.mst, n_mst, pk, hist);
-        EACB_CHECK_LAUNCH();
-    }
-    k_cut_plan<<<1, 32, 0, st>>>(hist, n_mst, n, max_dist, n_clusters, plan);
+    k_weight_hist<<<grid_for(n, 256, 148 * 4), 256, 0, st>>>(g.mst, g.cnt, pk, hist);
     EACB_CHECK_LAUNCH();
+    k_cut_plan<<<1, 32, 0, st>>>(hist, 0, &g.cnt[C_NMST], n, max_dist, n_clusters,
+                                  (CutPlan *)&g.cnt[C_PLAN]);
+    EACB_CHECK_LAUNCH();
+    int64_t h[C_COUNT];
+    if ((s = g.read_counts(st, h))) return s;
+    const int64_t n_mst = h[C_NMST];
     CutPlan hp;
-    EACB_CUDA(cudaMemcpyAsync(&hp, plan, sizeof(CutPlan), cudaMemcpyDeviceToHost, st));
-    EACB_CUDA(cudaStreamSynchronize(st));
+    memcpy(&hp, &h[C_PLAN], sizeof(hp));
     if (hp.status) return (int)hp.status;
     *host_n_fclusts = hp.n_clusters;
     if (!hp.need_labels) {
@@ -2731,10 +2729,9 @@ extern "C" int eacb_final_clustering(const int64_t *indptr, const int32_t *indic
     if ((s = g.reset(st))) return s;
     SrcForest sf{g.mst, n_mst, hp.wmax, pk};
     if ((s = g.filter<SEL_CC>(sf, n_mst, g.ea, st))) return s;
-    int64_t h[C_COUNT];
-    if ((s = g.read_counts(st, h))) return s;
-    int64_t nm2 = 0, nc2 = 0;
-    if ((s = g.run<SEL_CC>(pk, h[C_AUX0], n, st, &nm2, &nc2))) return s;
+    k_set_sizes<<<1, 32, 0, st>>>(g.cnt, n, -1, g.bar);      // the filter's count
+    EACB_CHECK_LAUNCH();
+    if ((s = g.rounds<SEL_CC>(pk, st, n_mst))) return s;
     // 4. number components by their smallest member
     EACB_CUDA(cudaMemsetAsync(cmin, 0x7f, sizeof(int32_t) * n, st));
     const unsigned gn = grid_for(n, 256);
@@ -2747,6 +2744,7 @@ extern "C" int eacb_final_clustering(const int64_t *indptr, const int32_t *indic
     k_canon<<<gn, 256, 0, st>>>(g.label, cmin, g.pos, n, labels);
     EACB_CHECK_LAUNCH();
     if ((s = g.read_counts(st, h))) return s;
+    if (h[C_DONE] != 1) return EACB_ERR_NOT_CONVERGED;
     *host_n_fclusts = h[C_AUX1];
     *host_labels_valid = 1;
     return EACB_OK;
@@ -2792,7 +2790,8 @@ extern "C" int eacb_lifetime_cut(const uint8_t *mst_weights, int64_t n_mst, int3
         const int s = launch_whist_u8(mst_weights, n_mst, hist, st);
         if (s) return s;
     }
-    k_cut_plan<<<1, 32, 0, st>>>((const int64_t *)hist, n_mst, n, max_dist, n_clusters, plan);
+    k_cut_plan<<<1, 32, 0, st>>>((const int64_t *)hist, n_mst, nullptr, n, max_dist, n_clusters,
+                                  plan);
     EACB_CHECK_LAUNCH();
     CutPlan hp;
     EACB_CUDA(cudaMemcpyAsync(&hp, plan, sizeof(CutPlan), cudaMemcpyDeviceToHost, st));

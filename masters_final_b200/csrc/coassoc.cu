@@ -86,8 +86,19 @@ constexpr int64_t kPairBytesMax = (int64_t)32 << 30;
 // half2 words per point in the FP16 label copy: P rounded up to 8 partitions
 __host__ __device__ constexpr int32_t pair_words(int32_t P) { return ((P + 7) / 8) * 4; }
 
+// what the host reads after a call, in one copy
+struct CoOut {
+    int err;
+    int maxcnt;                   // largest kept count (prepare: largest cluster)
+    unsigned long long disc;      // discarded counts
+    int64_t nnz;
+};
+
 struct CoWS {
-    int *err;
+    CoOut *out;           // its first word is the workspace's error word
+    int *err;             // ... and the fields' addresses
+    unsigned long long *disc;
+    int *maxcnt;
     int32_t *members;     // P*n, member lists of every partition, back to back
     int32_t *mypos;       // P*n, global position of point i in its member list (-1: none)
     int32_t *cnt;         // P*K*ntiles tile counts
@@ -99,8 +110,6 @@ struct CoWS {
                           //    bit 1 = the row's group takes the pair tiles
     int32_t *rowperm;     // n: the order the row kernels take rows in
     int *queue;           // work-queue counters
-    unsigned long long *disc;   // discarded counts
-    int *maxcnt;          // largest kept count
     int *prow;            // the partition whose clusters order the rows
     uint32_t *lt;         // n x Q: FP16 label pairs, point-major (pair tiles)
     int64_t *grp_off;     // K: a group's neighbourhood in nbr
@@ -120,7 +129,10 @@ struct CoWS {
     static CoWS carve(Carver &c, int32_t n, int32_t P, int32_t K)
     {
         CoWS w;
-        w.err = c.take<int>(1);
+        w.out = c.take<CoOut>(1);
+        w.err = &w.out->err;
+        w.disc = &w.out->disc;
+        w.maxcnt = &w.out->maxcnt;
         w.ntiles = ((int64_t)n + kMLTile - 1) / kMLTile;
         w.Q = pair_words(P);
         w.nbr_cap = 16 * (int64_t)n + 65536;
@@ -138,8 +150,6 @@ struct CoWS {
         w.rowflag = c.take<int32_t>(n);
         w.rowperm = c.take<int32_t>(n);
         w.queue = c.take<int>(kQueues);
-        w.disc = c.take<unsigned long long>(1);
-        w.maxcnt = c.take<int>(1);
         w.prow = c.take<int>(1);
         w.lt = c.take<uint32_t>((size_t)n * w.Q);
         w.grp_off = c.take<int64_t>(K);
@@ -1102,9 +1112,13 @@ __global__ void __launch_bounds__(256) k_diassoc_val(uint8_t *data, int64_t nnz,
     diassoc_span(data, nnz, top);
 }
 
-__global__ void __launch_bounds__(256) k_diassoc(uint8_t *data, int64_t nnz, const int *gmax)
+// (the number of entries and the largest count are read on the device;
+// nothing is written after an error)
+__global__ void __launch_bounds__(256)
+k_diassoc(uint8_t *data, const int64_t *d_nnz, const int *gmax, const int *err)
 {
-    diassoc_span(data, nnz, (uint32_t)(*gmax) + 1u);
+    if (*err) return;
+    diassoc_span(data, *d_nnz, (uint32_t)(*gmax) + 1u);
 }
 
 static unsigned diassoc_grid(int64_t nnz) { return grid_for((nnz + 63) / 64 + 32, 256, 148 * 16); }
@@ -1138,12 +1152,11 @@ static int check_args(const int32_t *labels, int32_t n, int32_t P, int32_t K)
     return EACB_OK;
 }
 
-static int read_err(int *err, cudaStream_t st)
+static int read_out(const CoWS &w, CoOut &h, cudaStream_t st)
 {
-    int e = 0;
-    EACB_CUDA(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    EACB_CUDA(cudaMemcpyAsync(&h, w.out, sizeof(h), cudaMemcpyDeviceToHost, st));
     EACB_CUDA(cudaStreamSynchronize(st));
-    return dev_err_to_status(e);
+    return dev_err_to_status(h.err);
 }
 
 static int row_grid(int ctas_per_sm = 2)
@@ -1194,7 +1207,7 @@ extern "C" int eacb_coassoc_prepare(const int32_t *labels, int32_t n, int32_t P,
     Carver c(ws, ws_bytes);
     CoWS w = CoWS::carve(c, n, P, K);
     if (c.overflow) return EACB_ERR_WORKSPACE;
-    EACB_CUDA(cudaMemsetAsync(w.err, 0, sizeof(int), st));
+    EACB_CUDA(cudaMemsetAsync(w.out, 0, sizeof(CoOut), st));
     EACB_CUDA(cudaMemsetAsync(w.queue, 0, kQueues * sizeof(int), st));
     const int64_t nt = w.ntiles;
     const int64_t m = (int64_t)P * K * nt;
@@ -1202,7 +1215,6 @@ extern "C" int eacb_coassoc_prepare(const int32_t *labels, int32_t n, int32_t P,
     EACB_CHECK_LAUNCH();
     if ((s = scan_launch<int32_t, int64_t>(w.cnt, w.S, m, 0, &w.S[m], w.scan, st))) return s;
     if ((s = launch_ml_place(st, labels, n, P, K, nt, w.S, w.members, w.mypos))) return s;
-    EACB_CUDA(cudaMemsetAsync(w.maxcnt, 0, sizeof(int), st));
     k_ncl<<<P, 256, 0, st>>>(w.S, K, nt, w.ncl, w.maxcnt);
     EACB_CHECK_LAUNCH();
     k_order<<<1, 32, 0, st>>>(w.ncl, P, w.order);
@@ -1228,10 +1240,9 @@ extern "C" int eacb_coassoc_prepare(const int32_t *labels, int32_t n, int32_t P,
     if ((s = scan_launch<int32_t, int64_t>(w.grp_tiles, w.grp_item0, K, 0, &w.grp_item0[K],
                                            w.scan, st)))
         return s;
-    int mc = 0;
-    EACB_CUDA(cudaMemcpyAsync(&mc, w.maxcnt, sizeof(int), cudaMemcpyDeviceToHost, st));
-    if ((s = read_err(w.err, st))) return s;
-    *host_max_cluster = mc;
+    CoOut h;
+    if ((s = read_out(w, h, st))) return s;
+    *host_max_cluster = h.maxcnt;
     return EACB_OK;
 }
 
@@ -1261,9 +1272,12 @@ extern "C" int eacb_coassoc_count(const int32_t *labels, int32_t n, int32_t P, i
         tc, w.order, w.rowlist, w.rowlist_n, cap_indptr, w.rowcnt, w.rowflag, &w.queue[0], w.err);
     EACB_CHECK_LAUNCH();
     ps.done(0.0);
-    if ((s = scan_launch<int32_t, int64_t>(w.rowcnt, indptr, n, 0, &indptr[n], w.scan, st))) return s;
-    EACB_CUDA(cudaMemcpyAsync(host_nnz, &indptr[n], sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    return read_err(w.err, st);
+    if ((s = scan_launch<int32_t, int64_t>(w.rowcnt, indptr, n, 0, &w.out->nnz, w.scan, st))) return s;
+    EACB_CUDA(cudaMemcpyAsync(&indptr[n], &w.out->nnz, sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
+    CoOut h;
+    if ((s = read_out(w, h, st))) return s;
+    *host_nnz = h.nnz;
+    return EACB_OK;
 }
 
 __global__ void k_cap_linear(int32_t n, double m, double b, int64_t ns, int64_t ne, int64_t vs,
@@ -1350,8 +1364,8 @@ extern "C" int eacb_coassoc_fill(const int32_t *labels, int32_t n, int32_t P, in
     CoWS w = CoWS::carve(c, n, P, K);
     if (c.overflow) return EACB_ERR_WORKSPACE;
     EACB_CUDA(cudaMemsetAsync(w.queue, 0, kQueues * sizeof(int), st));
-    EACB_CUDA(cudaMemsetAsync(w.disc, 0, sizeof(unsigned long long), st));
-    EACB_CUDA(cudaMemsetAsync(w.maxcnt, 0, sizeof(int), st));
+    // (the error word is the count's: kept)
+    EACB_CUDA(cudaMemsetAsync(w.maxcnt, 0, sizeof(CoOut) - offsetof(CoOut, maxcnt), st));
     TailCtx tc{labels, w.members, w.mypos, w.S, n, P, K, w.ntiles};
     EACB_CUDA(allow_max_dyn_smem(k_rows_fill));
     EACB_CUDA(allow_max_dyn_smem(k_rows_capped));
@@ -1376,19 +1390,14 @@ extern "C" int eacb_coassoc_fill(const int32_t *labels, int32_t n, int32_t P, in
         tc, w.order, w.rowlist, w.rowlist_n, w.rowflag, cap_indptr, indptr, indices, data,
         &w.queue[2], w.maxcnt, w.disc, w.err);
     EACB_CHECK_LAUNCH();
-    int64_t nnz = 0;
-    EACB_CUDA(cudaMemcpyAsync(&nnz, &indptr[n], sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    unsigned long long dh = 0;
-    int mh = 0;
-    EACB_CUDA(cudaMemcpyAsync(&dh, w.disc, sizeof(dh), cudaMemcpyDeviceToHost, st));
-    EACB_CUDA(cudaMemcpyAsync(&mh, w.maxcnt, sizeof(int), cudaMemcpyDeviceToHost, st));
-    if ((s = read_err(w.err, st))) return s;
-    if (make_diassoc && nnz > 0) {
-        k_diassoc<<<diassoc_grid(nnz), 256, 0, st>>>(data, nnz, w.maxcnt);
+    if (make_diassoc) {
+        k_diassoc<<<148 * 8, 256, 0, st>>>(data, indptr + n, w.maxcnt, w.err);
         EACB_CHECK_LAUNCH();
     }
-    *host_discarded = (int64_t)dh;
-    *host_max_count = mh;
+    CoOut h;
+    if ((s = read_out(w, h, st))) return s;
+    *host_discarded = (int64_t)h.disc;
+    *host_max_count = h.maxcnt;
     return EACB_OK;
 }
 
