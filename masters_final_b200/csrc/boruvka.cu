@@ -1367,11 +1367,11 @@ __device__ __forceinline__ void find_batch(int32_t *parent, int32_t (&x)[N], int
 // Successors of up to kRV active roots at once (s[i] < 0: none): the root of
 // the other end of each selected key, or the root itself when it selected
 // nothing.
+// b receives the selected keys.
 template <int MODE>
 __device__ __forceinline__ void succ_batch(const RoundArgs &a, const int32_t (&s)[kRV],
-                                           int32_t (&t)[kRV])
+                                           int32_t (&t)[kRV], uint64_t (&b)[kRV])
 {
-    uint64_t b[kRV];
 #pragma unroll
     for (int i = 0; i < kRV; ++i) b[i] = s[i] >= 0 ? __ldcg(a.best + s[i]) : kNone;
     if constexpr (MODE == SEL_CC) {
@@ -1474,21 +1474,29 @@ k_rounds(RoundArgs a)
             const int64_t n = __ldcg(a.alen + q);
             int64_t mine = 0;                   // (forest edges << 32) | merges
             for (int64_t ib = tid; ib < n; ib += (int64_t)kRT * kRV) {
-                int32_t s[kRV], t[kRV], tt[kRV], m[kRV];
+                int32_t s[kRV], t[kRV];
+                uint64_t b[kRV], bt[kRV];
 #pragma unroll
                 for (int i = 0; i < kRV; ++i) {
                     const int64_t j = ib + (int64_t)i * kRT;
                     s[i] = j < n ? __ldcg(al + j) : -1;
                 }
-                succ_batch<MODE>(a, s, t);
+                succ_batch<MODE>(a, s, t, b);
                 // mutual pick: only a smaller s with a successor needs t's
+                // selection.  CC keys name the other end; MST keys are one
+                // per edge word and every word is offered to both its ends,
+                // so two roots pick each other exactly when their keys are
+                // the same (no root has to be found again)
 #pragma unroll
-                for (int i = 0; i < kRV; ++i) m[i] = (s[i] >= 0 && s[i] < t[i]) ? t[i] : -1;
-                succ_batch<MODE>(a, m, tt);
+                for (int i = 0; i < kRV; ++i)
+                    bt[i] = (s[i] >= 0 && s[i] < t[i]) ? __ldcg(a.best + t[i]) : kNone;
 #pragma unroll
                 for (int i = 0; i < kRV; ++i) {
                     if (s[i] < 0) continue;
-                    const bool keep = t[i] != s[i] && !(m[i] >= 0 && tt[i] == s[i]);
+                    const bool mutual =
+                        MODE == SEL_MST ? bt[i] != kNone && bt[i] == b[i]
+                                        : bt[i] != kNone && (int32_t)(uint32_t)bt[i] == s[i];
+                    const bool keep = t[i] != s[i] && !mutual;
                     a.color[s[i]] = keep ? t[i] : s[i];
                     mine += keep ? ((MODE == SEL_MST ? (1ll << 32) : 0ll) | 1ll) : 0ll;
                 }
@@ -1677,14 +1685,14 @@ k_rounds(RoundArgs a)
             // the error flag is read beside the counts; the scans' block
             // barriers publish s_err
             const int e_now = tid == 0 ? *(volatile int *)a.err : 0;
-            int64_t x = 0, y = 0;
-            for (int64_t j = tid; j < Pe; j += kRT) {
-                x += __ldcg(a.seg + j);
-                y += __ldcg(a.alen + j);
-            }
+            // one scan of (edge words << 31) | active roots (below 2^31)
+            int64_t x = 0, tot = 0;
+            for (int64_t j = tid; j < Pe; j += kRT)
+                x += (__ldcg(a.seg + j) << 31) + __ldcg(a.alen + j);
             if (tid == 0) s_err = e_now;
-            block_excl_sum_shfl<kRT>(x, En);
-            block_excl_sum_shfl<kRT>(y, An);
+            block_excl_sum_shfl<kRT>(x, tot);
+            En = tot >> 31;
+            An = tot & 0x7fffffffll;
         }
         if (p == 0 && tid == 0 && round < kMaxRounds) {
             a.trace[3 * round] = V;
