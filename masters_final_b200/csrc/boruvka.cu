@@ -893,24 +893,44 @@ k_pick_giant(const int32_t *label, int64_t V0, int32_t *out)
 }
 
 // Same for an upper-triangle CSR with uint8 weights: one word per kept entry,
-// offered to both ends.  Co-association rows are long (thousands of entries), so a
-// warp takes one row and walks it in 128-entry groups, each lane taking four
-// consecutive entries: their four weights (one word) are read first and
-// tested against the phase's range four bytes at once, and the four column
-// indices (16 bytes) only when one of the weights falls in the range, so a
-// phase over a narrow range reads little more than the weight array; only
-// those entries gather the other end's label (none in the first phase, whose
-// labels are the identity).  Kept entries update the selection slots and the
-// per-weight counts as they are found and are staged in shared memory in walk
-// order; the warp then reserves the row's words with one atomic and copies
-// the staging out.  A row with more kept entries than the staging holds
-// walks again to write them.  Each entry is checked (j > i, j < n) in the
-// phase whose range holds its weight.
-constexpr int kUpStage = 128;      // staged edge words per warp
+// offered to both ends.  Co-association rows are long (thousands of entries)
+// and a phase keeps few of them, so the work is split in two.  A scan reads
+// the weights, tests them against the phase's range four bytes at once and
+// records the candidates' entry numbers in shared memory; when a warp's
+// records fill, a dense pass with a record per lane reads their columns and
+// labels, checks the entries (j > i, j < n), updates the selection slots and
+// the per-weight counts, and writes the kept ones' words with one cursor
+// atomic.  Records are carried from row to row, so both halves run with full
+// warps, and the chains of dependent loads are paid per 256 records, not per
+// row.  (One pass that handled its candidates as it found them spent 165
+// instructions and four dependent L2 latencies on each 128 entries; the two
+// sparse phases of 920M entries went from 2.26 and 1.60 to 0.50 and 0.53 ms,
+// 1.8 TB/s of weights, bound by the instructions of the byte tests.)
+struct UpArgs {
+    const int64_t *indptr;
+    const int32_t *indices;
+    const uint8_t *w;
+    int32_t n;
+    int64_t nnz;
+    int lo, hi;                      // weights in (lo, hi]
+    int ident;                       // labels are the identity (nothing merged yet)
+    int64_t row0, row1;
+    const int32_t *label;
+    Pack pk;
+    uint64_t *eout;
+    unsigned long long *cursor;
+    unsigned long long cap;
+    unsigned long long *best;
+    unsigned long long *khist;       // kept entries per weight
+    int *err;
+};
 
-// bit q: byte q of w lies in [L, H], with c1 = (0x8000 - L) and c2 = (0x7fff -
-// H) in both 16-bit halves: bytes 0, 2 and bytes 1, 3 are spread to 16-bit
-// lanes, where bit 15 of x + c1 is x >= L and bit 15 of x + c2 is x > H
+constexpr int kUpRec = 256;          // records per warp, k_phase_upper
+constexpr int kPairRec = 128;        // and k_pair_min
+
+// the words w's bytes q in [L, H] as bits q, with c1 = (0x8000 - L) and c2 =
+// (0x7fff - H) in both 16-bit halves: bytes 0, 2 and bytes 1, 3 are spread to
+// 16-bit lanes, where bit 15 of x + c1 is x >= L and bit 15 of x + c2 is x > H
 __device__ __forceinline__ unsigned bytes_in_range(uint32_t w, uint32_t c1, uint32_t c2)
 {
     const uint32_t e = __byte_perm(w, 0u, 0x4240), o = __byte_perm(w, 0u, 0x4341);
@@ -918,189 +938,496 @@ __device__ __forceinline__ unsigned bytes_in_range(uint32_t w, uint32_t c1, uint
     return ((me >> 15) & 1u) | ((mo >> 14) & 2u) | ((me >> 29) & 4u) | ((mo >> 28) & 8u);
 }
 
-__global__ void __launch_bounds__(kPhThreads, 3)
-k_phase_upper(const int64_t *indptr, const int32_t *indices, const uint8_t *w, int32_t n,
-              int64_t nnz, int lo, int hi, int dense, int ident, int64_t row0, int64_t row1,
-              const int32_t *label, Pack pk, uint64_t *eout, unsigned long long *cursor,
-              unsigned long long cap, unsigned long long *best, unsigned long long *khist,
-              int *err)
+// The warp's n records (entry numbers and their rows): checked, offered and
+// written.  The kept words replace the records from the front (a batch's
+// records are read before its words are written, and there are never more).
+__device__ __forceinline__ void up_flush(const UpArgs &a, uint64_t *rec, const int32_t *rrow, int n,
+                                      unsigned *s_kh)
 {
-    constexpr int G = 4;
-    __shared__ unsigned s_kh[256];           // kept entries per weight, this block
-    __shared__ uint64_t stage_all[kPhWarps][kUpStage];
-    for (int b = threadIdx.x; b < 256; b += blockDim.x) s_kh[b] = 0u;
-    __syncthreads();
+    constexpr int U = 2;
     const int lane = threadIdx.x & 31;
-    uint64_t *stage = stage_all[threadIdx.x >> 5];
-    const uint32_t c1 = 0x00010001u * (uint32_t)(0x8000 - (lo + 1));
-    const uint32_t c2 = 0x00010001u * (uint32_t)(0x7fff - hi);
-    const int64_t nwarps = (int64_t)gridDim.x * kPhWarps;
-    for (int64_t i = row0 + (int64_t)blockIdx.x * kPhWarps + (threadIdx.x >> 5); i < row1;
-         i += nwarps) {
-        const int64_t s = indptr[i], e_end = indptr[i + 1];
-        if (s < 0 || e_end < s || e_end > nnz) {
-            if (lane == 0) set_err(err, DEV_BAD_INPUT);
-            continue;
+    const unsigned below = (1u << lane) - 1u;
+    int out = 0;
+    __syncwarp();
+    for (int b = 0; b < n; b += 32 * U) {
+        int64_t e[U];
+        int32_t i[U], j[U], li[U], lj[U];
+        uint32_t wq[U];
+        uint64_t cj[U], ci[U];
+        bool ok[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int t = b + 32 * u + lane;
+            ok[u] = t < n;
+            e[u] = ok[u] ? (int64_t)rec[t] : 0;
+            i[u] = ok[u] ? rrow[t] : 0;
         }
-        if (s == e_end) continue;
-        const int32_t li = ident ? (int32_t)i : label[i];
-        const int64_t a0 = s & ~(int64_t)3;        // groups start on 16-byte index boundaries
-        // weights of the lane's entries e .. e+3 (zero outside the arrays)
-        auto wload = [&](int64_t e) -> uint32_t {
-            if (e >= e_end) return 0u;
-            if (e + 3 < nnz) return __ldg(reinterpret_cast<const uint32_t *>(w + e));
-            uint32_t v = 0u;
-            for (int q = 0; q < 4 && e + q < nnz; ++q) v |= (uint32_t)w[e + q] << (8 * q);
-            return v;
-        };
-        // bit q: entry e+q is in the row with its weight in (lo, hi]
-        auto cmask = [&](int64_t e, uint32_t wv) -> unsigned {
-            unsigned m = bytes_in_range(wv, c1, c2);
-            if (e < s || e + 4 > e_end) {
-                const int64_t a = s - e, b = e_end - e;     // valid entries [a, b)
-                const int qa = a < 0 ? 0 : (a > 4 ? 4 : (int)a);
-                const int qb = b < 0 ? 0 : (b > 4 ? 4 : (int)b);
-                m &= (0xfu << qa) & (0xfu >> (4 - qb));
-            }
-            return m;
-        };
-        // the indices of the entries in cm (all four in a dense phase)
-        auto jload = [&](int64_t e, unsigned cm) -> int4 {
-            if (dense) cm = e < e_end ? 15u : 0u;
-            if (!cm) return make_int4(0, 0, 0, 0);
-            if (e + 3 < nnz) return __ldg(reinterpret_cast<const int4 *>(indices + e));
-            int32_t t[4] = {0, 0, 0, 0};
-            for (int q = 0; q < 4; ++q)
-                if (((cm >> q) & 1u) && e + q < nnz) t[q] = indices[e + q];
-            return make_int4(t[0], t[1], t[2], t[3]);
-        };
-        // bit q: candidate q is kept (other end in another component); lj
-        // receives the candidates' other-end labels
-        auto keep = [&](unsigned cm, const int4 &jv, int32_t (&lj)[4]) -> unsigned {
-            const int32_t jj[4] = {jv.x, jv.y, jv.z, jv.w};
-            unsigned c2m = cm;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (((cm >> q) & 1u) && (jj[q] <= i || jj[q] >= n)) {
-                    set_err(err, DEV_BAD_INPUT);
-                    c2m &= ~(1u << q);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                lj[q] = ((c2m >> q) & 1u) ? (ident ? jj[q] : label[jj[q]]) : li;
-            unsigned km = 0u;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) km |= (lj[q] != li ? 1u : 0u) << q;
-            return km;
-        };
-        // the row's kept words in walk order: warp prefix of the lanes' counts
-        auto place = [&](unsigned km, int c, int &tot) -> int {
-            int incl = c;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int o = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += o;
-            }
-            tot = __shfl_sync(0xffffffffu, incl, 31);
-            return incl - c;
-        };
-        int cnt = 0, staged = 0;
-        bool spill = false;
-        uint64_t m = kNone;
-        for (int64_t g = a0; g < e_end; g += 128 * G) {
-            uint32_t wv[G];
-            unsigned cm[G];
-            int4 jv[G];
-            if (dense) {
-                // most entries are in range: the indices are read beside the
-                // weights instead of after them
-#pragma unroll
-                for (int u = 0; u < G; ++u) {
-                    wv[u] = wload(g + 128 * u + 4 * lane);
-                    jv[u] = jload(g + 128 * u + 4 * lane, 0u);
-                }
-#pragma unroll
-                for (int u = 0; u < G; ++u) cm[u] = cmask(g + 128 * u + 4 * lane, wv[u]);
-            } else {
-#pragma unroll
-                for (int u = 0; u < G; ++u) wv[u] = wload(g + 128 * u + 4 * lane);
-#pragma unroll
-                for (int u = 0; u < G; ++u) {
-                    cm[u] = cmask(g + 128 * u + 4 * lane, wv[u]);
-                    jv[u] = jload(g + 128 * u + 4 * lane, cm[u]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < G; ++u) {
-                int32_t lj[4];
-                const unsigned km = cm[u] ? keep(cm[u], jv[u], lj) : 0u;
-                if (!__any_sync(0xffffffffu, km != 0u)) continue;
-                const int c = __popc(km);
-                int tot;
-                int p = staged + place(km, c, tot);
-                if (staged + tot > kUpStage) spill = true;
-                const int32_t jj[4] = {jv[u].x, jv[u].y, jv[u].z, jv[u].w};
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (!((km >> q) & 1u)) continue;
-                    const uint32_t wq = (wv[u] >> (8 * q)) & 255u;
-                    const uint64_t k = pk.make(wq, (uint32_t)i, (uint32_t)jj[q]);
-                    atomicAdd(&s_kh[wq], 1u);
-                    m = (k >> 1) < m ? (k >> 1) : m;
-                    min_if_lower(&best[lj[q]], k >> 1);
-                    if (!spill) stage[p++] = k;
-                }
-                staged += tot;
-                cnt += c;
-            }
+        for (int u = 0; u < U; ++u) {
+            j[u] = ok[u] ? __ldg(a.indices + e[u]) : 0;
+            wq[u] = ok[u] ? __ldg(a.w + e[u]) : 0u;
+            li[u] = ok[u] && !a.ident ? a.label[i[u]] : i[u];
         }
-        cnt = __reduce_add_sync(0xffffffffu, cnt);
 #pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) {
-            const uint64_t x = __shfl_xor_sync(0xffffffffu, m, o);
-            m = x < m ? x : m;
+        for (int u = 0; u < U; ++u) {
+            if (ok[u] && (j[u] <= i[u] || j[u] >= a.n)) {
+                set_err(a.err, DEV_BAD_INPUT);
+                ok[u] = false;
+            }
+            lj[u] = ok[u] ? (a.ident ? j[u] : a.label[j[u]]) : li[u];
         }
-        if (cnt == 0) continue;
-        if (lane == 0 && m != kNone) min_if_lower(&best[li], m);
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(cursor, (unsigned long long)cnt);
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (at + (unsigned long long)cnt > cap) {
-            if (lane == 0) set_err(err, DEV_CAPACITY);
-            __syncwarp();
-            continue;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            ok[u] = ok[u] && lj[u] != li[u];
+            cj[u] = ok[u] ? __ldcg(a.best + lj[u]) : 0ull;
+            ci[u] = ok[u] ? __ldcg(a.best + li[u]) : 0ull;
         }
         __syncwarp();
-        if (!spill) {
-            for (int t = lane; t < cnt; t += 32) eout[at + t] = stage[t];
-            __syncwarp();                  // the staging is reused by the next row
-            continue;
-        }
-        // more kept entries than the staging holds: walk again to write them
-        for (int64_t g = a0; g < e_end; g += 128) {
-            const int64_t e = g + 4 * lane;
-            const uint32_t wv = wload(e);
-            const unsigned cm = cmask(e, wv);
-            const int4 jv = jload(e, cm);
-            int32_t lj[4];
-            const unsigned km = cm ? keep(cm, jv, lj) : 0u;
-            if (!__any_sync(0xffffffffu, km != 0u)) continue;
-            const int c = __popc(km);
-            int tot;
-            unsigned long long p = at + (unsigned long long)place(km, c, tot);
-            const int32_t jj[4] = {jv.x, jv.y, jv.z, jv.w};
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if ((km >> q) & 1u)
-                    eout[p++] = pk.make((wv >> (8 * q)) & 255u, (uint32_t)i, (uint32_t)jj[q]);
-            at += (unsigned long long)tot;
+        for (int u = 0; u < U; ++u) {
+            const unsigned bal = __ballot_sync(0xffffffffu, ok[u]);
+            if (!bal) continue;
+            const uint64_t k = a.pk.make(wq[u], (uint32_t)i[u], (uint32_t)j[u]);
+            if (ok[u]) {
+                atomicAdd(&s_kh[wq[u]], 1u);
+                if ((k >> 1) < cj[u]) atomicMin(a.best + lj[u], (unsigned long long)(k >> 1));
+                rec[out + __popc(bal & below)] = k;
+            }
+            // (a row's records are consecutive: one reduction for each run)
+            if (__any_sync(0xffffffffu, ok[u] && (k >> 1) < ci[u]))
+                seg_min_atomic(ok[u], li[u], k >> 1, a.best);
+            out += __popc(bal);
         }
         __syncwarp();
     }
+    if (out == 0) return;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(a.cursor, (unsigned long long)out);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (at + (unsigned long long)out > a.cap) {
+        if (lane == 0) set_err(a.err, DEV_CAPACITY);
+    } else {
+        for (int t = lane; t < out; t += 32) a.eout[at + t] = rec[t];
+    }
+    __syncwarp();                    // the records are written again
+}
+
+// Appends to the warp's records the entries of row i that the lanes' bits m
+// name: bit q is entry e + q of the lane's first load, and every PER bits a
+// load of the warp's further on.  More than CAP at once go 4 bits at a time.
+template <int CAP, int PER, typename Flush>
+__device__ __forceinline__ void up_record(unsigned m, int64_t e, int32_t i, uint64_t *rec,
+                                          int32_t *rrow, int &nrec, Flush flush)
+{
+    static_assert(CAP >= 4 * 32, "a piece of 4 bits fits");
+    const int lane = threadIdx.x & 31;
+    if (!__any_sync(0xffffffffu, m != 0u)) return;
+    unsigned rest = m;
+    int piece = 32;
+    while (true) {
+        const unsigned now = piece < 32 ? rest & ((1u << piece) - 1u) : rest;
+        int incl = __popc(now);
+        int p = -incl;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += o;
+        }
+        const int tot = __shfl_sync(0xffffffffu, incl, 31);
+        if (tot > CAP) {
+            piece = 4;
+            continue;
+        }
+        if (nrec + tot > CAP) {
+            flush(nrec);
+            nrec = 0;
+        }
+        p += nrec + incl;
+        for (unsigned t = now; t; t &= t - 1u, ++p) {
+            const int q = __ffs(t) - 1;
+            rec[p] = (uint64_t)(e + q + (q / PER) * (31 * PER));
+            rrow[p] = i;
+        }
+        nrec += tot;
+        rest &= ~now;
+        if (piece == 32) break;
+        piece += 4;
+        if (piece > 32 || !__any_sync(0xffffffffu, rest != 0u)) break;
+    }
+}
+
+// bits q of m kept for the entries e + q of N that lie in [s, e_end)
+template <int N>
+__device__ __forceinline__ unsigned up_clip(unsigned m, int64_t e, int64_t s, int64_t e_end)
+{
+    if (e >= s && e + N <= e_end) return m;
+    const int64_t a = s - e, b = e_end - e;
+    const int qa = a < 0 ? 0 : (a > N ? N : (int)a);
+    const int qb = b < 0 ? 0 : (b > N ? N : (int)b);
+    constexpr unsigned all = (1u << N) - 1u;
+    return m & (all << qa) & (all >> (N - qb));
+}
+
+// the 16 weights from entry e on, zero outside the array
+__device__ __noinline__ uint4 up_edge_bytes(const uint8_t *w, int64_t e, int64_t nnz)
+{
+    uint32_t t[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+        if (e + q >= 0 && e + q < nnz) t[q >> 2] |= (uint32_t)w[e + q] << (8 * (q & 3));
+    return make_uint4(t[0], t[1], t[2], t[3]);
+}
+
+// A warp per row, 16 weights per lane and load, two loads in flight with the
+// next row's extent; any order and any alignment of the arrays.
+__global__ void __launch_bounds__(kPhThreads, 4)
+k_phase_upper(const __grid_constant__ UpArgs a)
+{
+    constexpr int G = 2;
+    __shared__ unsigned s_kh[256];           // kept entries per weight, this block
+    __shared__ uint64_t rec_all[kPhWarps][kUpRec];
+    __shared__ int32_t row_all[kPhWarps][kUpRec];
+    for (int b = threadIdx.x; b < 256; b += blockDim.x) s_kh[b] = 0u;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    uint64_t *rec = rec_all[threadIdx.x >> 5];
+    int32_t *rrow = row_all[threadIdx.x >> 5];
+    int nrec = 0;
+    const uint32_t c1 = 0x00010001u * (uint32_t)(0x8000 - (a.lo + 1));
+    const uint32_t c2 = 0x00010001u * (uint32_t)(0x7fff - a.hi);
+    const int mis = (int)((uintptr_t)a.w & 15);
+    const int64_t nwarps = (int64_t)gridDim.x * kPhWarps;
+    int64_t i = a.row0 + (int64_t)blockIdx.x * kPhWarps + (threadIdx.x >> 5);
+    int64_t s1 = 0, e1 = 0;
+    if (i < a.row1) {
+        s1 = a.indptr[i];
+        e1 = a.indptr[i + 1];
+    }
+    for (; i < a.row1; i += nwarps) {
+        const int64_t s = s1, e_end = e1;
+        if (i + nwarps < a.row1) {
+            s1 = a.indptr[i + nwarps];
+            e1 = a.indptr[i + nwarps + 1];
+        }
+        if (s < 0 || e_end < s || e_end > a.nnz) {
+            if (lane == 0) set_err(a.err, DEV_BAD_INPUT);
+            continue;
+        }
+        // groups start on 16-byte boundaries of the weights (the first may
+        // start before the array: its loads are made byte by byte)
+        for (int64_t g = s - ((s + mis) & 15); g < e_end; g += 512 * G) {
+            uint4 v[G];
+#pragma unroll
+            for (int u = 0; u < G; ++u) {
+                const int64_t e = g + 512 * u + 16 * lane;
+                v[u] = make_uint4(0u, 0u, 0u, 0u);
+                if (e >= e_end) continue;
+                v[u] = e >= 0 && e + 15 < a.nnz ? __ldg(reinterpret_cast<const uint4 *>(a.w + e))
+                                                : up_edge_bytes(a.w, e, a.nnz);
+            }
+            unsigned m = 0u;
+#pragma unroll
+            for (int u = 0; u < G; ++u) {
+                const unsigned x =
+                    bytes_in_range(v[u].x, c1, c2) | bytes_in_range(v[u].y, c1, c2) << 4 |
+                    bytes_in_range(v[u].z, c1, c2) << 8 | bytes_in_range(v[u].w, c1, c2) << 12;
+                m |= up_clip<16>(x, g + 512 * u + 16 * lane, s, e_end) << (16 * u);
+            }
+            up_record<kUpRec, 16>(m, g + 16 * lane, (int32_t)i, rec, rrow, nrec,
+                                  [&](int c) { up_flush(a, rec, rrow, c, s_kh); });
+        }
+    }
+    up_flush(a, rec, rrow, nrec, s_kh);
     __syncthreads();
     for (int b = threadIdx.x; b < 256; b += blockDim.x)
-        if (s_kh[b]) atomicAdd(&khist[b], (unsigned long long)s_kh[b]);
+        if (s_kh[b]) atomicAdd(&a.khist[b], (unsigned long long)s_kh[b]);
+}
+
+// The last phase: all the weights left, once the components are few.  Of the
+// entries between two components only the least can be in the forest, so
+// none is written: pairs[c * V + d] receives the least key between rows of
+// component c and columns of component d (V of them, numbered in cid), and
+// k_pair_emit makes one word of each pair.  Nearly every entry joins a
+// component to itself, and telling so by gathering the other end's component
+// takes an L2 access per entry (920M entries of 300,000 rows: 4.9 ms, most
+// of it L1 misses; this kernel takes 1.5, 3.1 TB/s of the 5 bytes per entry).  Here the rows are taken component by component (ord,
+// the components of at least kPairMin vertices first): a block holds the
+// component's members as a bitmap in shared memory, an entry costs one
+// shared-memory read, and those that leave the component become records,
+// whose pass offers them to the block's least keys per component.  The rows
+// of the smaller components offer every entry to the pairs themselves.
+// Blocks take shares of the row list that are equal in entries (pre: the
+// rows' first entries in list order), several for each block: a share whose
+// rows mostly leave their component takes up to 2.5 times as long.
+constexpr int kPairThreads = 1024;
+constexpr int kPairWarps = kPairThreads / 32;
+constexpr int kPairMax = 2048;       // components at most
+constexpr int kPairMin = 32;         // vertices from which a bitmap is worth its making
+constexpr int kPairBlocks = 148;     // one per SM
+constexpr int kPairShares = 8;       // per block at most, of at least kPairShareMin entries
+constexpr int64_t kPairShareMin = (int64_t)1 << 17;
+constexpr size_t kPairRecBytes = (size_t)kPairWarps * kPairRec * (sizeof(uint64_t) + sizeof(int32_t));
+constexpr size_t kPairMaxSmem = 220 << 10;
+
+static size_t pair_smem(int32_t n, int V)
+{
+    return kPairRecBytes + (size_t)V * sizeof(uint64_t) + (size_t)(((int64_t)n + 31) / 32) * 4;
+}
+
+struct PairArgs {
+    const int32_t *ord;              // rows, component by component
+    const int64_t *pre;              // n + 1: entries of the rows before
+    const int32_t *size;             // vertices per root
+    const int32_t *off;              // first list place per root of a large component
+    int *share;                      // zeroed: shares taken
+    int shares;
+    const uint16_t *cid;             // component number per vertex
+    unsigned long long *pairs;       // V x V
+    int V;
+};
+
+// The warp's n records: checked, offered to the block's least keys (rows of
+// one component) or, with least null, to the pairs.
+__device__ __noinline__ void pair_flush(const UpArgs &a, const PairArgs &o,
+                                        unsigned long long *least, const uint64_t *rec,
+                                        const int32_t *rrow, int n)
+{
+    constexpr int U = 4;
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        static_assert(kPairRec == 32 * U, "one pass");
+        const int t = 32 * u + lane;
+        if (t >= n) continue;
+        const int64_t e = (int64_t)rec[t];
+        const int32_t i = rrow[t], j = __ldg(a.indices + e);
+        const uint32_t w = __ldg(a.w + e);
+        if (j <= i || j >= a.n) {
+            set_err(a.err, DEV_BAD_INPUT);
+            continue;
+        }
+        const unsigned long long k = a.pk.make(w, (uint32_t)i, (uint32_t)j) >> 1;
+        const int d = o.cid[j];
+        if (least) {
+            if (k < *(volatile unsigned long long *)(least + d)) atomicMin(least + d, k);
+        } else {
+            const int c = o.cid[i];
+            if (c != d) min_if_lower(o.pairs + (int64_t)c * o.V + d, k);
+        }
+    }
+    __syncwarp();                    // the records are written again
+}
+
+__global__ void __launch_bounds__(kPairThreads, 1)
+k_pair_min(const __grid_constant__ UpArgs a, const __grid_constant__ PairArgs o)
+{
+    constexpr int G = 4;
+    extern __shared__ __align__(16) uint8_t pair_smem_raw[];
+    uint64_t *rec_all = reinterpret_cast<uint64_t *>(pair_smem_raw);
+    unsigned long long *least = reinterpret_cast<unsigned long long *>(rec_all + kPairWarps * kPairRec);
+    int32_t *row_all = reinterpret_cast<int32_t *>(least + o.V);
+    uint32_t *bm = reinterpret_cast<uint32_t *>(row_all + kPairWarps * kPairRec);
+    __shared__ int s_next, s_share;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t *rec = rec_all + warp * kPairRec;
+    int32_t *rrow = row_all + warp * kPairRec;
+    const uint32_t c1 = 0x00010001u * (uint32_t)(0x8000 - (a.lo + 1));
+    const uint32_t c2 = 0x00010001u * (uint32_t)(0x7fff - a.hi);
+    const int shares = o.shares;
+    // where share b begins: the first row whose first entry lies in it
+    auto first_row = [&](int b) -> int {
+        if (b >= shares) return a.n;
+        const int64_t tot = o.pre[a.n];
+        const int64_t t = tot / shares * b + tot % shares * b / shares;
+        int lo = 0, hi = a.n;
+        while (lo < hi) {                    // 32 probes at a time
+            const int at = lo + (int)((int64_t)(hi - lo) * lane / 32);
+            const int c = __popc(__ballot_sync(0xffffffffu, o.pre[at] < t));
+            const int last = __shfl_sync(0xffffffffu, at, c ? c - 1 : 0);
+            const int next = __shfl_sync(0xffffffffu, at, c < 32 ? c : 31);
+            if (c < 32) hi = next;
+            if (c) lo = last + 1;
+        }
+        return lo;
+    };
+    const int words = (a.n + 31) / 32;
+    while (true) {
+        if (threadIdx.x == 0) s_share = atomicAdd(o.share, 1);
+        __syncthreads();
+        const int share = shares - 1 - s_share;    // (the small components' rows first)
+        if (share < 0) break;
+        int x = first_row(share);
+        const int x1 = first_row(share + 1);
+        while (x < x1) {
+            // the share's rows of one component, or those of small ones
+            const int32_t v0 = o.ord[x], root = a.label[v0];
+            const int members = o.size[root], c0 = o.off[root], row = o.cid[v0];
+            const bool own = members >= kPairMin;
+            const int xe = own ? min(x1, c0 + members) : x1;
+            auto flush = [&](int c) { pair_flush(a, o, own ? least : nullptr, rec, rrow, c); };
+            if (threadIdx.x == 0) s_next = x;
+            if (own) {
+                for (int b = threadIdx.x; b < words; b += kPairThreads) bm[b] = 0u;
+                for (int b = threadIdx.x; b < o.V; b += kPairThreads) least[b] = kNone;
+                __syncthreads();
+                for (int y = threadIdx.x; y < members; y += kPairThreads) {
+                    const int32_t v = o.ord[c0 + y];
+                    atomicOr(&bm[v >> 5], 1u << (v & 31));
+                }
+            }
+            __syncthreads();
+            // rows by a counter, the next one's extent loaded ahead
+            auto take = [&](int32_t &i, int64_t &s, int64_t &e) -> bool {
+                int y = 0;
+                if (lane == 0) y = atomicAdd(&s_next, 1);
+                y = __shfl_sync(0xffffffffu, y, 0);
+                if (y >= xe) return false;
+                i = o.ord[y];
+                s = a.indptr[i];
+                e = a.indptr[i + 1];
+                return true;
+            };
+            int nrec = 0;
+            int32_t i = 0, i1 = 0;
+            int64_t s = 0, e_end = 0, s1 = 0, e1 = 0;
+            bool more = take(i, s, e_end);
+            while (more) {
+                more = take(i1, s1, e1);
+                if (s < 0 || e_end < s || e_end > a.nnz) {
+                    if (lane == 0) set_err(a.err, DEV_BAD_INPUT);
+                    s = e_end = 0;
+                }
+                const uint32_t span = (uint32_t)(a.n - 1 - i);
+                for (int64_t g = s & ~(int64_t)3; g < e_end; g += 128 * G) {
+                    uint32_t wv[G];
+                    int4 jv[G];
+#pragma unroll
+                    for (int u = 0; u < G; ++u) {
+                        const int64_t e = g + 128 * u + 4 * lane;
+                        wv[u] = 0u;
+                        jv[u] = make_int4(0, 0, 0, 0);
+                        if (e >= e_end) continue;
+                        if (e + 3 < a.nnz) {
+                            wv[u] = __ldg(reinterpret_cast<const uint32_t *>(a.w + e));
+                            jv[u] = __ldg(reinterpret_cast<const int4 *>(a.indices + e));
+                        } else {
+                            int32_t t[4] = {0, 0, 0, 0};
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                if (e + q >= a.nnz) continue;
+                                wv[u] |= (uint32_t)a.w[e + q] << (8 * q);
+                                t[q] = a.indices[e + q];
+                            }
+                            jv[u] = make_int4(t[0], t[1], t[2], t[3]);
+                        }
+                    }
+                    unsigned m = 0u;
+#pragma unroll
+                    for (int u = 0; u < G; ++u) {
+                        unsigned x = up_clip<4>(bytes_in_range(wv[u], c1, c2), g + 128 * u + 4 * lane, s, e_end);
+                        const int32_t jj[4] = {jv[u].x, jv[u].y, jv[u].z, jv[u].w};
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            // (a column outside (i, n) is recorded: the records'
+                            // pass reports it)
+                            const bool in = (uint32_t)(jj[q] - i - 1) < span;
+                            const int32_t j = in ? jj[q] : i;
+                            if (own && in && ((bm[j >> 5] >> (j & 31)) & 1u)) x &= ~(1u << q);
+                        }
+                        m |= x << (4 * u);
+                    }
+                    up_record<kPairRec, 4>(m, g + 4 * lane, i, rec, rrow, nrec, flush);
+                }
+                i = i1;
+                s = s1;
+                e_end = e1;
+            }
+            flush(nrec);
+            __syncthreads();
+            if (own)
+                for (int b = threadIdx.x; b < o.V; b += kPairThreads)
+                    if (least[b] != kNone) min_if_lower(o.pairs + (int64_t)row * o.V + b, least[b]);
+            __syncthreads();                     // the bitmap, least and the counters start anew
+            x = xe;
+        }
+        __syncthreads();
+    }
+}
+
+// One word per pair of components with an entry between them, offered to both.
+__global__ void k_pair_emit(const unsigned long long *pairs, int V, const int32_t *roots,
+                            uint64_t *eout, unsigned long long *cursor, unsigned long long *best)
+{
+    const int c = blockIdx.x;
+    for (int d = c + 1 + threadIdx.x; d < V; d += blockDim.x) {
+        const uint64_t x = pairs[(int64_t)c * V + d], y = pairs[(int64_t)d * V + c];
+        const uint64_t m = x < y ? x : y;
+        if (m == kNone) continue;
+        eout[atomicAdd(cursor, 1ull)] = m << 1;
+        min_if_lower(best + roots[c], m);
+        min_if_lower(best + roots[d], m);
+    }
+}
+
+// The row list of k_pair_min: vertices per root; the components' numbers and
+// the large ones' sizes (a scan then places them); the list with its rows'
+// lengths.
+// (Lanes with the same root share an atomic: the components are few.)
+__global__ void k_pair_count(const int32_t *label, int32_t n, int32_t *size)
+{
+    for (int64_t vb = (int64_t)blockIdx.x * blockDim.x; vb < n; vb += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = vb + threadIdx.x;
+        const int32_t r = v < n ? label[v] : -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, r);
+        if (r >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&size[r], __popc(peers));
+    }
+}
+
+// (found: zeroed; V: the components there are)
+__global__ void k_pair_number(const int32_t *size, int32_t n, int V, int32_t *large, int32_t *number,
+                              int32_t *roots, int32_t *found)
+{
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
+         r += (int64_t)gridDim.x * blockDim.x) {
+        large[r] = size[r] >= kPairMin ? size[r] : 0;
+        if (size[r] == 0) continue;
+        const int c = atomicAdd(found, 1);
+        if (c < V) roots[c] = (int32_t)r;
+        number[r] = min(c, V - 1);
+    }
+}
+
+// given: zeroed, the places given out per root; *others likewise for the
+// small components' rows, which come after the *n_large others.  A
+// component's rows come in about ascending order, so that later rows' keys
+// are seldom the lower ones.
+__global__ void k_pair_place(const int64_t *indptr, const int32_t *label, int32_t n, int64_t nnz,
+                             const int32_t *size, const int32_t *off, const int64_t *n_large,
+                             const int32_t *number, int32_t *given, int32_t *others, int32_t *ord,
+                             int32_t *len, uint16_t *cid)
+{
+    const int lane = threadIdx.x & 31;
+    for (int64_t vb = (int64_t)blockIdx.x * blockDim.x; vb < n; vb += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = vb + threadIdx.x;
+        const int32_t r = v < n ? label[v] : -1;
+        const bool large = r >= 0 && size[r] >= kPairMin;
+        const unsigned peers = __match_any_sync(0xffffffffu, large ? r : r >= 0 ? -2 : -1);
+        const int lead = __ffs(peers) - 1, cnt = __popc(peers);
+        int base = 0;
+        if (lane == lead && r >= 0)
+            base = large ? off[r] + atomicAdd(&given[r], cnt)
+                         : (int)*n_large + atomicAdd(others, cnt);
+        base = __shfl_sync(0xffffffffu, base, lead);
+        if (v < n) {
+            const int at = base + __popc(peers & ((1u << lane) - 1u));
+            const int64_t s = indptr[v], e = indptr[v + 1];
+            ord[at] = (int32_t)v;
+            // (a bad extent counts as empty here; its row reports it)
+            len[at] = (s < 0 || e < s || e > nnz || e - s > 0x7fffffff) ? 0 : (int32_t)(e - s);
+            cid[v] = (uint16_t)number[r];
+        }
+    }
 }
 
 // One phase: the entries with weight bucket in (lo, hi] of rows [r0, r1);
@@ -1110,6 +1437,7 @@ struct Phase {
     int64_t r0, r1;
     int slot;
     int ident;            // the labels are still the identity (no merges yet)
+    int pairs = 0;        // components, in the phase that takes their pairs (k_pair_min)
 };
 
 // Phase ranges (lo, hi] of weight buckets: cut the bucket histogram at the
@@ -2146,10 +2474,12 @@ struct Engine {
     // Phases in order with a host read after each build (the final
     // clustering): the edge array holds a phase's usual output, and a phase
     // whose kept entries overflow it is discarded and redone as the pieces
-    // split() cuts from the build's per-weight kept counts, in order.
+    // split() cuts from the build's per-weight kept counts, in order.  From
+    // at most pair_max components on, one phase takes the rest by pairs of
+    // components.
     template <typename Build, typename Split>
     int run_phased_retry(Pack pk, std::vector<Phase> plan, Build build, Split split,
-                         cudaStream_t st)
+                         int64_t pair_max, cudaStream_t st)
     {
         int64_t V = V0, n_mst = 0;
         size_t q = 0;
@@ -2192,12 +2522,13 @@ struct Engine {
             // few most entries join a component to itself, so the remaining
             // phases would keep few words each; a merged phase that does
             // overflow the edge array is redone in pieces like any other.
-            if (q + 1 < plan.size() && V * kMergeBelow <= V0) {
+            const bool pairs = V <= pair_max && 2 * V * V <= Emax;
+            if (q < plan.size() && (pairs || (q + 1 < plan.size() && V * kMergeBelow <= V0))) {
                 bool full = true;
                 for (size_t r = q; r < plan.size(); ++r)
                     full = full && plan[r].r0 == 0 && plan[r].r1 == V0;
                 if (full) {
-                    const Phase rest{plan[q].lo, plan.back().hi, 0, V0, -1, 0};
+                    const Phase rest{plan[q].lo, plan.back().hi, 0, V0, -1, 0, pairs ? (int)V : 0};
                     plan.resize(q);
                     plan.push_back(rest);
                 }
@@ -2630,12 +2961,39 @@ static int split_final_phase(const Phase &ph, const unsigned long long kh[256], 
     return EACB_OK;
 }
 
+// Matrices of this many entries read the number of components after each
+// phase, to end with a phase by pairs of components (k_pair_min: its rows'
+// members are a bitmap in shared memory, up to about 1.2 million points);
+// smaller ones queue all phases with no read between them.  (1.7M entries:
+// 0.65 ms queued, 0.70 by pairs; 4.2M: 0.77 either way; 12.6M: 1.14 and
+// 0.95.)
+constexpr int64_t kPairEntries = (int64_t)1 << 22;
+
+static bool pair_phase(int32_t n, int64_t nnz)
+{
+    return nnz >= kPairEntries && pair_smem(n, kPairMax) <= kPairMaxSmem;
+}
+
+struct PairList {
+    int32_t *ord, *len, *roots, *found;
+    int64_t *pre;
+    uint16_t *cid;
+};
+
 static void carve_final(Carver &c, int32_t n, int64_t nnz, Engine *g, int64_t **hist,
-                        int32_t **cmin)
+                        int32_t **cmin, PairList *pl)
 {
     *g = Engine::carve(c, n, final_edge_cap(n, nnz));
     *hist = c.take<int64_t>(256);
     *cmin = c.take<int32_t>(n);
+    *pl = PairList{};
+    if (!pair_phase(n, nnz)) return;
+    pl->ord = c.take<int32_t>(n);
+    pl->len = c.take<int32_t>(n);
+    pl->roots = c.take<int32_t>(kPairMax);
+    pl->found = c.take<int32_t>(3);      // components numbered, small ones' rows, shares taken
+    pl->pre = c.take<int64_t>((int64_t)n + 1);
+    pl->cid = c.take<uint16_t>(n);
 }
 
 extern "C" size_t eacb_final_clustering_workspace_size(int32_t n, int64_t nnz)
@@ -2644,7 +3002,8 @@ extern "C" size_t eacb_final_clustering_workspace_size(int32_t n, int64_t nnz)
     Engine g;
     int64_t *h;
     int32_t *m;
-    carve_final(c, n, nnz, &g, &h, &m);
+    PairList pl;
+    carve_final(c, n, nnz, &g, &h, &m, &pl);
     return c.off;
 }
 
@@ -2665,7 +3024,8 @@ extern "C" int eacb_final_clustering(const int64_t *indptr, const int32_t *indic
     Engine g;
     int64_t *hist;
     int32_t *cmin;
-    carve_final(c, n, nnz, &g, &hist, &cmin);
+    PairList pl;
+    carve_final(c, n, nnz, &g, &hist, &cmin, &pl);
     if (c.overflow) return EACB_ERR_WORKSPACE;
     g.kind = 1;
     if ((s = g.reset(st))) return s;
@@ -2678,23 +3038,43 @@ extern "C" int eacb_final_clustering(const int64_t *indptr, const int32_t *indic
     if ((s = g.read_hist(st, wh))) return s;
     std::vector<Phase> phases;
     plan_final_phases(wh, n, phases);
-    unsigned long long wtot = 0;
-    for (int b = 0; b < 256; ++b) wtot += wh[b];
-    // a phase whose range holds over a quarter of the entries reads every
-    // 16-byte run of indices anyway
-    auto dense = [&](const Phase &ph) -> int {
-        unsigned long long in = 0;
-        for (int b = ph.lo + 1; b <= ph.hi; ++b) in += wh[b];
-        return 4 * in > wtot ? 1 : 0;
-    };
     auto build = [&](const Phase &ph) -> int {
         if (nnz == 0) return EACB_OK;
         ProfScope ps(PROF_PHASE, st);
-        k_phase_upper<<<grid_for((ph.r1 - ph.r0) * 32, kPhThreads), kPhThreads, 0, st>>>(
-            indptr, indices, diassoc, n, nnz, ph.lo, ph.hi, dense(ph), ph.ident, ph.r0, ph.r1,
-            g.label, pk, g.ea,
-            (unsigned long long *)&g.cnt[C_CURSOR], (unsigned long long)g.Emax, g.best, g.hist,
-            g.err);
+        const UpArgs ua{indptr, indices, diassoc, n, nnz, ph.lo, ph.hi, ph.ident, ph.r0, ph.r1,
+                        g.label, pk, g.ea, (unsigned long long *)&g.cnt[C_CURSOR],
+                        (unsigned long long)g.Emax, g.best, g.hist, g.err};
+        if (ph.pairs) {
+            const unsigned gn = grid_for(n, 256, 148 * 8);
+            const int64_t V = ph.pairs;
+            // the pairs at the end of the edge array, their words at its start
+            unsigned long long *pairs = (unsigned long long *)g.ea + (g.Emax - V * V);
+            EACB_CUDA(cudaMemsetAsync(pairs, 0xff, sizeof(uint64_t) * V * V, st));
+            EACB_CUDA(cudaMemsetAsync(g.flag, 0, sizeof(int32_t) * n, st));
+            EACB_CUDA(cudaMemsetAsync(pl.found, 0, 3 * sizeof(int32_t), st));
+            k_pair_count<<<gn, 256, 0, st>>>(g.label, n, g.flag);
+            EACB_CHECK_LAUNCH();
+            k_pair_number<<<gn, 256, 0, st>>>(g.flag, n, (int)V, g.act, cmin, pl.roots, pl.found);
+            EACB_CHECK_LAUNCH();
+            int t = scan_launch<int32_t, int32_t>(g.act, g.pos, n, 0, &g.cnt[C_AUX1], g.scan, st);
+            if (t) return t;
+            EACB_CUDA(cudaMemsetAsync(g.act, 0, sizeof(int32_t) * n, st));
+            k_pair_place<<<gn, 256, 0, st>>>(indptr, g.label, n, nnz, g.flag, g.pos, &g.cnt[C_AUX1],
+                                            cmin, g.act, pl.found + 1, pl.ord, pl.len, pl.cid);
+            EACB_CHECK_LAUNCH();
+            if ((t = scan_launch<int32_t, int64_t>(pl.len, pl.pre, n, 0, &pl.pre[n], g.scan, st)))
+                return t;
+            EACB_CUDA(allow_max_dyn_smem(k_pair_min));
+            const int shares = (int)std::min<int64_t>(
+                kPairBlocks * kPairShares, std::max<int64_t>(kPairBlocks, nnz / kPairShareMin));
+            k_pair_min<<<kPairBlocks, kPairThreads, pair_smem(n, (int)V), st>>>(
+                ua, PairArgs{pl.ord, pl.pre, g.flag, g.pos, pl.found + 2, shares, pl.cid, pairs, (int)V});
+            EACB_CHECK_LAUNCH();
+            k_pair_emit<<<(unsigned)V, 256, 0, st>>>(pairs, (int)V, pl.roots, g.ea,
+                                                     (unsigned long long *)&g.cnt[C_CURSOR], g.best);
+        } else {
+            k_phase_upper<<<grid_for((ph.r1 - ph.r0) * 32, kPhThreads, 148 * 4), kPhThreads, 0, st>>>(ua);
+        }
         EACB_CHECK_LAUNCH();
         // compulsory reads: row pointers and labels (12 B per row), column and
         // weight (5 B per entry; a row-range phase is counted in proportion to
@@ -2707,10 +3087,12 @@ extern "C" int eacb_final_clustering(const int64_t *indptr, const int32_t *indic
     auto split = [&](const Phase &ph, const unsigned long long kh[256], std::vector<Phase> &out) {
         return split_final_phase(ph, kh, g.Emax, indptr, n, hip, st, out);
     };
-    if (g.Emax >= nnz) {
+    // (the pairs' phase reads the arrays in 4-entry vectors)
+    const bool vec = ((uintptr_t)indices & 15) == 0 && ((uintptr_t)diassoc & 3) == 0;
+    if (g.Emax >= nnz && !pl.ord) {
         if ((s = g.run_phased(pk, phases, build, st))) return s;
     } else {
-        if ((s = g.run_phased_retry(pk, phases, build, split, st))) return s;
+        if ((s = g.run_phased_retry(pk, phases, build, split, pl.ord && vec ? kPairMax : 0, st))) return s;
     }
     // 2. lifetime rule on the weight histogram
     static_assert(sizeof(CutPlan) == (C_COUNT - C_PLAN) * sizeof(int64_t), "the plan is read with the counts");

@@ -206,3 +206,52 @@ def test_capped_rows(n, P, K, cap):
         a, e = ip[i], ip[i + 1]
         assert np.array_equal(ind[a:e].cpu().numpy(), cols), i
         assert np.array_equal(dat[a:e].cpu().numpy(), counts), i
+
+
+@pytest.mark.parametrize("order", ["ascending", "shuffled"])
+@pytest.mark.parametrize("off_w,off_i", [(0, 0), (4, 0), (3, 1)])
+def test_final_clustering_pairs(order, off_w, off_i):
+    """The last phase by pairs of components: large and small components
+    (around the 32 vertices that give one a bitmap), single points, columns in
+    any order, arrays off their vector boundaries, entries that are not
+    between two components' least; against the oracle.  A column outside
+    (row, n) in that phase is refused."""
+    import torch
+    import oracle
+    from masters_final_b200._lib import EACBError
+    from masters_final_b200.EAC.eac import sp_sl_lifetime_csr
+    rng = np.random.default_rng(5)
+    sizes = [700, 600, 500, 400, 300, 200, 33, 32, 31, 20, 9, 4, 2, 1, 1] + [64] * 10
+    n = sum(sizes)
+    group = rng.permutation(np.repeat(np.arange(len(sizes)), sizes))
+    a, b = np.triu_indices(n, 1)
+    keep = (group[a] == group[b]) | (group[a] + group[b] > 1)        # 0 and 1 share no entry
+    a, b = a[keep], b[keep]
+    assert a.size >= 1 << 22
+    inside = group[a] == group[b]
+    w = np.where(inside, rng.integers(1, 60, a.size), rng.integers(100, 220, a.size)).astype(np.uint8)
+    small = np.isin(group[a], np.nonzero(np.array(sizes) < 64)[0])
+    w[inside & small] = 2                                            # whole after the first phase
+    indptr = np.zeros(n + 1, dtype=np.int64)
+    np.cumsum(np.bincount(a, minlength=n), out=indptr[1:])
+    cols, wts = b.astype(np.int32), w.copy()
+    if order == "shuffled":
+        p = np.lexsort((rng.random(a.size), a))
+        cols, wts = cols[p], wts[p]
+
+    def dev(x, off):
+        t = torch.empty(x.size + off, dtype=getattr(torch, x.dtype.name), device="cuda")[off:]
+        t.copy_(torch.from_numpy(x))
+        return t
+    wd, cd = dev(wts, off_w), dev(cols, off_i)
+    for P in (219, 250):
+        nc, labels = sp_sl_lifetime_csr(indptr, cd, wd, n, P)
+        nc2, lab2 = oracle.sp_sl_lifetime(n, a.astype(np.int64), b.astype(np.int64), w, P)
+        assert nc == nc2
+        if nc > 1:
+            assert np.array_equal(labels, lab2)
+    at = int(np.nonzero(wts >= 210)[0][1000])
+    for bad in (0, n):
+        cd[at] = bad
+        with pytest.raises(EACBError):
+            sp_sl_lifetime_csr(indptr, cd, wd, n, 219)
