@@ -40,6 +40,7 @@
 #include "eacb_common.cuh"
 #include "scan_impl.cuh"
 #include "members.cuh"
+#include "tcgen05.cuh"
 
 #include <cuda_fp16.h>
 
@@ -123,6 +124,8 @@ struct CoWS {
     uint8_t *pbuf;        // pair counts of the count pass's tiles, read by the fill
     unsigned long long *pused;
     int64_t *islot;       // per pair-tile item: its place in pbuf (-1: none)
+    int32_t *left;        // pair-tile items counted by comparison
+    int *left_n;
     ScanScratch scan;
     int64_t ntiles, nbr_cap, pcap, nitems_max;
     int32_t Q;            // half2 words per point in lt
@@ -163,6 +166,8 @@ struct CoWS {
         w.pbuf = c.take<uint8_t>(w.pcap);
         w.pused = c.take<unsigned long long>(1);
         w.islot = c.take<int64_t>(w.nitems_max);
+        w.left = c.take<int32_t>(w.nitems_max);
+        w.left_n = c.take<int>(1);
         w.scan = ScanScratch::carve(c, m + 1 > n ? m + 1 : n, w.err);
         return w;
     }
@@ -605,10 +610,11 @@ k_rows_capped(TailCtx tc, const int32_t *order, const int32_t *rows, const int *
 // of every cluster (any partition) that holds one of its rows, cut to the
 // columns above the group's first row; every column that co-occurs with a
 // row of the group lies in it.  The count of a pair (i, j) is then a
-// comparison of the two label vectors: with the labels in FP16 (exact below
-// 2048; -1 and padding are NaN, which equals nothing) two partitions take one
-// HSET2 and one HADD2, and a 128 x 128 tile of pairs runs as a register-
-// blocked product with no atomics and no scattered loads.  A group takes the
+// comparison of the two label vectors, 128 x 128 pairs at a time, with no
+// atomics and no scattered loads: on the tensor cores as a product of one-hot
+// rows (k_pairs_tc), or with the labels as FP16 bit patterns (below 2048; -1
+// and padding are NaN, which equals nothing), two partitions by one HSET2 and
+// one HADD2 (k_pairs).  A group takes the
 // tiles when their compare work (rows x |N(g)| x partition pairs) is at most
 // `ratio` times the member visits the streaming kernels would spend on its
 // rows; the others, and every row over its capacity, stay on the streaming
@@ -616,10 +622,10 @@ k_rows_capped(TailCtx tc, const int32_t *order, const int32_t *rows, const int *
 
 __device__ __forceinline__ uint32_t label_half(int32_t l)
 {
-    return l >= 0 ? (uint32_t)__half_as_ushort(__int2half_rn(l)) : 0x7e00u;    // NaN
+    return l >= 0 ? (uint32_t)l : 0x7e00u;    // equal as halves when equal as bits; NaN
 }
 
-// lt[i*Q + w]: partitions (2w, 2w+1) of point i as a half2 (low half first)
+// lt[i*Q + w]: the labels of partitions (2w, 2w+1) of point i (low half first)
 __global__ void k_labels_f16(const int32_t *labels, int32_t n, int32_t P, int32_t Q,
                              uint32_t *lt)
 {
@@ -817,6 +823,8 @@ struct PairCtx {
     int64_t pcap;
     unsigned long long *pused;
     int64_t *islot;
+    int32_t *left;            // items k_pairs_tc leaves to the comparison
+    int *left_n;
 };
 
 // Column c of a tile sits at slot 8 (c % 16) + c / 16, so that the eight
@@ -846,9 +854,12 @@ __device__ __forceinline__ void load_pairs(uint32_t *s, const int32_t *idx, cons
 // Thread (tx, ty) of a 16 x 16 grid owns rows 8ty..8ty+7 and columns tx +
 // 16b (b = 0..7) of each tile.  A row's 16 consecutive columns 16b..16b+15
 // are then one per lane of a half-warp: a ballot places its kept entries, and
-// the half-warp writes them to consecutive positions with one store.
+// the half-warp writes them to consecutive positions with one store.  (With 8
+// consecutive columns per lane and a scan of the lanes' counts the stores
+// scatter: 7.3 ms for 3.9.)
 // COUNT: distinct columns per row -> rowcnt, rowflag (and the first
-// partition's overflow check).  FILL: the kept entries at indptr[i].
+// partition's overflow check), for the items k_pairs_tc left.  FILL: the kept
+// entries at indptr[i].
 template <bool FILL>
 __global__ void __launch_bounds__(kPairThreads, 2)
 k_pairs(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr,
@@ -870,8 +881,8 @@ k_pairs(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr,
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
         __syncthreads();
-        const int64_t t = s_item;
-        if (t >= nitems) break;
+        if (s_item >= (FILL ? nitems : *pc.left_n)) break;
+        const int64_t t = FILL ? s_item : pc.left[s_item];
         int glo = 0, ghi = K;                       // item0[glo] <= t < item0[ghi]
         while (ghi - glo > 1) {
             const int m = (glo + ghi) >> 1;
@@ -1055,6 +1066,316 @@ k_pairs(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr,
     }
 }
 
+// The count pass on the tensor cores.  A row block's labels take few distinct
+// clusters (its rows share one in the row-order partition and neighbour each
+// other), so its 128 rows, as one-hot E4M3 rows over just those clusters, are
+// some hundred columns wide; a tile of 128 columns' points in the same
+// clusters' columns makes the pair counts one 128 x 128 product, exact in
+// FP32.  A bitmap of the row block's clusters with running counts turns a
+// label into its column.  The rows' operand is built once per item; per tile
+// the columns' operand is cleared and written while the last tile's counts
+// are read from the other accumulator, and both wait for its product.
+// Bound by the instructions that turn 128 x P labels into one-hot bytes and by
+// the two barriers around them (the product itself takes a tenth of the
+// time).  The count pass of 300,000 points and 100 partitions (545 cluster
+// columns on average) took 9.1 ms by comparison and takes 4.05; 4.56 with 16
+// warps instead of 32.  An item whose operands do not fit shared memory (more
+// than about 700 cluster columns) is left to the comparison, and so is every
+// item when P * K passes the cluster map.
+constexpr int kTcPairThreads = 1024;
+constexpr int kTcPairSmem = 216 * 1024;
+constexpr int64_t kTcMapBits = 1 << 17;          // P * K at most
+constexpr int kTcPairCols = 2 * kPT;             // TMEM columns: two accumulators
+constexpr int kTcUnits = 4;                      // of 8 partitions, per thread at most
+
+// E4M3 x E4M3 -> FP32, both K-major, 128 x 128
+constexpr uint32_t kTcPairIdesc =
+    (1u << 4) | ((uint32_t)(kPT >> 3) << 17) | ((uint32_t)(kPT >> 4) << 24);
+
+__device__ __forceinline__ void mma_e4m3(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                         uint32_t idesc, uint32_t accumulate)
+{
+    const uint32_t z = 0;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(
+            tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(z), "r"(z), "r"(z), "r"(z));
+}
+
+// Labels of 128 points, 8 partitions per thread and unit: lane l of warp w
+// takes row l % 8 of row group w % 16 and partitions 8 (l / 8 + 4 (w / 16) +
+// 8 u) .. + 7, so that a warp's one-hot bytes fall into few equal banks.
+struct TcLabels {
+    uint4 x[kTcUnits];
+    __device__ __forceinline__ static int chunk()
+    {
+        return ((threadIdx.x & 31) >> 3) + 4 * (threadIdx.x >> 9);
+    }
+    __device__ __forceinline__ void load(const uint32_t *lt, int Q, int32_t i)
+    {
+#pragma unroll
+        for (int u = 0; u < kTcUnits; ++u) {
+            const int c = chunk() + 8 * u;
+            x[u] = i >= 0 && 4 * c < Q
+                       ? __ldg(reinterpret_cast<const uint4 *>(lt + (int64_t)i * Q) + c)
+                       : make_uint4(0x7e007e00u, 0x7e007e00u, 0x7e007e00u, 0x7e007e00u);
+        }
+    }
+    // f(bit) with bit = p * K + label for each label there is
+    template <typename F> __device__ __forceinline__ void each(int Q, int K, F f) const
+    {
+        int pK = 8 * chunk() * K;
+#pragma unroll
+        for (int u = 0; u < kTcUnits; ++u, pK += 64 * K) {
+            if (4 * (4 * (int)(threadIdx.x >> 9) + 8 * u) >= Q) break;   // uniform: none in the warp
+            const uint32_t w[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int l = (int)((w[e >> 1] >> (16 * (e & 1))) & 0xffffu);
+                if (l < K) f(pK + e * K + l);
+            }
+        }
+    }
+};
+
+// 16 accumulator columns of the warp's 32 TMEM lanes (one per thread)
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
+{
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__global__ void __launch_bounds__(kTcPairThreads, 1)
+k_pairs_tc(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr, int32_t *rowcnt,
+           int32_t *rowflag, int *queue, int *err)
+{
+    extern __shared__ __align__(128) uint8_t tsm[];
+    const int32_t Q = pc.Q, K = pc.K;
+    const int words = (int)(((int64_t)tc.P * K + 31) >> 5);
+    uint2 *map = reinterpret_cast<uint2 *>(tsm);         // (clusters, their number before, less 1)
+    uint8_t *sA = tsm + (((size_t)words * sizeof(uint2) + 127) & ~(size_t)127);
+    __shared__ int32_t s_row[kPT];
+    __shared__ __align__(16) int32_t s_col[2][kPT];      // (read four at a time)
+    __shared__ int s_cnt[kPT];
+    __shared__ int64_t s_slot;
+    __shared__ int s_item, s_c0;
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_slot;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r8 = 8 * (warp & 15) + (lane & 7);         // the row of this thread's labels
+    const int wq = warp & 3, cq = warp >> 2;             // accumulator lanes and columns it reads
+    const int row = 32 * wq + lane;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_addr(&tmem_slot)),
+                     "r"(kTcPairCols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    const int pr = *pc.prow;
+    const int64_t nitems = pc.item0[K];
+    uint32_t phase = 0;
+    bool ok = true;
+    while (ok) {
+        __syncthreads();                                 // the last item is done with
+        if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
+        __syncthreads();
+        const int64_t t = s_item;
+        if (t >= nitems) break;
+        int glo = 0, ghi = K;                            // item0[glo] <= t < item0[ghi]
+        while (ghi - glo > 1) {
+            const int m = (glo + ghi) >> 1;
+            if (pc.item0[m] <= t) glo = m; else ghi = m;
+        }
+        const int g = glo;
+        const int64_t gb = pc.S[((int64_t)pr * K + g) * pc.ntiles];
+        const int64_t size = pc.S[((int64_t)pr * K + g + 1) * pc.ntiles] - gb;
+        const int64_t r0 = (t - pc.item0[g]) * kPT;
+        const int nrow = (int)(size - r0 < kPT ? size - r0 : kPT);
+        const int32_t *nb = pc.nbr + pc.grp_off[g];
+        const int32_t len = pc.grp_len[g];
+        // ---- the row block's clusters and their columns -------------------
+        TcLabels lab;
+        lab.load(pc.lt, Q, r8 < nrow ? pc.members[gb + r0 + r8] : -1);
+        for (int w = threadIdx.x; w < words; w += kTcPairThreads) map[w] = make_uint2(0u, 0u);
+        if (threadIdx.x < kPT) {
+            s_row[threadIdx.x] = (int)threadIdx.x < nrow ? pc.members[gb + r0 + threadIdx.x] : -1;
+            s_cnt[threadIdx.x] = 0;
+        }
+        __syncthreads();
+        lab.each(Q, K, [&](int bit) {
+            const uint32_t b = 1u << (bit & 31);
+            if (!(*(volatile uint32_t *)&map[bit >> 5].x & b)) atomicOr(&map[bit >> 5].x, b);
+        });
+        __syncthreads();
+        const int per = (words + kTcPairThreads - 1) / kTcPairThreads;
+        const int w0 = min(words, (int)threadIdx.x * per), w1 = min(words, w0 + per);
+        int64_t mine = 0, total;
+        for (int w = w0; w < w1; ++w) mine += __popc(map[w].x);
+        int64_t run = block_excl_sum_shfl<kTcPairThreads>(mine, total);
+        for (int w = w0; w < w1; ++w) {
+            map[w].y = (uint32_t)run - 1u;
+            run += __popc(map[w].x);
+        }
+        const int KB = total < 32 ? 32 : (int)((total + 31) & ~(int64_t)31);
+        uint8_t *sB = sA + (size_t)kPT * KB;
+        if ((sB - tsm) + (int64_t)kPT * KB > kTcPairSmem) {
+            // too many clusters: the comparison takes the item
+            if (threadIdx.x == 0) pc.left[atomicAdd(pc.left_n, 1)] = (int32_t)t;
+            continue;
+        }
+        if (threadIdx.x == 0) {
+            int a = 0, b = len;
+            const int32_t first = s_row[0];
+            while (a < b) {
+                const int m = (a + b) >> 1;
+                if (nb[m] > first) b = m; else a = m + 1;
+            }
+            s_c0 = a;
+            // a place for the item's counts, which the fill reads
+            const int64_t need = (int64_t)((len - a + kPT - 1) / kPT) * kPairThreads * 64;
+            int64_t at = -1;
+            if (need > 0) {
+                at = (int64_t)atomicAdd(pc.pused, (unsigned long long)need);
+                if (at + need > pc.pcap) at = -1;
+            }
+            pc.islot[t] = at;
+            s_slot = at;
+        }
+        for (int v = threadIdx.x; v < kPT * KB / 16; v += kTcPairThreads)
+            reinterpret_cast<uint4 *>(sA)[v] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();                                 // map, s_c0 and the cleared rows
+        // one-hot bytes of this thread's labels into rows of KB columns: 8
+        // rows x 16 bytes per core matrix, core matrices along K first
+        const uint32_t rbase = (uint32_t)((r8 >> 3) * (KB >> 4) * 128 + (r8 & 7) * 16);
+        auto onehot = [&](uint8_t *dst) {
+            lab.each(Q, K, [&](int bit) {
+                const uint2 m = map[bit >> 5];
+                // the word's bits up to the label's, that one on top
+                const uint32_t y = __funnelshift_l(0u, m.x, ~(uint32_t)bit);
+                if ((int32_t)y >= 0) return;
+                const uint32_t k = m.y + (uint32_t)__popc(y);
+                dst[rbase + k + (k >> 4) * 112] = 0x38;              // 1.0, at (k / 16) 128 + k % 16
+            });
+        };
+        onehot(sA);
+        const int c0 = s_c0;
+        const int64_t slot = s_slot;
+        const int tiles = (len - c0 + kPT - 1) / kPT;
+        const int32_t ri = s_row[row] >= 0 ? s_row[row] : 0x7fffffff;
+        int kept = 0;
+        // tile ci's counts: distinct columns of the thread's row, and the
+        // bytes for the fill
+        auto counts = [&](int ci) {
+            float v[16];
+            tmem_ld16(tmem + ((uint32_t)(32 * wq) << 16) + (uint32_t)(kPT * (ci & 1) + 16 * cq), v);
+            const int4 *cols = reinterpret_cast<const int4 *>(&s_col[ci & 1][16 * cq]);
+            uint32_t out[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int4 cj = cols[q];
+                kept += (cj.x > ri && v[4 * q] > 0.f) + (cj.y > ri && v[4 * q + 1] > 0.f) +
+                        (cj.z > ri && v[4 * q + 2] > 0.f) + (cj.w > ri && v[4 * q + 3] > 0.f);
+                // (below 256: the low byte of v + 2^23)
+                uint32_t b[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) b[e] = __float_as_uint(v[4 * q + e] + 8388608.f);
+                out[q] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040),
+                                     0x5410);
+            }
+            if (slot >= 0) {
+                // (the fill's threads: 8 columns of one residue, 8 rows)
+                uint8_t *dst = pc.pbuf + slot +
+                               ((int64_t)ci * kPairThreads + (row >> 3) * 16 + 2 * cq) * 64 + (row & 7) * 8;
+                *reinterpret_cast<uint2 *>(dst) = make_uint2(out[0], out[1]);
+                *reinterpret_cast<uint2 *>(dst + 64) = make_uint2(out[2], out[3]);
+            }
+        };
+        // the point of tile ci's operand row s: columns in slot order
+        auto column = [&](int ci, int s) -> int32_t {
+            const int at = c0 + ci * kPT + (s >> 3) + 16 * (s & 7);
+            return ci < tiles && at < len ? nb[at] : -1;
+        };
+        lab.load(pc.lt, Q, column(0, r8));
+        for (int ci = 0; ci < tiles; ++ci) {
+            for (int v = threadIdx.x; v < kPT * KB / 16; v += kTcPairThreads)
+                reinterpret_cast<uint4 *>(sB)[v] = make_uint4(0u, 0u, 0u, 0u);
+            if (threadIdx.x < kPT) s_col[ci & 1][threadIdx.x] = column(ci, threadIdx.x);
+            __syncthreads();
+            onehot(sB);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            tc_fence_before();
+            __syncthreads();
+            if (threadIdx.x == kTcPairThreads - 32) {
+                tc_fence_after();
+                const uint32_t sbo = 8u * (uint32_t)KB;
+                for (int s = 0; s < KB / 32; ++s)
+                    mma_e4m3(tmem + (uint32_t)(kPT * (ci & 1)), umma_desc(sA + s * 256, 128, sbo),
+                             umma_desc(sB + s * 256, 128, sbo), kTcPairIdesc, s > 0 ? 1u : 0u);
+                mma_commit(&bar);
+            }
+            __syncwarp();
+            lab.load(pc.lt, Q, column(ci + 1, r8));
+            if (ci > 0) counts(ci - 1);
+            const bool got = mbar_wait(&bar, phase);
+            phase ^= 1u;
+            tc_fence_after();
+            if (__syncthreads_or(!got)) {
+                if (threadIdx.x == 0) set_err(err, DEV_SPIN_LIMIT);
+                ok = false;
+                break;
+            }
+        }
+        if (!ok) break;
+        if (tiles > 0) counts(tiles - 1);
+        if (kept) atomicAdd(&s_cnt[row], kept);
+        __syncthreads();
+        if (threadIdx.x < kPT && s_row[threadIdx.x] >= 0) {
+            const int32_t i = s_row[threadIdx.x];
+            const int64_t d = s_cnt[threadIdx.x], cap = cap_indptr[i + 1] - cap_indptr[i];
+            rowcnt[i] = (int32_t)(d < cap ? d : cap);
+            rowflag[i] = 2 | (d > cap ? 1 : 0);
+            // the first partition in processing order takes no capacity check
+            int64_t s, e;
+            tc.tail(i, order[0], s, e);
+            if (e - s > cap) set_err(err, DEV_FIRST_OVERFLOW);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                     "r"(kTcPairCols));
+}
+
+// every item to the comparison
+__global__ void k_pairs_all(const int64_t *item0, int K, int32_t *left, int *left_n)
+{
+    const int64_t n = item0[K];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *left_n = (int)n;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
+         t += (int64_t)gridDim.x * blockDim.x)
+        left[t] = (int32_t)t;
+}
+
 // rows of the row order whose flag bits under `mask` equal `want`, kept in
 // that order within each warp's 32 (the lists the streaming kernels take)
 __global__ void k_pick_rows(const int32_t *rowperm, int32_t n, const int32_t *rowflag, int mask,
@@ -1176,8 +1497,19 @@ static int launch_pairs(const CoWS &w, const TailCtx &tc, const int64_t *cap_ind
     if (smem > 200 * 1024) return EACB_ERR_UNSUPPORTED;
     EACB_CUDA(allow_max_dyn_smem(k_pairs<FILL>));
     PairCtx pc{w.lt, w.members, w.nbr, w.S, w.grp_off, w.grp_item0, w.grp_len, w.prow,
-               tc.n, tc.K, w.Q, w.ntiles, w.pbuf, w.pcap, w.pused, w.islot};
-    if (!FILL) EACB_CUDA(cudaMemsetAsync(w.pused, 0, sizeof(unsigned long long), st));
+               tc.n, tc.K, w.Q, w.ntiles, w.pbuf, w.pcap, w.pused, w.islot, w.left, w.left_n};
+    if (!FILL) {
+        EACB_CUDA(cudaMemsetAsync(w.pused, 0, sizeof(unsigned long long), st));
+        if ((int64_t)tc.P * tc.K <= kTcMapBits) {
+            EACB_CUDA(cudaMemsetAsync(w.left_n, 0, sizeof(int), st));
+            EACB_CUDA(allow_max_dyn_smem(k_pairs_tc));
+            k_pairs_tc<<<row_grid(1), kTcPairThreads, kTcPairSmem, st>>>(
+                pc, tc, w.order, cap_indptr, w.rowcnt, w.rowflag, &w.queue[7], w.err);
+        } else {
+            k_pairs_all<<<148, 256, 0, st>>>(w.grp_item0, tc.K, w.left, w.left_n);
+        }
+        EACB_CHECK_LAUNCH();
+    }
     k_pairs<FILL><<<row_grid(2), kPairThreads, smem, st>>>(
         pc, tc, w.order, cap_indptr, indptr, w.rowcnt, w.rowflag, indices, data,
         &w.queue[FILL ? 6 : 5], w.maxcnt, w.err);

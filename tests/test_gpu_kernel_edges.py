@@ -255,3 +255,35 @@ def test_final_clustering_pairs(order, off_w, off_i):
         cd[at] = bad
         with pytest.raises(EACBError):
             sp_sl_lifetime_csr(indptr, cd, wd, n, 219)
+
+
+@pytest.mark.parametrize("n,P,K,near", [
+    (129, 2, 3, True), (3000, 7, 11, True), (2600, 8, 10, False), (5000, 100, 40, True),
+    (2500, 255, 60, True),
+    (2600, 200, 8, False),       # too many clusters per row block for one operand
+    (6000, 255, 600, True),      # more (partition, cluster) pairs than the cluster map holds
+])
+def test_pair_tiles(n, P, K, near):
+    """Pair counts of row blocks as one-hot products and by comparison,
+    against the row restatement: row blocks of one to 128 rows, one to 32
+    units of eight partitions, clusters that neighbour each other or not."""
+    import oracle
+    from masters_final_b200.EAC.sparse import CoassocBuilder, capacity_indptr
+    rng = np.random.default_rng(n + P + K)
+    pos = rng.permutation(n) / n
+    if near:
+        L = np.stack([((pos + rng.random()) % 1.0 * max(2, K - int(rng.integers(0, 3)))).astype(np.int32)
+                      for _ in range(P)])
+    else:
+        L = rng.integers(0, K, (P, n)).astype(np.int32)
+        L[P // 2] = rng.integers(0, K + 3, n)
+    L[rng.random((P, n)) < 0.02] = -1
+    b = CoassocBuilder(L, n)
+    caps = capacity_indptr(n, n, "constant")
+    ip, ind, dat, nnz, disc, mx = b.build(caps)
+    assert disc == 0
+    ip, ind, dat = (x.cpu().numpy() for x in (ip, ind, dat))
+    rows = np.unique(np.concatenate([[0, 1, n - 2, n - 1], rng.integers(0, n, 200)]))
+    for i, (cols, counts) in zip(rows, oracle.coassoc_rows(L, caps.cpu().numpy(), rows)):
+        assert np.array_equal(ind[ip[i]:ip[i + 1]], cols), i
+        assert np.array_equal(dat[ip[i]:ip[i + 1]], counts), i
