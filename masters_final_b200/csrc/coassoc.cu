@@ -121,7 +121,7 @@ struct CoWS {
     unsigned long long *nbr_used;
     int32_t *rowlist;     // n: rows a streaming kernel takes
     int *rowlist_n;
-    uint8_t *pbuf;        // pair counts of the count pass's tiles, read by the fill
+    uint8_t *pbuf;        // pair counts of the count pass's items, read by the fill
     unsigned long long *pused;
     int64_t *islot;       // per pair-tile item: its place in pbuf (-1: none)
     int32_t *left;        // pair-tile items counted by comparison
@@ -819,7 +819,9 @@ struct PairCtx {
     const int *prow;
     int32_t n, K, Q;
     int64_t ntiles;
-    uint8_t *pbuf;            // kept pair counts (count pass writes, fill reads)
+    // kept pair counts (count pass writes, fill reads): an item's rows one
+    // after another, a byte per column of its tiles
+    uint8_t *pbuf;
     int64_t pcap;
     unsigned long long *pused;
     int64_t *islot;
@@ -832,6 +834,10 @@ struct PairCtx {
 // tx, tx + 16, ..., tx + 112: each group of 16 consecutive columns is then
 // held by the 16 lanes of a half-warp, one column per lane.
 __device__ __forceinline__ int col_slot(int c) { return ((c & 15) << 3) | (c >> 4); }
+
+// Column c of a tile of kept counts: byte 4 (c % 32) + c / 32, so that a lane
+// reads the counts of columns lane, lane + 32, ... as one word.
+__device__ __forceinline__ int count_slot(int c) { return ((c & 31) << 2) | (c >> 5); }
 
 // 128 points' label pairs into s[w*128 + slot] (-1: a NaN point); idx is
 // indexed by slot
@@ -854,12 +860,10 @@ __device__ __forceinline__ void load_pairs(uint32_t *s, const int32_t *idx, cons
 // Thread (tx, ty) of a 16 x 16 grid owns rows 8ty..8ty+7 and columns tx +
 // 16b (b = 0..7) of each tile.  A row's 16 consecutive columns 16b..16b+15
 // are then one per lane of a half-warp: a ballot places its kept entries, and
-// the half-warp writes them to consecutive positions with one store.  (With 8
-// consecutive columns per lane and a scan of the lanes' counts the stores
-// scatter: 7.3 ms for 3.9.)
+// the half-warp writes them to consecutive positions with one store.
 // COUNT: distinct columns per row -> rowcnt, rowflag (and the first
 // partition's overflow check), for the items k_pairs_tc left.  FILL: the kept
-// entries at indptr[i].
+// entries at indptr[i], for the items whose counts found no place.
 template <bool FILL>
 __global__ void __launch_bounds__(kPairThreads, 2)
 k_pairs(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr,
@@ -883,6 +887,10 @@ k_pairs(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr,
         __syncthreads();
         if (s_item >= (FILL ? nitems : *pc.left_n)) break;
         const int64_t t = FILL ? s_item : pc.left[s_item];
+        if (FILL && pc.islot[t] >= 0) {             // k_pairs_fill's
+            __syncthreads();
+            continue;
+        }
         int glo = 0, ghi = K;                       // item0[glo] <= t < item0[ghi]
         while (ghi - glo > 1) {
             const int m = (glo + ghi) >> 1;
@@ -913,12 +921,9 @@ k_pairs(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr,
                 if (nb[m] > first) b = m; else a = m + 1;
             }
             s_c0 = a;
-            // the item's counts: a place reserved by the count pass, which
-            // the fill reads instead of comparing again
-            if (FILL) {
-                s_slot = pc.islot[t];
-            } else {
-                const int64_t need = (int64_t)((len - a + kPT - 1) / kPT) * kPairThreads * 64;
+            // a place for the item's counts, which k_pairs_fill reads
+            if (!FILL) {
+                const int64_t need = (int64_t)((len - a + kPT - 1) / kPT) * kPT * kPT;
                 int64_t at = -1;
                 if (need > 0) {
                     at = (int64_t)atomicAdd(pc.pused, (unsigned long long)need);
@@ -940,7 +945,8 @@ k_pairs(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr,
             dcount[a] = 0;
         }
         __syncthreads();
-        const int64_t slot = s_slot;
+        const int64_t slot = FILL ? -1 : s_slot;
+        const int64_t width = (int64_t)((len - s_c0 + kPT - 1) / kPT) * kPT;
         for (int cb = s_c0, ci = 0; cb < len; cb += kPT, ++ci) {
             for (int c = threadIdx.x; c < kPT; c += blockDim.x)
                 s_col[col_slot(c)] = cb + c < len ? nb[cb + c] : -1;
@@ -948,19 +954,7 @@ k_pairs(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr,
             // the thread's 64 counts, one byte each: pw[2a + b/4] byte b%4 is
             // (row 8ty + a, column tx + 16b)
             uint32_t pw[16];
-            uint4 *kept = slot >= 0 ? reinterpret_cast<uint4 *>(
-                              pc.pbuf + slot + ((int64_t)ci * kPairThreads + threadIdx.x) * 64)
-                                    : nullptr;
-            if (FILL && slot >= 0) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const uint4 v = kept[q];
-                    pw[4 * q] = v.x;
-                    pw[4 * q + 1] = v.y;
-                    pw[4 * q + 2] = v.z;
-                    pw[4 * q + 3] = v.w;
-                }
-            } else {
+            {
                 load_pairs(sC, s_col, pc.lt, Q);
                 __syncthreads();
                 __half2 acc[8][8];
@@ -999,8 +993,11 @@ k_pairs(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr,
                     }
                 if (!FILL && slot >= 0)
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        kept[q] = make_uint4(pw[4 * q], pw[4 * q + 1], pw[4 * q + 2], pw[4 * q + 3]);
+                    for (int a = 0; a < 8; ++a)
+#pragma unroll
+                        for (int b = 0; b < 8; ++b)
+                            pc.pbuf[slot + (8 * ty + a) * width + ci * kPT + count_slot(tx + 16 * b)] =
+                                (uint8_t)(pw[2 * a + (b >> 2)] >> (8 * (b & 3)));
             }
             int32_t cj[8];
 #pragma unroll
@@ -1251,7 +1248,7 @@ k_pairs_tc(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indp
             }
             s_c0 = a;
             // a place for the item's counts, which the fill reads
-            const int64_t need = (int64_t)((len - a + kPT - 1) / kPT) * kPairThreads * 64;
+            const int64_t need = (int64_t)((len - a + kPT - 1) / kPT) * kPT * kPT;
             int64_t at = -1;
             if (need > 0) {
                 at = (int64_t)atomicAdd(pc.pused, (unsigned long long)need);
@@ -1301,17 +1298,14 @@ k_pairs_tc(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indp
                 out[q] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040),
                                      0x5410);
             }
-            if (slot >= 0) {
-                // (the fill's threads: 8 columns of one residue, 8 rows)
-                uint8_t *dst = pc.pbuf + slot +
-                               ((int64_t)ci * kPairThreads + (row >> 3) * 16 + 2 * cq) * 64 + (row & 7) * 8;
-                *reinterpret_cast<uint2 *>(dst) = make_uint2(out[0], out[1]);
-                *reinterpret_cast<uint2 *>(dst + 64) = make_uint2(out[2], out[3]);
-            }
+            if (slot >= 0)
+                *reinterpret_cast<uint4 *>(pc.pbuf + slot + (int64_t)row * tiles * kPT + ci * kPT + 16 * cq) =
+                    make_uint4(out[0], out[1], out[2], out[3]);
         };
-        // the point of tile ci's operand row s: columns in slot order
+        // the point of tile ci's operand row s: the columns in the order of
+        // the kept counts
         auto column = [&](int ci, int s) -> int32_t {
-            const int at = c0 + ci * kPT + (s >> 3) + 16 * (s & 7);
+            const int at = c0 + ci * kPT + (s >> 2) + 32 * (s & 3);
             return ci < tiles && at < len ? nb[at] : -1;
         };
         lab.load(pc.lt, Q, column(0, r8));
@@ -1364,6 +1358,112 @@ k_pairs_tc(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indp
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                      "r"(kTcPairCols));
+}
+
+// The fill pass from the kept counts: a warp per row, a column per lane.  A
+// lane's four bytes of a tile are the counts of columns lane, lane + 32, ...
+// (count_slot), so that a ballot places 32 consecutive columns' kept entries
+// and the warp writes them side by side.  Items go to the blocks 32 rows at a
+// time.  Issue bound (about 16 instructions per 32 columns): 300,000 points
+// and 100 partitions took 3.9 ms in 16 warps per SM with a thread's 64 counts
+// in registers, and take 2.3 in 40.  (Entries collected in shared memory and
+// written in runs of 32 took 5.8: bank conflicts.)
+constexpr int kPfThreads = 256;
+constexpr int kPfWarps = kPfThreads / 32;
+constexpr int kPfRows = 32;
+constexpr int kPfUnits = kPT / kPfRows;          // of an item
+constexpr int kPfTiles = 4;                      // tiles with loads in flight
+
+__global__ void __launch_bounds__(kPfThreads, 5)
+k_pairs_fill(PairCtx pc, const int64_t *indptr, const int32_t *rowflag, int32_t *indices,
+             uint8_t *data, int *queue, int *gmax, int *err)
+{
+    __shared__ int s_unit;
+    const int K = pc.K, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const int pr = *pc.prow;
+    const int64_t nunits = pc.item0[K] * kPfUnits;
+    uint32_t maxc = 0;
+    // the first of x[0, n) above v: 32 probes at a time
+    auto above = [&](const auto *x, int n, int64_t v) -> int {
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int at = lo + (int)((int64_t)(hi - lo) * lane / 32);
+            const int c = __popc(__ballot_sync(0xffffffffu, (int64_t)x[at] <= v));
+            const int last = __shfl_sync(0xffffffffu, at, c ? c - 1 : 0);
+            const int next = __shfl_sync(0xffffffffu, at, c < 32 ? c : 31);
+            if (c < 32) hi = next;
+            if (c) lo = last + 1;
+        }
+        return lo;
+    };
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_unit = atomicAdd(queue, 1);
+        __syncthreads();
+        if (s_unit >= nunits) break;
+        const int64_t t = s_unit / kPfUnits;
+        const int64_t slot = pc.islot[t];
+        if (slot < 0) continue;
+        const int g = above(pc.item0, K + 1, t) - 1;         // item0[g] <= t < item0[g + 1]
+        const int64_t gb = pc.S[((int64_t)pr * K + g) * pc.ntiles];
+        const int64_t size = pc.S[((int64_t)pr * K + g + 1) * pc.ntiles] - gb;
+        const int64_t r0 = (t - pc.item0[g]) * kPT;
+        const int nrow = (int)(size - r0 < kPT ? size - r0 : kPT);
+        const int first_row = (int)(s_unit % kPfUnits) * kPfRows;
+        if (first_row >= nrow) continue;
+        const int32_t *rows = pc.members + gb + r0;
+        const int32_t *nb = pc.nbr + pc.grp_off[g];
+        const int len = pc.grp_len[g];
+        const int c0 = above(nb, len, rows[0]);
+        const int32_t *col = nb + c0;                        // the item's columns
+        const int ncol = len - c0;
+        const int tiles = (ncol + kPT - 1) / kPT;
+        for (int r = first_row + warp; r < min(nrow, first_row + kPfRows); r += kPfWarps) {
+            const int32_t i = rows[r];
+            if (rowflag[i] & 1) continue;                    // over its capacity: not this way
+            const uint32_t *cnt = reinterpret_cast<const uint32_t *>(pc.pbuf + slot) +
+                                  (int64_t)r * tiles * (kPT / 4) + lane;
+            const int64_t begin = indptr[i];
+            const int room = (int)(indptr[i + 1] - begin);
+            int32_t *ip = indices + begin;
+            uint8_t *dp = data + begin;
+            int at = 0;                                      // entries written
+            const int first = above(col, ncol, i);           // columns before it are not above the row
+            for (int tb = first / kPT; tb < tiles; tb += kPfTiles) {
+                uint32_t w[kPfTiles];
+#pragma unroll
+                for (int u = 0; u < kPfTiles; ++u)
+                    w[u] = tb + u < tiles ? __ldcs(cnt + (int64_t)(tb + u) * (kPT / 4)) : 0u;
+                if (tb * kPT < first) {                      // (the first tile's columns up to the row)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (tb * kPT + 32 * e + lane < first) w[0] &= ~(255u << (8 * e));
+                }
+#pragma unroll
+                for (int u = 0; u < kPfTiles; ++u) {
+                    if (!__any_sync(0xffffffffu, w[u] != 0u)) continue;
+                    const int32_t *cp = col + (tb + u) * kPT + lane;
+                    maxc = __vmaxu4(maxc, w[u]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const uint32_t k = (w[u] >> (8 * e)) & 255u;
+                        const unsigned bal = __ballot_sync(0xffffffffu, k != 0u);
+                        const int pos = at + __popc(bal & below);
+                        if (k != 0u && pos < room) {
+                            ip[pos] = __ldg(cp + 32 * e);
+                            dp[pos] = (uint8_t)k;
+                        }
+                        at += __popc(bal);
+                    }
+                }
+            }
+            if (lane == 0 && at != room) set_err(err, DEV_CAPACITY);
+        }
+    }
+    int m = (int)max(max(maxc & 255u, (maxc >> 8) & 255u), max((maxc >> 16) & 255u, maxc >> 24));
+    for (int d = 16; d >= 1; d >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+    if (lane == 0) atomicMax(gmax, m);
 }
 
 // every item to the comparison
@@ -1508,6 +1608,11 @@ static int launch_pairs(const CoWS &w, const TailCtx &tc, const int64_t *cap_ind
         } else {
             k_pairs_all<<<148, 256, 0, st>>>(w.grp_item0, tc.K, w.left, w.left_n);
         }
+        EACB_CHECK_LAUNCH();
+    }
+    if (FILL) {
+        k_pairs_fill<<<grid_for(w.nitems_max * kPfUnits, 1, row_grid(1) * 5), kPfThreads, 0, st>>>(
+            pc, indptr, w.rowflag, indices, data, &w.queue[7], w.maxcnt, w.err);
         EACB_CHECK_LAUNCH();
     }
     k_pairs<FILL><<<row_grid(2), kPairThreads, smem, st>>>(
