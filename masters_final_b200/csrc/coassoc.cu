@@ -31,11 +31,11 @@
 //     redone by a rank-aware kernel: a column's rank (first partition in
 //     processing order that associates it) is an atomicMin per visit, and
 //     the keep rule is applied from the rank histogram.
-//  4. the pair tiles (k_nbr, k_pairs): rows grouped by their
-//     cluster in the partition with the most clusters are counted by
-//     comparing label vectors over the group's neighbourhood instead of
-//     streaming tails, when that is cheaper; the count pass keeps each
-//     tile's pair counts for the fill.  Steps 2 and 3 then take only the
+//  4. the pair tiles (k_nbr, k_pairs_tc, k_pairs_fill): rows grouped by
+//     their cluster in the partition with the most clusters are counted
+//     against the group's neighbourhood, as products of one-hot rows on the
+//     tensor cores, instead of streaming tails, when that is cheaper; the
+//     count pass keeps the pair counts for the fill.  Steps 2 and 3 then take only the
 //     rows outside those groups (and every row over its capacity).
 #include "eacb_common.cuh"
 #include "scan_impl.cuh"
@@ -67,7 +67,7 @@ constexpr int kMaxP = 255;
 // 4 neighbourhoods, 5 pair tiles (count), 6 pair tiles (fill)
 constexpr int kQueues = 8;
 
-// pair tiles: 128 rows x 128 columns, labels as FP16 pairs (exact below 2048)
+// pair tiles: 128 rows x 128 columns, labels as 16-bit words (below 2048)
 constexpr int kPT = 128;
 constexpr int kPairThreads = 256;
 constexpr int kDenseMaxK = 2048;
@@ -84,7 +84,7 @@ constexpr int64_t kDenseRatioDefault = 16;
 constexpr int64_t kPairBytesPerPoint = 8192;
 constexpr int64_t kPairBytesMax = (int64_t)32 << 30;
 
-// half2 words per point in the FP16 label copy: P rounded up to 8 partitions
+// 32-bit words per point in the point-major label copy: P rounded up to 8
 __host__ __device__ constexpr int32_t pair_words(int32_t P) { return ((P + 7) / 8) * 4; }
 
 // what the host reads after a call, in one copy
@@ -112,7 +112,7 @@ struct CoWS {
     int32_t *rowperm;     // n: the order the row kernels take rows in
     int *queue;           // work-queue counters
     int *prow;            // the partition whose clusters order the rows
-    uint32_t *lt;         // n x Q: FP16 label pairs, point-major (pair tiles)
+    uint32_t *lt;         // n x Q: label pairs, point-major (pair tiles)
     int64_t *grp_off;     // K: a group's neighbourhood in nbr
     int32_t *grp_len;     // K: its length
     int32_t *grp_tiles;   // K (+1): pair-tile row blocks of a group (0: streamed)
@@ -128,7 +128,7 @@ struct CoWS {
     int *left_n;
     ScanScratch scan;
     int64_t ntiles, nbr_cap, pcap, nitems_max;
-    int32_t Q;            // half2 words per point in lt
+    int32_t Q;            // words per point in lt
     static CoWS carve(Carver &c, int32_t n, int32_t P, int32_t K)
     {
         CoWS w;

@@ -160,43 +160,6 @@ __device__ __forceinline__ int64_t warp_incl_sum(int64_t v)
     return v;
 }
 
-// Exclusive sum across the block; `total` receives the block sum.  The
-// warp totals are combined with a Blelloch up-sweep / down-sweep in shared
-// memory (work-efficient tree, 2 log2(warps) steps).
-template <int THREADS>
-__device__ __forceinline__ int64_t block_excl_sum(int64_t v, int64_t &total)
-{
-    constexpr int W = THREADS / 32;
-    __shared__ int64_t tree[W];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int64_t inc = warp_incl_sum(v);
-    if (lane == 31) tree[warp] = inc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        // up-sweep
-        for (int d = 1; d < W; d <<= 1)
-            for (int i = 2 * d - 1; i < W; i += 2 * d) tree[i] += tree[i - d];
-    }
-    __syncthreads();
-    int64_t tot = tree[W - 1];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        tree[W - 1] = 0;
-        // down-sweep
-        for (int d = W >> 1; d >= 1; d >>= 1)
-            for (int i = 2 * d - 1; i < W; i += 2 * d) {
-                int64_t t = tree[i - d];
-                tree[i - d] = tree[i];
-                tree[i] += t;
-            }
-    }
-    __syncthreads();
-    int64_t r = tree[warp] + inc - v;
-    total = tot;
-    __syncthreads();
-    return r;
-}
-
 // The same result with the warp totals combined by warp 0 in shuffles (three
 // barriers, no serial steps): for the row kernels, which scan once per
 // column chunk.
