@@ -368,7 +368,7 @@ k_whist_csr(const WT *weight, int64_t E, int wbits, unsigned long long *hist)
 constexpr int kHist8Threads = 64;
 constexpr size_t kHist8Smem = (size_t)(kHist8Threads / 32) * 256 * 32 * sizeof(uint32_t);
 __global__ void __launch_bounds__(kHist8Threads, 1)
-k_whist_u8(const uint8_t *w, int64_t n, unsigned long long *hist)
+k_whist_u8(const uint8_t *w, int64_t n, int skip, unsigned long long *hist)
 {
     extern __shared__ uint32_t hs[];
     for (int i = threadIdx.x; i < (kHist8Threads / 32) * 256 * 32; i += blockDim.x) hs[i] = 0;
@@ -376,7 +376,10 @@ k_whist_u8(const uint8_t *w, int64_t n, unsigned long long *hist)
     uint32_t *mine = hs + (threadIdx.x >> 5) * 256 * 32 + (threadIdx.x & 31);
     int64_t head = (int64_t)((16 - ((uintptr_t)w & 15)) & 15);
     if (head > n) head = n;
-    const int64_t nv = (n - head) >> 4;               // whole 16-byte vectors
+    // the whole 16-byte vectors read: with skip > 1, 32 of each 32 * skip
+    const int64_t whole = (n - head) >> 4;
+    const int64_t nv = skip == 1 ? whole : whole / (32 * skip) * 32;
+    auto at = [&](int64_t q) -> int64_t { return skip == 1 ? q : (q >> 5) * (32 * skip) + (q & 31); };
     const uint4 *v = reinterpret_cast<const uint4 *>(w + head);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     auto add16 = [&](const uint4 &x) {
@@ -392,7 +395,7 @@ k_whist_u8(const uint8_t *w, int64_t n, unsigned long long *hist)
     for (; q + (kU - 1) * stride < nv; q += kU * stride) {
         uint4 x[kU];
 #pragma unroll
-        for (int u = 0; u < kU; ++u) x[u] = __ldcs(v + q + u * stride);
+        for (int u = 0; u < kU; ++u) x[u] = __ldcs(v + at(q + u * stride));
         // all eight loads are issued before the first is consumed
 #pragma unroll
         for (int u = 0; u < kU; ++u)
@@ -400,9 +403,9 @@ k_whist_u8(const uint8_t *w, int64_t n, unsigned long long *hist)
 #pragma unroll
         for (int u = 0; u < kU; ++u) add16(x[u]);
     }
-    for (; q < nv; q += stride) add16(__ldcs(v + q));
+    for (; q < nv; q += stride) add16(__ldcs(v + at(q)));
     // the unaligned head and the ragged tail (< 32 bytes), by the first block
-    if (blockIdx.x == 0) {
+    if (blockIdx.x == 0 && skip == 1) {
         const int64_t tail0 = head + (nv << 4);
         const int64_t rest = head + (n - tail0);
         const int64_t t = threadIdx.x;
@@ -417,11 +420,13 @@ k_whist_u8(const uint8_t *w, int64_t n, unsigned long long *hist)
     }
 }
 
-static int launch_whist_u8(const uint8_t *w, int64_t n, unsigned long long *hist, cudaStream_t st)
+// (skip > 1: of one in `skip` of the bytes, 512 of each 512 * skip)
+static int launch_whist_u8(const uint8_t *w, int64_t n, unsigned long long *hist, cudaStream_t st,
+                           int skip = 1)
 {
     EACB_CUDA(allow_max_dyn_smem(k_whist_u8));
-    k_whist_u8<<<grid_for((n + 15) / 16, kHist8Threads, 148 * 3), kHist8Threads, kHist8Smem,
-                 st>>>(w, n, hist);
+    k_whist_u8<<<grid_for((n / skip + 15) / 16, kHist8Threads, 148 * 3), kHist8Threads, kHist8Smem,
+                 st>>>(w, n, skip, hist);
     EACB_CHECK_LAUNCH();
     return EACB_OK;
 }
@@ -2866,6 +2871,11 @@ extern "C" int eacb_connected_components(const int32_t *dest, const void *weight
 // bounded edge array below and may redo an overflowing phase in pieces.
 constexpr int64_t kFinalQueuedEntries = (int64_t)1 << 26;
 
+// The phases of such a larger matrix are planned from an eighth of its
+// weights (8M or more), spread evenly: the plan only chooses where the phases
+// end.  (920M entries: 355 us for all the weights, 53 for the sample.)
+constexpr int kWhistSkip = 8;
+
 // Edge words of the final clustering (one per kept entry): every entry when
 // the matrix is small, else 256 words per point (at least 2^20): room for
 // the usual output of a phase, not its worst case (a phase that overflows is
@@ -2885,11 +2895,13 @@ static int64_t final_edge_cap(int32_t n, int64_t nnz)
 // the lightest few per point already join most points: later phases keep
 // only entries between different components, so they write few edges, and a
 // phase over a narrow range reads little more than the weights.
-static void plan_final_phases(const unsigned long long h[256], int32_t n, std::vector<Phase> &plan)
+//
+// h may be of a sample of the entries: every weight lies in some range, and
+// which one changes the phases' sizes only.
+static void plan_final_phases(const unsigned long long h[256], int32_t n, int64_t nnz,
+                              std::vector<Phase> &plan)
 {
-    unsigned long long tot = 0;
-    for (int b = 0; b < 256; ++b) tot += h[b];
-    const double t = tot ? (double)tot : 1.0;
+    const double t = nnz ? (double)nnz : 1.0;
     double fracs[6];
     for (int f = 0; f < 5; ++f) fracs[f] = std::min(1.0, (double)(8 << (2 * f)) * n / t);
     fracs[5] = 1.0;
@@ -3032,12 +3044,14 @@ extern "C" int eacb_final_clustering(const int64_t *indptr, const int32_t *indic
     // 1. minimum spanning forest of the dissimilarity graph, by weight phases
     //    (the reset cleared the histogram)
     if (nnz > 0) {
-        if ((s = launch_whist_u8(diassoc, nnz, g.hist, st))) return s;
+        if ((s = launch_whist_u8(diassoc, nnz, g.hist, st,
+                                 nnz > kFinalQueuedEntries ? kWhistSkip : 1)))
+            return s;
     }
     unsigned long long wh[256];
     if ((s = g.read_hist(st, wh))) return s;
     std::vector<Phase> phases;
-    plan_final_phases(wh, n, phases);
+    plan_final_phases(wh, n, nnz, phases);
     auto build = [&](const Phase &ph) -> int {
         if (nnz == 0) return EACB_OK;
         ProfScope ps(PROF_PHASE, st);

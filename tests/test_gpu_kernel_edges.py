@@ -287,3 +287,28 @@ def test_pair_tiles(n, P, K, near):
     for i, (cols, counts) in zip(rows, oracle.coassoc_rows(L, caps.cpu().numpy(), rows)):
         assert np.array_equal(ind[ip[i]:ip[i + 1]], cols), i
         assert np.array_equal(dat[ip[i]:ip[i + 1]], counts), i
+
+
+@pytest.mark.parametrize("n", [11_585, 11_600])
+def test_final_clustering_sampled_plan(n):
+    """Just below and above 2^26 entries, where the phases are planned from a
+    sample of the weights: three cliques whose light edges join them, heavy
+    edges between them, some weights in one entry each."""
+    import torch
+    from masters_final_b200.EAC.eac import sp_sl_lifetime_csr
+    assert (n * (n - 1) // 2 > 1 << 26) == (n == 11_600)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    group = torch.randint(0, 3, (n,), generator=g, device="cuda")
+    i, j = torch.triu_indices(n, n, 1, device="cuda")
+    w = torch.randint(2, 40, (i.numel(),), generator=g, device="cuda", dtype=torch.uint8)
+    w[group[i] != group[j]] = 200
+    w[torch.tensor([3, 1000, i.numel() - 1], device="cuda")] += 7
+    indptr = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    indptr[1:] = torch.cumsum(torch.arange(n - 1, -1, -1, device="cuda"), 0)
+    nc, labels = sp_sl_lifetime_csr(indptr, j.int(), w, n, 220)
+    assert nc == 3
+    group = group.cpu().numpy()
+    first = {}
+    want = np.array([first.setdefault(int(x), len(first)) for x in group])
+    assert np.array_equal(labels, want)
