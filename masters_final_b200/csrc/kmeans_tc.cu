@@ -187,7 +187,11 @@ __global__ void k_prep_centroids(const float *C, const int32_t *kk, int32_t kmax
         float nrm;
         put_row(v, mu, D, Kp, c % kTN, tile, false, nrm);
         nc[e] = real ? nrm : __int_as_float(0x7f800000);
-        if (real) atomicMax(reinterpret_cast<int *>(&cmax2[p]), __float_as_int(nrm));
+        // a NaN norm (which no screen may judge) counts only at centroid 0:
+        // there the reference keeps it, elsewhere it never compares as smaller
+        if (real && (nrm == nrm || c == 0))
+            atomicMax(reinterpret_cast<int *>(&cmax2[p]),
+                      nrm == nrm ? __float_as_int(nrm) : 0x7fffffff);
     }
 }
 
@@ -420,23 +424,32 @@ k_label_tc(const float *__restrict__ X, int32_t n, int32_t D, int32_t Kp, const 
                 // |c|^2) of the exact one.  A column c* that the exact
                 // arithmetic could rank at or before the least screened one,
                 // w, has |x - c*|^2 <= |x - c_w|^2 <= w1 + |x|^2 + e(w), so
-                // |c*| and |c_w| are at most |x| + sqrt(w1 + |x|^2 + e(w))
-                // and at most the partition's largest norm (which bounds the
-                // e(w) under the root).  No column outside w's chunk comes
-                // before w when the least of them is more than e(w) + e(c*)
-                // above it (the bound taken 1% wide for the rounding of this
-                // arithmetic).
+                // |c*| is at most |x| + sqrt(w1 + |x|^2 + e(w)) and at most
+                // the partition's largest norm; |c_w| is at most the largest
+                // finite norm of its chunk (columns past K have an infinite
+                // one, and no other infinite or NaN norm can win).  No column
+                // outside w's chunk comes before w when the least of them is
+                // more than e(w) + e(c*) above it (the bound taken 1% wide for
+                // the rounding of this arithmetic, with an absolute part for
+                // products that underflow: 6 D of them, below 2^-126 each).
+                const float inf = __int_as_float(0x7f800000);
                 const float cm2 = cmax2[p];
-                const float rc = sqrtf(xn) + sqrtf(fmaxf(0.f, w1 + xn + 0.5f * E * (xn + cm2)));
-                const float bound = 1.01f * E * (xn + fminf(rc * rc, cm2));
+                constexpr int CK = kTcChunk;
+                static_assert(CK == 4, "the chunk's norms are one vector");
+                const float4 cn = *reinterpret_cast<const float4 *>(
+                    nc + ((int64_t)p * kt_max * kTN + CK * wi));
+                const float nw = fmaxf(fmaxf(cn.x < inf ? cn.x : 0.f, cn.y < inf ? cn.y : 0.f),
+                                       fmaxf(cn.z < inf ? cn.z : 0.f, cn.w < inf ? cn.w : 0.f));
+                const float ew = 0.5f * E * (xn + nw);
+                const float rc = sqrtf(xn) + sqrtf(fmaxf(0.f, w1 + xn + ew));
+                const float bound = 1.01f * (ew + 0.5f * E * (xn + fminf(rc * rc, cm2))) + 1e-35f;
                 // inside the chunk: direct float32 distances, within (D + 2)
                 // 2^-24 of the reference's (relative), so the least is
                 // certain when the next is beyond four times that
                 const int64_t row0 = (int64_t)p * kmax;
-                constexpr int CK = kTcChunk;
                 float xv[DM], cv[DM];
                 load_row<DM, VEC>(X + i * D, D, xv);
-                float bd = __int_as_float(0x7f800000), bd2 = bd;
+                float bd = inf, bd2 = inf;
                 int w = -1;
 #pragma unroll
                 for (int c = 0; c < CK; ++c) {
@@ -450,7 +463,7 @@ k_label_tc(const float *__restrict__ X, int32_t n, int32_t D, int32_t Kp, const 
                 const float thr = __fadd_ru(__fmul_ru(bd, 1.f + 4.f * (float)(D + 2) * 5.9604645e-8f),
                                             1e-38f);
                 const int64_t o = (int64_t)p * n + i;
-                if (w2 - w1 > bound && bd2 > thr && w >= 0) {
+                if (w2 - w1 > bound && bd2 > thr && w >= 0 && cm2 == cm2) {
                     load_row<DM, VEC>(C + (row0 + w) * D, D, cv);
                     labels[o] = w;
                     dists[o] = (float)exact_dist_reg<DM>(xv, cv, D);
