@@ -576,6 +576,11 @@ constexpr int kFillThreads = 1024;
 constexpr int kFillItems = 8;
 constexpr int kFillTile = kFillThreads * kFillItems;
 constexpr int kFillSeqMax = 256;
+// steps of that loop at most.  A step whose pivot is the least of the range
+// only rotates the range by one place, so the range may stand still while
+// copies of that value pass the middle (fewer than its length) before it
+// shrinks: at most length x length steps (two values, 256 keys: 257).
+constexpr int kFillSeqSteps = kFillSeqMax * kFillSeqMax;
 constexpr int kFillRounds = 1 << 15;     // steps shrink the range; equal keys take one per cluster
 // blocks per partition: a cluster from this many points on (below, one
 // block's passes cost no more than the cluster's barriers)
@@ -757,7 +762,7 @@ k_fill_empty(const float *X, int32_t n, int32_t D, float *dists, const int64_t *
     if (threadIdx.x == 0) {
         int a = 0, b = L - 1, steps = 0;
         while (a < b) {
-            if (++steps > kFillSeqMax) {               // a NaN pivot does not shrink the range
+            if (++steps > kFillSeqSteps) {             // a NaN pivot does not shrink the range
                 set_err(err, DEV_CHASE_LIMIT);
                 break;
             }

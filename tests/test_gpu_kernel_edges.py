@@ -63,6 +63,26 @@ def test_empty_cluster_selection(kind, n, empty):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("n,ones,empty", [(256, 126, 129), (256, 126, 128), (255, 125, 129),
+                                          (257, 126, 130), (40, 18, 20)])
+def test_empty_cluster_selection_standing_range(n, ones, empty):
+    """Two distance values with the smaller one from the middle on: the
+    quickselect's range stands still for steps on end, and it takes more steps
+    than the range has keys."""
+    import oracle
+    from masters_final_b200.cluster.KMeans import kmeans_centroids
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, 2)).astype(np.float32)
+    full = 5
+    k = full + empty
+    ids = np.sort(rng.choice(k, full, replace=False)).astype(np.int32)
+    labels = ids[rng.integers(0, full, n)]
+    labels[:full] = ids
+    dist = np.where(np.arange(n) < ones, 1.0, 0.0).astype(np.float32)
+    got = kmeans_centroids(x, labels, dist, k).cpu().numpy()
+    assert np.array_equal(got, oracle.kmeans_centroids(x, labels, dist, k))
+
+
 @pytest.mark.parametrize("n", [1, 7, 8, 128, 129, 255, 257, 1023, 2049, 4111, 16385, 131073, 262207,
                                1000003])
 def test_inertia_order(n):
