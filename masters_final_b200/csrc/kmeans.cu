@@ -248,10 +248,14 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
         // winner's distance (capped by the partition's largest norm).  The
         // bound is 1% wide for this arithmetic's rounding, with an absolute
         // part for products that underflow.
+        // (A winner whose squared distance may pass the largest float is not
+        // judged: the reference's squares are then infinite, and it keeps the
+        // first of the centroids that far.)
         const float ew = E * (xn[q] + ncw);
-        const float rc = sqrtf(xn[q]) + sqrtf(fmaxf(0.f, xn[q] + 2.f * b1[q] + ew));
+        const float far = xn[q] + 2.f * b1[q] + ew;
+        const float rc = sqrtf(xn[q]) + sqrtf(fmaxf(0.f, far));
         const float bound = 1.01f * (ew + E * (xn[q] + fminf(rc * rc, cmax))) + 1e-36f;
-        if (2.f * (b2[q] - b1[q]) > bound && bi >= 0 && b1[q] < inf && cmax == cmax) {
+        if (2.f * (b2[q] - b1[q]) > bound && bi >= 0 && far < 3e38f && cmax == cmax) {
             float xv[DM], cv[DM];
             load_row<DM, VEC>(X + i * D, D, xv);
             load_row<DM, VEC>(C + ((int64_t)p * kmax + w) * D, D, cv);

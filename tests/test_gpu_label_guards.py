@@ -88,3 +88,18 @@ def test_ensemble_nan_row_two_passes(mode):
     assert np.array_equal(cent[0].cpu().numpy(), c2, equal_nan=True)
     assert np.array_equal(lab[0].cpu().numpy(), l2)
     assert np.array_equal(dist[0].cpu().numpy(), d2, equal_nan=True)
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("d", [1, 2, 5, 16])
+def test_label_overflowing_distances(mode, d):
+    """Finite points whose squared distances to every centroid pass the
+    largest float: the reference's distances are all infinite and it keeps
+    label 0; nearer points are labelled as ever."""
+    rng = np.random.default_rng(d)
+    x = rng.standard_normal((4000, d)).astype(np.float32)
+    side = np.where(rng.random(4000) < 0.5, 1.0, -1.0)
+    x[:, 0] = side * (1.1e19 + 1e17 * rng.standard_normal(4000))
+    c = rng.standard_normal((6, d)).astype(np.float32)
+    c[:, 0] = [1.16e19, 1.1e19, 1.12e19, 1.07e19, 1.14e19, 1.11e19]
+    _check(x, c, mode)
