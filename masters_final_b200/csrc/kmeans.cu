@@ -57,8 +57,10 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src)
 // moves the distance by at most 4 u S, the half norm and the chain of D
 // products by (3 D + 1) u S, and the reference's own float32 squares by 6 u S:
 // a screened distance is within e(c) = (3 D + 12) u S of the reference's.  A
-// point whose runner-up is not certainly behind its winner goes to the exact
-// re-check.
+// point whose runner-up is not certainly behind its winner is open: a block's
+// few open points go to the exact re-check, a block with many to
+// k_label_direct, because S is large against the distances' gaps for all
+// points of a blob that lies far from the mean.
 //
 // Bound by the FMA pipe (half of its cycles) and the shared-memory reads.
 // One pass: 500,000 x 16 points, 20 partitions of 530: 20.5 ms with a
@@ -105,65 +107,69 @@ __global__ void k_prep_label_f32(const float *__restrict__ C, const int32_t *__r
     }
 }
 
-// CK: centroids per chunk; VEC: D equals DM and the rows of X and C can be
-// read as vectors
-template <int DM, int NP, int CK, bool VEC>
-__global__ void __launch_bounds__(kLT, 4)
-k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__restrict__ C,
-            const float *__restrict__ rows, const int32_t *__restrict__ kk, int32_t kmax,
-            int32_t kpad, const int32_t *__restrict__ active, const float *__restrict__ mu,
-            const float *__restrict__ cmax2, float E, int32_t *__restrict__ labels,
-            float *__restrict__ dists, int32_t *__restrict__ amb, int *__restrict__ namb)
+// The thread's 2 NP points as pairs (point q: i0 + q kLT; past the last one
+// its row again, never written), CENTRED less mu with their norms in xn, or
+// as they are.
+template <int DM, int NP, bool VEC, bool CENTRED>
+__device__ __forceinline__ void label_points(const float *__restrict__ X, int32_t n, int32_t D,
+                                             int64_t i0, const float *__restrict__ mu,
+                                             uint64_t (&x)[DM][NP], float (&xn)[2 * NP])
 {
-    constexpr int RF = LabelRow<DM>::RF, CH = LabelRow<DM>::CH, Q = 2 * NP;
-    __shared__ __align__(16) float cs[2][(CH + 4) * RF];
-    static_assert(CH % CK == 0 && kTcCentPad % CK == 0, "whole chunks");
-    const int p = blockIdx.y;
-    if (!active[p]) return;
-    const int K = kk[p];
-    const float inf = __int_as_float(0x7f800000), cmax = cmax2[p];
-    uint64_t x[DM][NP];
-    float xn[Q], b1[Q], b2[Q];
-    int i1[Q];
-    const int64_t i0 = (int64_t)blockIdx.x * (Q * kLT) + threadIdx.x;    // point q: i0 + q kLT
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        xn[q] = 0.f;
-        b1[q] = b2[q] = inf;
-        i1[q] = 0;
-    }
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
         float v[2][DM];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            // past the last point: its row again, never written
             const int64_t i = min((int64_t)n - 1, i0 + (2 * j + h) * kLT);
             load_row<DM, VEC>(X + i * D, D, v[h]);
+            if (CENTRED) xn[2 * j + h] = 0.f;
         }
 #pragma unroll
         for (int d = 0; d < DM; ++d) {
-            const float m = VEC || d < D ? mu[d] : 0.f;
+            if (CENTRED) {
+                const float m = VEC || d < D ? mu[d] : 0.f;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                v[h][d] = __fsub_rn(v[h][d], m);
-                xn[2 * j + h] = fmaf(v[h][d], v[h][d], xn[2 * j + h]);
+                for (int h = 0; h < 2; ++h) {
+                    v[h][d] = __fsub_rn(v[h][d], m);
+                    xn[2 * j + h] = fmaf(v[h][d], v[h][d], xn[2 * j + h]);
+                }
             }
             x[d][j] = pack2(v[0][d], v[1][d]);
         }
     }
-    const float *src = rows + (int64_t)p * kpad * RF;
-    auto stage = [&](int c0, int buf) {          // kpad is a multiple of CH
-        for (int e = threadIdx.x; e < CH * RF / 4; e += kLT)
-            cp_async<16>(&cs[buf][4 * e], src + (int64_t)c0 * RF + 4 * e);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    stage(0, 0);
+}
+
+// One dimension's part of a score: of the centred rows less the product, of
+// the rows as they are (DIRECT) the square of the difference.
+template <bool DIRECT>
+__device__ __forceinline__ uint64_t score_step2(uint64_t x, uint64_t w, uint64_t acc)
+{
+    if (!DIRECT) return ffma2(x, w, acc);
+    const uint64_t t = fadd2(x, w);
+    return ffma2(t, t, acc);
+}
+
+// The best two chunk minima of every point's scores and the winner's chunk,
+// over K rows; stage(dst, c0) begins to bring rows c0 to c0 + CH - 1 (padded
+// to whole chunks) into a buffer.
+template <int DM, int NP, int CK, bool DIRECT, typename Stage>
+__device__ __forceinline__ void
+label_sweep(float (&cs)[2][(LabelRow<DM>::CH + 4) * LabelRow<DM>::RF], int K,
+            const uint64_t (&x)[DM][NP], float (&b1)[2 * NP], float (&b2)[2 * NP],
+            int (&i1)[2 * NP], Stage stage)
+{
+    constexpr int RF = LabelRow<DM>::RF, CH = LabelRow<DM>::CH, Q = 2 * NP;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        b1[q] = b2[q] = __int_as_float(0x7f800000);
+        i1[q] = 0;
+    }
+    stage(cs[0], 0);
     int buf = 0;
     for (int c0 = 0; c0 < K; c0 += CH, buf ^= 1) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                         // this buffer is there, the other one is free
-        if (c0 + CH < K) stage(c0 + CH, buf ^ 1);
+        if (c0 + CH < K) stage(cs[buf ^ 1], c0 + CH);
         const int g1 = min(CH, (K - c0 + CK - 1) / CK * CK) >> 2;    // groups of four
         float cmin[Q];                           // the chunk's least scores
         // the four rows' next 16-byte vectors are read while the current ones
@@ -191,7 +197,7 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
                         const uint64_t w = twice(e);
 #pragma unroll
                         for (int j = 0; j < NP; ++j)
-                            acc[c][j] = d < 0 ? w : ffma2(x[d < 0 ? 0 : d][j], w, acc[c][j]);
+                            acc[c][j] = d < 0 ? w : score_step2<DIRECT>(x[d < 0 ? 0 : d][j], w, acc[c][j]);
                     }
                 }
 #pragma unroll
@@ -214,13 +220,76 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
             }
         }
     }
+}
+
+// The block's points without a certain label (open: the thread's), by all its
+// threads: up to one in eight go to the list that label_exact_points takes,
+// which is a warp and a read of every centroid's row for each.  More stay, and
+// the block has to go on with them (false).
+template <int Q>
+__device__ __forceinline__ bool label_listed(unsigned open, int64_t o0, int *s_open, int32_t *amb,
+                                             int *namb)
+{
+    const int mine = (int)__reduce_add_sync(0xffffffffu, (unsigned)__popc(open));
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(s_open, mine);
+    __syncthreads();
+    if (amb ? *s_open * 8 > Q * kLT : *s_open > 0) return false;
+    for (unsigned t = open; t; t &= t - 1u)
+        amb[atomicAdd(namb, 1)] = (int32_t)(o0 + (int64_t)(__ffs(t) - 1) * kLT);
+    return true;
+}
+
+// a certain label and the reference's distance to its centroid
+template <int DM, bool VEC>
+__device__ __forceinline__ void label_settle(const float *__restrict__ xrow,
+                                             const float *__restrict__ crow, int32_t D, int w,
+                                             int32_t *label, float *dist)
+{
+    float xv[DM], cv[DM];
+    load_row<DM, VEC>(xrow, D, xv);
+    load_row<DM, VEC>(crow, D, cv);
+    *label = w;
+    *dist = (float)exact_dist<DM>(xv, cv, D);
+}
+
+// CK: centroids per chunk; VEC: D equals DM and the rows of X and C can be
+// read as vectors
+template <int DM, int NP, int CK, bool VEC>
+__global__ void __launch_bounds__(kLT, 4)
+k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__restrict__ C,
+            const float *__restrict__ rows, const int32_t *__restrict__ kk, int32_t kmax,
+            int32_t kpad, const int32_t *__restrict__ active, const float *__restrict__ mu,
+            const float *__restrict__ cmax2, float E, int32_t *__restrict__ labels,
+            float *__restrict__ dists, int32_t *__restrict__ amb, int *__restrict__ namb,
+            int32_t *__restrict__ blk, int *__restrict__ nblk)
+{
+    constexpr int RF = LabelRow<DM>::RF, CH = LabelRow<DM>::CH, Q = 2 * NP;
+    __shared__ __align__(16) float cs[2][(CH + 4) * RF];
+    __shared__ int s_open;
+    static_assert(CH % CK == 0 && kTcCentPad % CK == 0, "whole chunks");
+    const int p = blockIdx.y;
+    if (!active[p]) return;
+    const int K = kk[p];
+    const float inf = __int_as_float(0x7f800000), cmax = cmax2[p];
+    const int64_t i0 = (int64_t)blockIdx.x * (Q * kLT) + threadIdx.x;    // point q: i0 + q kLT
+    if (threadIdx.x == 0) s_open = 0;
+    uint64_t x[DM][NP];
+    float xn[Q], b1[Q], b2[Q];
+    int i1[Q];
+    label_points<DM, NP, VEC, true>(X, n, D, i0, mu, x, xn);
+    const float *src = rows + (int64_t)p * kpad * RF;
+    label_sweep<DM, NP, CK, false>(cs, K, x, b1, b2, i1, [&](float *dst, int c0) {
+        for (int e = threadIdx.x; e < CH * RF / 4; e += kLT)     // kpad is a multiple of CH
+            cp_async<16>(dst + 4 * e, src + (int64_t)c0 * RF + 4 * e);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    });
+    unsigned open = 0;                           // points that are not certain
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const int64_t i = i0 + q * kLT;
         if (i >= n) continue;
-        const int64_t o = (int64_t)p * n + i;
         // the winner and the runner-up inside its chunk, by the same scores
-        const float *rg = rows + ((int64_t)p * kpad + CK * i1[q]) * RF;
+        const float *rg = src + (int64_t)CK * i1[q] * RF;
         int bi = -1;
         float ncw = 0.f, best = inf;
 #pragma unroll
@@ -255,14 +324,160 @@ k_label_f32(const float *__restrict__ X, int32_t n, int32_t D, const float *__re
         const float far = xn[q] + 2.f * b1[q] + ew;
         const float rc = sqrtf(xn[q]) + sqrtf(fmaxf(0.f, far));
         const float bound = 1.01f * (ew + E * (xn[q] + fminf(rc * rc, cmax))) + 1e-36f;
-        if (2.f * (b2[q] - b1[q]) > bound && bi >= 0 && far < 3e38f && cmax == cmax) {
-            float xv[DM], cv[DM];
-            load_row<DM, VEC>(X + i * D, D, xv);
-            load_row<DM, VEC>(C + ((int64_t)p * kmax + w) * D, D, cv);
-            labels[o] = w;
-            dists[o] = (float)exact_dist<DM>(xv, cv, D);
-        } else {
-            amb[atomicAdd(namb, 1)] = (int32_t)o;
+        if (2.f * (b2[q] - b1[q]) > bound && bi >= 0 && far < 3e38f && cmax == cmax)
+            label_settle<DM, VEC>(X + i * D, C + ((int64_t)p * kmax + w) * D, D, w,
+                                  labels + (int64_t)p * n + i, dists + (int64_t)p * n + i);
+        else
+            open |= 1u << q;
+    }
+    if (!label_listed<Q>(open, (int64_t)p * n + i0, &s_open, amb, namb) && threadIdx.x == 0)
+        blk[atomicAdd(nblk, 1)] = p * (int)gridDim.x + (int)blockIdx.x;
+}
+
+// The blocks of k_label_f32 that were left with many open points (pts points
+// each, nb blocks per partition): their points lie far from the mean compared
+// with the gaps between their centroids, or are tied.  Or every block (blk
+// null), where the work is too small for the mean, the centred rows and the
+// launches that k_label_f32 needs.  Scores are the float32 squared distances,
+// whose error is relative to the distance -- within (D + 2) 2^-24 of the
+// reference's -- so a winner is certain when the next is beyond four times
+// that.  Where more than one point in eight is open even so (ties; any point
+// at all without a list), a last sweep takes every centroid within that bound
+// in the reference's arithmetic and order.
+//
+// Bound by the FMA pipe: an addition and a multiply-add per dimension.  Blobs
+// 1,000 standard deviations apart, 500,000 x 16 points, 4 partitions of 530:
+// 8.9 ms a pass with a warp per open point, 2.35 now (5.06 with scalar
+// differences for every point); 800,000 x 32 in 300: 7.7 -> 1.3.
+template <int DM, int NP, bool VEC>
+__global__ void __launch_bounds__(kLT, 4)
+k_label_direct(const float *__restrict__ X, int32_t n, int32_t D, const float *__restrict__ C,
+               const int32_t *__restrict__ kk, int32_t kmax, int32_t P,
+               const int32_t *__restrict__ active, int32_t *__restrict__ labels,
+               float *__restrict__ dists, int32_t *__restrict__ amb, int *__restrict__ namb,
+               const int32_t *__restrict__ blk, const int *__restrict__ nblk, int pts, int nb)
+{
+    constexpr int RF = LabelRow<DM>::RF, CH = LabelRow<DM>::CH, Q = 2 * NP, CK = 4;
+    __shared__ __align__(16) float cs[2][(CH + 4) * RF];
+    __shared__ int s_open;
+    const float inf = __int_as_float(0x7f800000);
+    const float grow = 1.f + 4.f * (float)(D + 2) * 5.9604645e-8f;       // 2^-24
+    const int per = pts / (Q * kLT);             // steps per block
+    const int64_t steps = (blk ? (int64_t)*nblk : (int64_t)P * nb) * per;
+    for (int64_t t = blockIdx.x; t < steps; t += gridDim.x) {
+        const int b = blk ? blk[t / per] : (int)(t / per), p = b / nb;
+        const int64_t first = (int64_t)(b - p * nb) * pts + (t % per) * (Q * kLT);
+        if (first >= n || !active[p]) continue;  // uniform across the block
+        const int K = kk[p];
+        const int64_t i0 = first + threadIdx.x, o0 = (int64_t)p * n + i0;
+        const float *Cp = C + (int64_t)p * kmax * D;
+        // rows as in k_prep_label_f32, with a zero for the half norm
+        auto stage = [&](float *dst, int c0) {
+            const int m = min(CH, (K - c0 + CK - 1) / CK * CK);
+            for (int e = threadIdx.x; e < m * RF; e += kLT) {
+                const int c = e / RF, d = e % RF - 1;
+                const bool real = c0 + c < K;
+                float v = real || d >= 0 ? 0.f : inf;
+                if (real && d >= 0 && d < D) v = -__ldg(Cp + (int64_t)(c0 + c) * D + d);
+                dst[e] = v;
+            }
+        };
+        uint64_t x[DM][NP];
+        float b1[Q], b2[Q], thr[Q];
+        int i1[Q];
+        label_points<DM, NP, VEC, false>(X, n, D, i0, nullptr, x, thr);
+        // a NaN centroid 0 keeps every point in the reference: none is certain
+        bool nan_first = false;
+        for (int d = 0; d < D; ++d) nan_first |= !(__ldg(Cp + d) == __ldg(Cp + d));
+        __syncthreads();                         // the last step's rows and count are done with
+        if (threadIdx.x == 0) s_open = 0;
+        label_sweep<DM, NP, CK, true>(cs, K, x, b1, b2, i1, stage);
+        unsigned open = 0;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            // the winner and the runner-up inside its chunk, by the same scores
+            int w = -1;
+            float best = inf;
+#pragma unroll
+            for (int c = 0; c < CK; ++c) {
+                if (CK * i1[q] + c >= K) break;
+                float e[DM], s = 0.f;
+                load_row<DM, VEC>(Cp + (int64_t)(CK * i1[q] + c) * D, D, e);
+#pragma unroll
+                for (int d = 0; d < DM; ++d) {
+                    float v[2];
+                    unpack2(x[d][q / 2], v[0], v[1]);
+                    const float diff = __fsub_rn(v[q & 1], e[d]);
+                    s = fmaf(diff, diff, s);
+                }
+                w = s < best ? CK * i1[q] + c : w;
+                b2[q] = fminf(b2[q], fmaxf(best, s));
+                best = fminf(best, s);
+            }
+            // (the absolute part: subnormal squares, D 2^-149 at most)
+            thr[q] = __fadd_ru(__fmul_ru(best, grow), 1e-42f);
+            if (i0 + q * kLT >= n) continue;
+            if (b2[q] > thr[q] && w >= 0 && !nan_first)
+                label_settle<DM, VEC>(X + (i0 + q * kLT) * D, Cp + (int64_t)w * D, D, w,
+                                      labels + o0 + q * kLT, dists + o0 + q * kLT);
+            else
+                open |= 1u << q;
+        }
+        if (label_listed<Q>(open, o0, &s_open, amb, namb)) continue;
+        // (a NaN distance never compares as smaller: the reference keeps one
+        // only from centroid 0, and then to the end)
+        double bd[Q];
+        int bl[Q];
+        unsigned nan0 = 0;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            bd[q] = 0.0;
+            bl[q] = -1;
+        }
+        for (int c0 = 0; c0 < K; c0 += CH) {
+            __syncthreads();
+            stage(cs[0], c0);
+            __syncthreads();
+            const int cn = min(CH, K - c0);
+            for (int c = 0; c < cn; ++c) {
+                const float *row = cs[0] + c * RF;
+                uint64_t acc[NP];
+#pragma unroll
+                for (int j = 0; j < NP; ++j) acc[j] = 0ull;
+#pragma unroll
+                for (int d = 0; d < DM; ++d) {
+                    const uint64_t w = twice(row[1 + d]);
+#pragma unroll
+                    for (int j = 0; j < NP; ++j) acc[j] = score_step2<true>(x[d][j], w, acc[j]);
+                }
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    float s[2];
+                    unpack2(acc[q / 2], s[0], s[1]);
+                    if (!((open >> q) & 1u) || s[q & 1] > thr[q]) continue;
+                    double dist = 0.0;
+#pragma unroll
+                    for (int d = 0; d < DM; ++d) {
+                        float v[2];
+                        unpack2(x[d][q / 2], v[0], v[1]);
+                        const float diff = __fadd_rn(v[q & 1], row[1 + d]);
+                        dist = __dadd_rn(dist, (double)__fmul_rn(diff, diff));
+                    }
+                    if (dist != dist) {
+                        if (c0 + c == 0) nan0 |= 1u << q;
+                    } else if (bl[q] < 0 || dist < bd[q]) {
+                        bd[q] = dist;
+                        bl[q] = c0 + c;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            if (!((open >> q) & 1u)) continue;
+            const bool nan = ((nan0 >> q) & 1u) != 0u;
+            labels[o0 + q * kLT] = nan ? 0 : bl[q];
+            dists[o0 + q * kLT] = nan ? __int_as_float(0x7fffffff) : (float)bd[q];
         }
     }
 }
@@ -896,42 +1111,74 @@ struct KMWS {
     }
 };
 
+// few: k_label_direct alone, for every point
 template <int DM, int NP, int CK>
-static int launch_label(cudaStream_t st, const float *X, int32_t n, int32_t D, int32_t P,
+static int launch_label(cudaStream_t st, bool few, const float *X, int32_t n, int32_t D, int32_t P,
                         const float *C, const int32_t *kk, int32_t kmax, const int32_t *active,
                         int32_t *labels, float *dists, int32_t *amb, int *namb, const TcScratch &s)
 {
+    constexpr int ND = NP < 2 ? NP : 2;           // (k_label_direct has no registers for more)
     static_assert(kTcCentPad % LabelRow<DM>::CH == 0, "whole staging buffers of rows");
-    const int32_t kpad = (int32_t)s.kt_max * kTcCentPad;
-    if (LabelRow<DM>::RF * sizeof(float) > (size_t)2 * s.Kp) return EACB_ERR_INTERNAL;
-    float *rows = reinterpret_cast<float *>(s.B);
-    k_prep_label_f32<DM><<<grid_for((int64_t)P * kpad, 128), 128, 0, st>>>(
-        C, kk, kmax, kpad, P, D, s.mu, active, rows, s.cmax2);
-    EACB_CHECK_LAUNCH();
-    const float E = (float)((3 * D + 12) * ldexp(1.0, -24));
-    const dim3 grid((unsigned)((n + 2 * NP * kLT - 1) / (2 * NP * kLT)), (unsigned)P);
-    ProfScope ps(PROF_KMEANS, st);
+    constexpr int pts = 2 * NP * kLT;
+    static_assert(pts >= kLabelPts, "the block list is sized for blocks of that many points");
+    const int nb = (n + pts - 1) / pts;
     // rows as vectors where their length and place allow it
     const uintptr_t at = (uintptr_t)X | (uintptr_t)C;
-    if (D == DM && at % (DM % 4 == 0 ? 16 : 8) == 0)
-        k_label_f32<DM, NP, CK, true><<<grid, kLT, 0, st>>>(X, n, D, C, rows, kk, kmax, kpad, active,
-                                                        s.mu, s.cmax2, E, labels, dists, amb, namb);
+    const bool vec = D == DM && at % (DM % 4 == 0 ? 16 : 8) == 0;
+    ProfScope ps(PROF_KMEANS, st);
+    if (!few) {
+        const int32_t kpad = (int32_t)s.kt_max * kTcCentPad;
+        if (LabelRow<DM>::RF * sizeof(float) > (size_t)2 * s.Kp) return EACB_ERR_INTERNAL;
+        float *rows = reinterpret_cast<float *>(s.B);
+        k_prep_label_f32<DM><<<grid_for((int64_t)P * kpad, 128), 128, 0, st>>>(
+            C, kk, kmax, kpad, P, D, s.mu, active, rows, s.cmax2);
+        EACB_CHECK_LAUNCH();
+        const float E = (float)((3 * D + 12) * ldexp(1.0, -24));
+        const dim3 grid((unsigned)nb, (unsigned)P);
+        if (vec)
+            k_label_f32<DM, NP, CK, true><<<grid, kLT, 0, st>>>(
+                X, n, D, C, rows, kk, kmax, kpad, active, s.mu, s.cmax2, E, labels, dists, amb, namb,
+                s.blk, s.nblk);
+        else
+            k_label_f32<DM, NP, CK, false><<<grid, kLT, 0, st>>>(
+                X, n, D, C, rows, kk, kmax, kpad, active, s.mu, s.cmax2, E, labels, dists, amb, namb,
+                s.blk, s.nblk);
+        EACB_CHECK_LAUNCH();
+    }
+    const unsigned gd = (unsigned)std::min<int64_t>((int64_t)nb * P * (NP / ND), 148 * 4 * (few ? 4 : 1));
+    int32_t *list = few ? nullptr : amb;
+    const int32_t *blk = few ? nullptr : s.blk;
+    if (vec)
+        k_label_direct<DM, ND, true><<<gd, kLT, 0, st>>>(X, n, D, C, kk, kmax, P, active, labels, dists,
+                                                         list, namb, blk, s.nblk, pts, nb);
     else
-        k_label_f32<DM, NP, CK, false><<<grid, kLT, 0, st>>>(X, n, D, C, rows, kk, kmax, kpad, active,
-                                                         s.mu, s.cmax2, E, labels, dists, amb, namb);
+        k_label_direct<DM, ND, false><<<gd, kLT, 0, st>>>(X, n, D, C, kk, kmax, P, active, labels, dists,
+                                                          list, namb, blk, s.nblk, pts, nb);
     EACB_CHECK_LAUNCH();
     ps.done(0.0);
     return EACB_OK;
 }
 
+// k_label_direct alone up to this many centroids, or this many float32
+// differences (points x centroids x dimensions) in all: it costs twice the
+// arithmetic of k_label_f32 and saves some 20 us of kernels around it.  One
+// pass over 400,000 points: 5 dimensions, 16 centroids 20 us (40 with
+// k_label_f32), 128 centroids 48 (61); 16 dimensions, 16 centroids 41 (57);
+// 32 dimensions, 200 centroids, above the line, 299 and 220.
+constexpr int kLabelFewK = 32;
+constexpr double kLabelFewWork = (double)(1 << 28);
+
 int label_pass_f32(const float *X, int32_t n, int32_t D, int32_t P, const float *C,
                    const int32_t *kk, int32_t kmax, const int32_t *active, int32_t *labels,
                    float *dists, int32_t *amb, int *namb, TcScratch &s, cudaStream_t st)
 {
-    int r = data_mean(X, n, D, s, st);
-    if (r) return r;
-    EACB_CUDA(cudaMemsetAsync(s.cmax2, 0, sizeof(float) * P, st));
-    EACB_CUDA(cudaMemsetAsync(namb, 0, sizeof(int), st));
+    int r;
+    const bool few = kmax <= kLabelFewK || (double)n * P * kmax * D <= kLabelFewWork;
+    if (!few) {
+        if ((r = data_mean(X, n, D, s, st))) return r;
+        EACB_CUDA(cudaMemsetAsync(s.cmax2, 0, sizeof(float) * ((size_t)P + 1), st));   // and nblk
+        EACB_CUDA(cudaMemsetAsync(namb, 0, sizeof(int), st));
+    }
     // more points per thread (fewer reads of the staged rows per distance)
     // while that leaves every SM four blocks
     auto many = [&](int np) {
@@ -943,12 +1190,12 @@ int label_pass_f32(const float *X, int32_t n, int32_t D, int32_t P, const float 
     // tracked throughout; 100 x 10,000, k 75: 39 us against 26 with four)
     const bool wide = kmax >= 256;
 #define EACB_LABEL(DM, NPW, CKW)                                                                 \
-    (!many(NPW) ? launch_label<DM, 1, 4>(st, X, n, D, P, C, kk, kmax, active, labels, dists, amb, \
-                                         namb, s)                                                 \
-     : wide     ? launch_label<DM, NPW, CKW>(st, X, n, D, P, C, kk, kmax, active, labels, dists,  \
-                                             amb, namb, s)                                        \
-                : launch_label<DM, NPW, 4>(st, X, n, D, P, C, kk, kmax, active, labels, dists,    \
-                                           amb, namb, s))
+    (!many(NPW) ? launch_label<DM, 1, 4>(st, few, X, n, D, P, C, kk, kmax, active, labels, dists, \
+                                         amb, namb, s)                                            \
+     : wide     ? launch_label<DM, NPW, CKW>(st, few, X, n, D, P, C, kk, kmax, active, labels,    \
+                                             dists, amb, namb, s)                                 \
+                : launch_label<DM, NPW, 4>(st, few, X, n, D, P, C, kk, kmax, active, labels,      \
+                                           dists, amb, namb, s))
     if (D <= 2) r = EACB_LABEL(2, 4, 8);
     else if (D <= 4) r = EACB_LABEL(4, 4, 8);
     else if (D <= 6) r = EACB_LABEL(6, 4, 4);
@@ -958,7 +1205,7 @@ int label_pass_f32(const float *X, int32_t n, int32_t D, int32_t P, const float 
     else if (D <= 24) r = EACB_LABEL(24, 1, 4);
     else r = EACB_LABEL(32, 1, 4);
 #undef EACB_LABEL
-    if (r) return r;
+    if (r || few) return r;
     return label_exact_points(X, n, D, P, C, kk, kmax, labels, dists, amb, namb, nullptr, st);
 }
 

@@ -37,6 +37,12 @@ __device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
+__device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b)
+{
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ float min3(float a, float b, float c)
 {
     float d;
@@ -96,9 +102,10 @@ static __global__ void k_set2(int32_t *a, int32_t *b, int32_t va, int32_t vb)
 }
 
 // Scratch of the label passes.  Tensor cores: operands in the UMMA layout.
-// Float32: B holds the staged centroid rows (a row's 8 D + 16 bytes, D
-// rounded up to the kernel's, fit the 2 Kp >= 12 D of a tile row).
+// Float32: B holds the staged centroid rows (up to 4 (D + 4) bytes each, D
+// rounded up to the kernel's, which fit the 2 Kp bytes of a tile row).
 constexpr int kTcCentPad = 128;      // centroid rows are padded to tiles of this many
+constexpr int kLabelPts = 256;       // points per block of the float32 pass at least
 struct TcScratch {
     int Kp;              // 6d rounded up to a multiple of 16
     int64_t n_pad;       // points rounded up to the 128-point tile
@@ -108,6 +115,8 @@ struct TcScratch {
     uint8_t *B;          // centroid tiles
     float *nc;           // |c - mu|^2 (+inf for padding)
     float *cmax2;        // per partition max |c - mu|^2
+    int *nblk;           // (behind cmax2) blocks of the float32 pass left with many open points
+    int32_t *blk;        // and which
     float *mu;           // data mean
     double *part;        // column-sum partials
     int *err;

@@ -636,7 +636,9 @@ TcScratch TcScratch::carve(Carver &c, int32_t n, int32_t D, int32_t P, int32_t k
     s.nx = c.take<float>((size_t)s.n_pad);
     s.B = c.take<uint8_t>((size_t)P * s.kt_max * kTN * s.Kp * 2);
     s.nc = c.take<float>((size_t)P * s.kt_max * kTN);
-    s.cmax2 = c.take<float>((size_t)P);
+    s.cmax2 = c.take<float>((size_t)P + 1);
+    s.nblk = (int *)(s.cmax2 + P);
+    s.blk = c.take<int32_t>((size_t)P * (((int64_t)n + kLabelPts - 1) / kLabelPts));
     s.mu = c.take<float>(32);
     s.part = c.take<double>((size_t)32 * kMeanBlocks);
     s.err = c.take<int>(1);

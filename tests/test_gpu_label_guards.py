@@ -103,3 +103,99 @@ def test_label_overflowing_distances(mode, d):
     c = rng.standard_normal((6, d)).astype(np.float32)
     c[:, 0] = [1.16e19, 1.1e19, 1.12e19, 1.07e19, 1.14e19, 1.11e19]
     _check(x, c, mode)
+
+
+def _check_sample(x, c, rows):
+    """The whole call on the GPU, the oracle on some of its points."""
+    from masters_final_b200.cluster.KMeans import kmeans_label
+    with np.errstate(all="ignore"):
+        want = oracle.kmeans_label(x[rows], c)
+    lab, dist = kmeans_label(x, c, label_mode="cuda")
+    assert np.array_equal(lab.cpu().numpy()[rows], want[0])
+    assert np.array_equal(dist.cpu().numpy()[rows], want[1], equal_nan=True)
+
+
+# points from which a thread takes eight or four points at once, and fewer;
+# with these clusters the work is above what the direct kernel takes alone
+SCREEN = [(1, 620_003, 515), (1, 620_003, 1031), (1, 310_003, 1029), (2, 620_003, 257),
+          (2, 620_003, 260), (2, 310_003, 515), (3, 620_003, 261), (3, 620_003, 150),
+          (4, 620_003, 259), (4, 620_003, 131), (4, 310_003, 258), (5, 620_003, 130),
+          (6, 620_003, 127), (6, 310_003, 161), (7, 620_003, 129), (8, 620_003, 66),
+          (8, 310_003, 133), (9, 310_003, 129), (12, 310_003, 130), (12, 120_001, 257),
+          (13, 310_003, 127), (16, 310_003, 67), (16, 120_001, 150), (17, 120_001, 161),
+          (24, 120_001, 130), (25, 120_001, 129), (32, 120_001, 131)]
+
+
+def _screen_case(d, n, k, spread, seed):
+    """Blobs `spread` standard deviations apart at most, centroids among the
+    points with two equal ones, and rows to compare: points on centroids, the
+    last ones, others at random."""
+    rng = np.random.default_rng(seed)
+    at = rng.uniform(-spread, spread, (20, d)).astype(np.float32)
+    x = rng.standard_normal((n, d), dtype=np.float32) + at[rng.integers(0, 20, n)]
+    c = x[rng.choice(n, k, replace=False)].copy()
+    c[k - 1] = c[0]
+    x[:300] = c[rng.integers(0, k, 300)]
+    rows = np.unique(np.concatenate([np.arange(300), np.arange(n - 300, n), rng.choice(n, 2500)]))
+    return x, c, rows
+
+
+@pytest.mark.parametrize("spread", [0.0, 3000.0])
+@pytest.mark.parametrize("d,n,k", SCREEN)
+def test_label_f32_screen(d, n, k, spread):
+    """The screening kernel in each of its shapes: every padded dimension,
+    chunks of four and eight with ragged last ones, all points-per-thread
+    variants; and the direct kernel after it, for blobs so far apart that the
+    screen leaves most points open."""
+    assert d * n * k > 1 << 28 and k > 32
+    _check_sample(*_screen_case(d, n, k, spread, d + n + k))
+
+
+@pytest.mark.parametrize("d,n,k", [(2, 620_003, 260), (5, 620_003, 130), (16, 310_003, 67),
+                                   (32, 120_001, 131)])
+@pytest.mark.parametrize("kind", ["ties", "nan0", "inf", "tiny"])
+def test_label_f32_screen_open_points(kind, d, n, k):
+    """Most points left to the direct kernel's last sweep: integer points with
+    ties all over, a NaN centroid 0, infinite points, subnormal squares."""
+    x, c, rows = _screen_case(d, n, k, 0.0, d)
+    if kind == "ties":
+        x, c = np.round(x), np.round(c)
+    elif kind == "nan0":
+        c[0, d - 1] = np.nan
+    elif kind == "inf":
+        x[1::3, 0] = np.inf
+        x[2::9] = np.nan
+        c[0, 0] = np.inf
+    else:
+        x *= np.float32(1e-22)
+        c *= np.float32(1e-22)
+    _check_sample(x, c, rows)
+
+
+def test_label_time_far_from_mean():
+    """Well-separated blobs cost more than one (a second sweep), by less than
+    the factor of five that makes the screen no faster than differences to
+    begin with."""
+    import torch
+    from masters_final_b200.cluster.KMeans import kmeans_ensemble
+    n, d, k, P = 400_000, 16, 530, 4
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    z = torch.randn((n, d), generator=g, device="cuda")
+    at = (torch.rand((20, d), generator=g, device="cuda") * 2 - 1) * 3000.0
+    far = at[torch.randint(0, 20, (n,), generator=g, device="cuda")] + z
+    rng = np.random.default_rng(1)
+    inits = [rng.choice(n, k, replace=False).tolist() for _ in range(P)]
+
+    def ms(x):
+        best = float("inf")
+        for _ in range(6):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            kmeans_ensemble(x, [k] * P, inits, max_iter=1)
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+
+    assert ms(far) < 5.0 * ms(z)
