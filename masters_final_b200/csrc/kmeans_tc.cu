@@ -424,14 +424,15 @@ k_label_tc(const float *__restrict__ X, int32_t n, int32_t D, int32_t Kp, const 
                 // |c|^2) of the exact one.  A column c* that the exact
                 // arithmetic could rank at or before the least screened one,
                 // w, has |x - c*|^2 <= |x - c_w|^2 <= w1 + |x|^2 + e(w), so
-                // |c*| is at most |x| + sqrt(w1 + |x|^2 + e(w)) and at most
-                // the partition's largest norm; |c_w| is at most the largest
-                // finite norm of its chunk (columns past K have an infinite
-                // one, and no other infinite or NaN norm can win).  No column
-                // outside w's chunk comes before w when the least of them is
-                // more than e(w) + e(c*) above it (the bound taken 1% wide for
-                // the rounding of this arithmetic, with an absolute part for
-                // products that underflow: 6 D of them, below 2^-126 each).
+                // |c*| and |c_w| are at most |x| + sqrt(w1 + |x|^2 + e(w))
+                // and at most the partition's largest norm.  Under the root
+                // |c_w| is at most the largest finite norm of its chunk
+                // (columns past K have an infinite one, and no other infinite
+                // or NaN norm can win).  No column outside w's chunk comes
+                // before w when the least of them is more than e(w) + e(c*)
+                // above it (the bound taken 1% wide for the rounding of this
+                // arithmetic, with an absolute part for products that
+                // underflow: 6 D of them, below 2^-126 each).
                 const float inf = __int_as_float(0x7f800000);
                 const float cm2 = cmax2[p];
                 constexpr int CK = kTcChunk;
@@ -440,9 +441,8 @@ k_label_tc(const float *__restrict__ X, int32_t n, int32_t D, int32_t Kp, const 
                     nc + ((int64_t)p * kt_max * kTN + CK * wi));
                 const float nw = fmaxf(fmaxf(cn.x < inf ? cn.x : 0.f, cn.y < inf ? cn.y : 0.f),
                                        fmaxf(cn.z < inf ? cn.z : 0.f, cn.w < inf ? cn.w : 0.f));
-                const float ew = 0.5f * E * (xn + nw);
-                const float rc = sqrtf(xn) + sqrtf(fmaxf(0.f, w1 + xn + ew));
-                const float bound = 1.01f * (ew + 0.5f * E * (xn + fminf(rc * rc, cm2))) + 1e-35f;
+                const float rc = sqrtf(xn) + sqrtf(fmaxf(0.f, w1 + xn + 0.5f * E * (xn + nw)));
+                const float bound = 1.01f * E * (xn + fminf(rc * rc, cm2)) + 1e-35f;
                 // inside the chunk: direct float32 distances, within (D + 2)
                 // 2^-24 of the reference's (relative), so the least is
                 // certain when the next is beyond four times that
