@@ -121,6 +121,25 @@ def test_centroid_batches(d, offset, f64):
     assert np.array_equal(got.cpu().numpy(), oracle.kmeans_centroids(x, labels, dist, len(sizes), f64=f64))
 
 
+@pytest.mark.parametrize("d", [1, 2, 3, 7, 8, 11, 16, 17, 22, 31, 32])
+@pytest.mark.parametrize("per", [1, 16, 47, 48, 130])
+@pytest.mark.parametrize("f64", [False, True])
+def test_centroid_small_clusters(d, per, f64):
+    """Centroid sums around the average size where the kernel changes, with
+    clusters of one to a few hundred points, and at the dimensions whose rows
+    are copied one, two or more at a time."""
+    import oracle
+    from masters_final_b200.cluster.KMeans import kmeans_centroids
+    rng = np.random.default_rng(d * 1000 + per)
+    k = 90
+    labels = np.minimum((rng.random(k * per) ** 2 * k).astype(np.int32), k - 1)
+    labels[:k] = np.arange(k)
+    x = (rng.standard_normal((labels.size, d)) * 100).astype(np.float32)
+    dist = rng.random(labels.size).astype(np.float32)
+    got = kmeans_centroids(x, labels, dist, k, centroid_mode="f64" if f64 else "numba")
+    assert np.array_equal(got.cpu().numpy(), oracle.kmeans_centroids(x, labels, dist, k, f64=f64))
+
+
 @pytest.mark.parametrize("d", [1, 2, 3, 5, 7, 9, 13, 16, 17, 25, 32])
 @pytest.mark.parametrize("k", [1, 3, 5, 127, 130, 515])
 def test_label_f32_shapes(d, k):
