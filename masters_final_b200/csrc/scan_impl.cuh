@@ -27,7 +27,7 @@ constexpr int64_t scan_tile(int items) { return (int64_t)kScanThreads * items; }
 constexpr int kScanSmallThreads = 1024;
 constexpr int kScanSmallItems = 16;
 constexpr int64_t kScanSmallStep = (int64_t)kScanSmallThreads * kScanSmallItems;
-constexpr int64_t kScanSmallMax = 2 * kScanSmallStep;
+constexpr int64_t kScanSmallMax = 2 * kScanSmallStep;     // (see scan_launch)
 
 struct ScanScratch {
     uint64_t *status;      // kStatusStride words per tile, from the counter's line on
@@ -265,9 +265,12 @@ inline int scan_launch_tiles(const TIn *in, TOut *out, int64_t n, int64_t init, 
 }
 
 // clear_err: also zero the scratch's own error word (the one in the line
-// before the counter).  Up to kScanSmallMax elements (two steps of one
-// block) the clearing memset and the look-back cost more than the one
-// block's second step does.
+// before the counter).  One block takes a stream of one step, and of two where
+// they move 8 bytes per element in whole vectors: there the clearing memset and
+// the look-back cost as much as the second step.  Device time of 20,011 and
+// 32,768 elements, one block against tiles: int32 6.2, 6.0 / 6.2, 6.2 us; off
+// the 16-byte boundary 10.3, 13.6 / 8.2, 8.3; int32 to int64 8.1, 8.9 / 8.2,
+// 6.3, unaligned 16.4, 23.1 / 8.2, 8.2; int64 9.7, 10.8 / 7.9, 6.9.
 template <typename TIn, typename TOut>
 inline int scan_launch(const TIn *in, TOut *out, int64_t n, int64_t init, int64_t *d_total,
                        const ScanScratch &s, cudaStream_t st, bool clear_err = false)
@@ -282,7 +285,7 @@ inline int scan_launch(const TIn *in, TOut *out, int64_t n, int64_t init, int64_
     // 16-byte input vectors, and as many outputs as one holds in one store
     const bool vec = ((uintptr_t)in % 16 == 0) &&
                      ((uintptr_t)out % (16 / sizeof(TIn) * sizeof(TOut)) == 0);
-    if (n <= kScanSmallMax) {
+    if (n <= (vec && sizeof(TIn) + sizeof(TOut) == 8 ? kScanSmallMax : kScanSmallStep)) {
         int *ce = clear_err ? s.err : nullptr;
         if (vec)
             k_scan_small<TIn, TOut, true><<<1, kScanSmallThreads, 0, st>>>(in, out, n, init,
