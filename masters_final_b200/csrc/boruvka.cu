@@ -1580,6 +1580,12 @@ constexpr long long kBarrierSpins = 1ll << 21;  // about a second of waiting
 constexpr int64_t kSoloActive = 1024;           // block 0 alone below these sizes
 constexpr int64_t kSoloEdges = 8192;
 constexpr int kFindLimit = 1 << 20;             // parent-chain steps (a forest is shorter)
+// bits for the active roots beside a count of edge words: a word holds 8 bits
+// of weight or more, two vertices and a spare bit, so there are at most 2^27
+// roots, which leaves the words 2^35 (with 31 bits for the roots, 2^32 words
+// -- a phase of 17 million points can keep as many -- turned the count negative)
+constexpr int kActiveBits = 28;
+static_assert((64 - 1 - 8) / 2 < kActiveBits, "every root counts");
 
 struct GridBarrier {
     unsigned count;       // arrivals since the launch began (never reset inside one)
@@ -2022,14 +2028,14 @@ k_rounds(RoundArgs a)
             // the error flag is read beside the counts; the scans' block
             // barriers publish s_err
             const int e_now = tid == 0 ? *(volatile int *)a.err : 0;
-            // one scan of (edge words << 31) | active roots (below 2^31)
+            // one scan of (edge words << kActiveBits) | active roots
             int64_t x = 0, tot = 0;
             for (int64_t j = tid; j < Pe; j += kRT)
-                x += (__ldcg(a.seg + j) << 31) + __ldcg(a.alen + j);
+                x += (__ldcg(a.seg + j) << kActiveBits) + __ldcg(a.alen + j);
             if (tid == 0) s_err = e_now;
             block_excl_sum_shfl<kRT>(x, tot);
-            En = tot >> 31;
-            An = tot & 0x7fffffffll;
+            En = tot >> kActiveBits;
+            An = tot & (((int64_t)1 << kActiveBits) - 1);
         }
         if (p == 0 && tid == 0 && round < kMaxRounds) {
             a.trace[3 * round] = V;
