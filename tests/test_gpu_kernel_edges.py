@@ -39,6 +39,22 @@ def test_scan_edges(types, n, offset):
         assert np.array_equal(xd.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("fill", [0, 255])
+def test_scan_empty_stream(fill):
+    """No element: the total is the initial value, and the workspace's error
+    word, whatever was there, reads as no error."""
+    import torch
+    from masters_final_b200 import _lib
+    L = _lib.load()
+    total = torch.empty(1, dtype=torch.int64, device="cuda")
+    for f in (L.eacb_scan_excl_i32, L.eacb_scan_excl_i32_i64, L.eacb_scan_excl_i64):
+        ws = torch.full((int(L.eacb_scan_workspace_size(0)),), fill, dtype=torch.uint8, device="cuda")
+        _lib.check(f(None, None, 0, 42, _lib.ptr(total), _lib.ptr(ws), ws.numel(),
+                     _lib.stream_handle()), "scan")
+        _lib.check(L.eacb_workspace_status(_lib.ptr(ws), _lib.stream_handle()), "scan")
+        assert int(total.item()) == 42
+
+
 @pytest.mark.parametrize("kind", ["random", "equal", "few", "ascending", "descending"])
 @pytest.mark.parametrize("n,empty", [(40, 3), (256, 1), (257, 5), (2000, 300), (16383, 2),
                                      (16384, 2), (70001, 1), (70001, 300), (300001, 7)])
