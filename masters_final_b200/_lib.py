@@ -3,9 +3,12 @@
 PyTorch is used only for device buffers and streams.  There is no fallback:
 if the library or a CUDA device is missing, every entry point raises.
 """
+import collections
 import contextlib
 import ctypes
 import os
+import threading
+import weakref
 
 import numpy as np
 
@@ -303,6 +306,38 @@ def to_host(x):
     h.copy_(x.contiguous(), non_blocking=True)
     t.cuda.current_stream(x.device).synchronize()
     return h.numpy()
+
+
+# Page-locked bytes that results kept by to_host_bounded's callers may hold
+# together (torch's allocator keeps as much for reuse once they are dropped).
+PINNED_RESULTS_MAX = 1 << 30
+_pinned = {"bytes": 0}
+_pinned_lock = threading.Lock()
+_pinned_back = collections.deque()        # sizes of dropped results (appended by finalizers)
+
+
+def to_host_bounded(x):
+    """to_host for arrays that live as long as an object a program may keep
+    many of: page-locked while all such arrays together stay within
+    PINNED_RESULTS_MAX, an ordinary array (and copy) past that."""
+    n = x.numel() * x.element_size()
+    with _pinned_lock:
+        while _pinned_back:
+            _pinned["bytes"] -= _pinned_back.popleft()
+        fits = _pinned["bytes"] + n <= PINNED_RESULTS_MAX
+        if fits:
+            _pinned["bytes"] += n
+    if not fits:
+        return x.cpu().numpy()
+    a = None
+    try:
+        a = to_host(x)
+    finally:
+        if a is None or a.base is None:
+            _pinned_back.append(n)
+        else:                              # the buffer's owner, which every view keeps alive
+            weakref.finalize(a.base, _pinned_back.append, n).atexit = False
+    return a
 
 
 def np_dtype_of(x):

@@ -94,7 +94,10 @@ def kmeans_centroids(X, labels, dists, k, centroid_mode="numba", stream=None):
 
 
 class K_Means:
-    """MyML/MyML/cluster/KMeans.py:26 (same arguments and attributes)."""
+    """MyML/MyML/cluster/KMeans.py:26 (same arguments and attributes).
+
+    The arrays that fit leaves behind are views of page-locked memory, up to
+    1 GiB over all estimators that are alive; past that they are ordinary."""
 
     def __init__(self, n_clusters=8, tol=1e-4, max_iter=300, init='random', **kwargs):
         self.n_clusters = n_clusters
@@ -141,9 +144,9 @@ class K_Means:
                                       "through kmeans_ensemble")
         # through pinned buffers: pageable copies of 1,000,000 labels and
         # distances took 2 ms, more than the fit
-        self.labels_ = _lib.to_host(labels[0])
-        self.cluster_centers_ = _lib.to_host(cent[0, :self.n_clusters])
+        self.labels_ = _lib.to_host_bounded(labels[0])
+        self.cluster_centers_ = _lib.to_host_bounded(cent[0, :self.n_clusters])
         self.iters_ = int(iters[0].item())
         self.inertia_ = np.float32(inertia[0].item())
-        self._dists = _lib.to_host(dists[0])
+        self._dists = _lib.to_host_bounded(dists[0])
         return self

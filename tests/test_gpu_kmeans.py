@@ -172,3 +172,38 @@ def test_eac_drop_in_api(T):
     labels = e.finalClustering()
     assert e.n_fclusts == g["n_fclusts"]
     assert np.array_equal(labels, g["final_labels"])
+
+
+def test_fit_pinned_results_are_bounded(T, monkeypatch):
+    """Estimators that are kept hold page-locked results up to the limit
+    together; dropped ones give their share back."""
+    import gc
+    from masters_final_b200 import _lib
+    from masters_final_b200.cluster.KMeans import K_Means
+    gc.collect()
+    monkeypatch.setattr(_lib, "PINNED_RESULTS_MAX", 200_000, raising=False)
+    x = np.random.default_rng(3).standard_normal((20_000, 4)).astype(np.float32)
+
+    def fit():
+        random.seed(5)
+        return K_Means(n_clusters=10, max_iter=2).fit(x)
+
+    def pinned(a):
+        return T.from_numpy(a).is_pinned()
+
+    first = fit()                             # 80,000 + 160 + 80,000 bytes
+    assert pinned(first.labels_) and pinned(first._dists)
+    second = fit()
+    assert not pinned(second.labels_) and not pinned(second._dists)
+    assert np.array_equal(first.labels_, second.labels_)
+    assert np.array_equal(first._dists, second._dists)
+    part = first.labels_[5:9]
+    del first
+    gc.collect()
+    third = fit()                             # the kept view holds the labels' share
+    assert pinned(third.labels_) and not pinned(third._dists)
+    assert np.array_equal(part, third.labels_[5:9])
+    del part, third
+    gc.collect()
+    fourth = fit()
+    assert pinned(fourth.labels_) and pinned(fourth._dists)
