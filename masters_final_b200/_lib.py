@@ -316,28 +316,36 @@ _pinned_lock = threading.Lock()
 _pinned_back = collections.deque()        # sizes of dropped results (appended by finalizers)
 
 
-def to_host_bounded(x):
-    """to_host for arrays that live as long as an object a program may keep
-    many of: page-locked while all such arrays together stay within
-    PINNED_RESULTS_MAX, an ordinary array (and copy) past that."""
-    n = x.numel() * x.element_size()
-    with _pinned_lock:
-        while _pinned_back:
-            _pinned["bytes"] -= _pinned_back.popleft()
-        fits = _pinned["bytes"] + n <= PINNED_RESULTS_MAX
-        if fits:
-            _pinned["bytes"] += n
-    if not fits:
-        return x.cpu().numpy()
-    a = None
-    try:
-        a = to_host(x)
-    finally:
-        if a is None or a.base is None:
-            _pinned_back.append(n)
-        else:                              # the buffer's owner, which every view keeps alive
-            weakref.finalize(a.base, _pinned_back.append, n).atexit = False
-    return a
+def to_host_bounded(*xs):
+    """to_host for the arrays of an object that a program may keep many of:
+    page-locked while all such arrays together stay within PINNED_RESULTS_MAX,
+    ordinary arrays (and copies) past that.  One wait for all of them."""
+    t = torch()
+    out = []
+    for x in xs:
+        n = x.numel() * x.element_size()
+        with _pinned_lock:
+            while _pinned_back:
+                _pinned["bytes"] -= _pinned_back.popleft()
+            fits = 0 < n <= PINNED_RESULTS_MAX - _pinned["bytes"]
+            if fits:
+                _pinned["bytes"] += n
+        if not fits:
+            out.append(x.cpu().numpy())
+            continue
+        a = None
+        try:
+            h = t.empty(tuple(x.shape), dtype=x.dtype, pin_memory=True)
+            h.copy_(x.contiguous(), non_blocking=True)
+            a = h.numpy()
+        finally:
+            if a is None:
+                _pinned_back.append(n)
+            else:                          # the buffer's owner, which every view keeps alive
+                weakref.finalize(a.base, _pinned_back.append, n).atexit = False
+        out.append(a)
+    t.cuda.current_stream(xs[0].device).synchronize()
+    return out
 
 
 def np_dtype_of(x):

@@ -144,9 +144,8 @@ class K_Means:
                                       "through kmeans_ensemble")
         # through pinned buffers: pageable copies of 1,000,000 labels and
         # distances took 2 ms, more than the fit
-        self.labels_ = _lib.to_host_bounded(labels[0])
-        self.cluster_centers_ = _lib.to_host_bounded(cent[0, :self.n_clusters])
+        self.labels_, self.cluster_centers_, self._dists = _lib.to_host_bounded(
+            labels[0], cent[0, :self.n_clusters], dists[0])
         self.iters_ = int(iters[0].item())
         self.inertia_ = np.float32(inertia[0].item())
-        self._dists = _lib.to_host_bounded(dists[0])
         return self

@@ -1149,7 +1149,7 @@ __global__ void k_init_centroids(const float *X, int32_t D, const int32_t *init,
 struct KMWS {
     int *err;
     float *dists;
-    int32_t *active, *iters, *nempty, *amb, *namb;
+    int32_t *active, *iters, *nempty, *amb;
     float *inertia;
     int32_t *members, *mypos, *cnt, *args;
     int64_t *S;
@@ -1169,7 +1169,6 @@ struct KMWS {
         w.active = c.take<int32_t>(P);
         w.iters = c.take<int32_t>(P);
         w.nempty = c.take<int32_t>(P);
-        w.namb = c.take<int32_t>(1);
         w.inertia = c.take<float>(P);
         w.amb = c.take<int32_t>(pn);
         w.members = c.take<int32_t>(pn);
@@ -1191,7 +1190,7 @@ struct KMWS {
 template <int DM, int NP, int CK>
 static int launch_label(cudaStream_t st, bool few, const float *X, int32_t n, int32_t D, int32_t P,
                         const float *C, const int32_t *kk, int32_t kmax, const int32_t *active,
-                        int32_t *labels, float *dists, int32_t *amb, int *namb, const TcScratch &s)
+                        int32_t *labels, float *dists, int32_t *amb, const TcScratch &s)
 {
     constexpr int ND = NP < 2 ? NP : 2;           // (k_label_direct has no registers for more)
     static_assert(kTcCentPad % LabelRow<DM>::CH == 0, "whole staging buffers of rows");
@@ -1213,12 +1212,12 @@ static int launch_label(cudaStream_t st, bool few, const float *X, int32_t n, in
         const dim3 grid((unsigned)nb, (unsigned)P);
         if (vec)
             k_label_f32<DM, NP, CK, true><<<grid, kLT, 0, st>>>(
-                X, n, D, C, rows, kk, kmax, kpad, active, s.mu, s.cmax2, E, labels, dists, amb, namb,
-                s.blk, s.nblk);
+                X, n, D, C, rows, kk, kmax, kpad, active, s.mu, s.cmax2, E, labels, dists, amb,
+                s.namb, s.blk, s.nblk);
         else
             k_label_f32<DM, NP, CK, false><<<grid, kLT, 0, st>>>(
-                X, n, D, C, rows, kk, kmax, kpad, active, s.mu, s.cmax2, E, labels, dists, amb, namb,
-                s.blk, s.nblk);
+                X, n, D, C, rows, kk, kmax, kpad, active, s.mu, s.cmax2, E, labels, dists, amb,
+                s.namb, s.blk, s.nblk);
         EACB_CHECK_LAUNCH();
     }
     const unsigned gd = (unsigned)std::min<int64_t>((int64_t)nb * P * (NP / ND), 148 * 4 * (few ? 4 : 1));
@@ -1226,10 +1225,10 @@ static int launch_label(cudaStream_t st, bool few, const float *X, int32_t n, in
     const int32_t *blk = few ? nullptr : s.blk;
     if (vec)
         k_label_direct<DM, ND, true><<<gd, kLT, 0, st>>>(X, n, D, C, kk, kmax, P, active, labels, dists,
-                                                         list, namb, blk, s.nblk, pts, nb);
+                                                         list, s.namb, blk, s.nblk, pts, nb);
     else
         k_label_direct<DM, ND, false><<<gd, kLT, 0, st>>>(X, n, D, C, kk, kmax, P, active, labels, dists,
-                                                          list, namb, blk, s.nblk, pts, nb);
+                                                          list, s.namb, blk, s.nblk, pts, nb);
     EACB_CHECK_LAUNCH();
     ps.done(0.0);
     return EACB_OK;
@@ -1246,14 +1245,14 @@ constexpr double kLabelFewWork = (double)(1 << 28);
 
 int label_pass_f32(const float *X, int32_t n, int32_t D, int32_t P, const float *C,
                    const int32_t *kk, int32_t kmax, const int32_t *active, int32_t *labels,
-                   float *dists, int32_t *amb, int *namb, TcScratch &s, cudaStream_t st)
+                   float *dists, int32_t *amb, TcScratch &s, cudaStream_t st)
 {
     int r;
     const bool few = kmax <= kLabelFewK || (double)n * P * kmax * D <= kLabelFewWork;
     if (!few) {
         if ((r = data_mean(X, n, D, s, st))) return r;
-        EACB_CUDA(cudaMemsetAsync(s.cmax2, 0, sizeof(float) * ((size_t)P + 1), st));   // and nblk
-        EACB_CUDA(cudaMemsetAsync(namb, 0, sizeof(int), st));
+        // (and nblk, namb)
+        EACB_CUDA(cudaMemsetAsync(s.cmax2, 0, sizeof(float) * ((size_t)P + 2), st));
     }
     // more points per thread (fewer reads of the staged rows per distance)
     // while that leaves every SM four blocks
@@ -1267,11 +1266,11 @@ int label_pass_f32(const float *X, int32_t n, int32_t D, int32_t P, const float 
     const bool wide = kmax >= 256;
 #define EACB_LABEL(DM, NPW, CKW)                                                                 \
     (!many(NPW) ? launch_label<DM, 1, 4>(st, few, X, n, D, P, C, kk, kmax, active, labels, dists, \
-                                         amb, namb, s)                                            \
+                                         amb, s)                                                  \
      : wide     ? launch_label<DM, NPW, CKW>(st, few, X, n, D, P, C, kk, kmax, active, labels,    \
-                                             dists, amb, namb, s)                                 \
+                                             dists, amb, s)                                       \
                 : launch_label<DM, NPW, 4>(st, few, X, n, D, P, C, kk, kmax, active, labels,      \
-                                           dists, amb, namb, s))
+                                           dists, amb, s))
     if (D <= 2) r = EACB_LABEL(2, 4, 8);
     else if (D <= 4) r = EACB_LABEL(4, 4, 8);
     else if (D <= 6) r = EACB_LABEL(6, 4, 4);
@@ -1282,7 +1281,7 @@ int label_pass_f32(const float *X, int32_t n, int32_t D, int32_t P, const float 
     else r = EACB_LABEL(32, 1, 4);
 #undef EACB_LABEL
     if (r || few) return r;
-    return label_exact_points(X, n, D, P, C, kk, kmax, labels, dists, amb, namb, nullptr, st);
+    return label_exact_points(X, n, D, P, C, kk, kmax, labels, dists, amb, s.namb, nullptr, st);
 }
 
 }  // namespace eacb
@@ -1324,10 +1323,10 @@ extern "C" int eacb_kmeans_ensemble(const float *X, int32_t n, int32_t d, int32_
         int s;
         if (label_mode == 1)
             s = label_pass_tc(X, n, d, P, centroids, k, kmax, w.active, labels, w.dists, w.amb,
-                              w.namb, w.tc, st);
+                              w.tc, st);
         else
             s = label_pass_f32(X, n, d, P, centroids, k, kmax, w.active, labels, w.dists, w.amb,
-                               w.namb, w.tc, st);
+                               w.tc, st);
         if (s) return s;
         // the member scratch is free here: at most n / 32 node sums per partition
         if ((s = launch_inertia(st, w.dists, n, P, (float *)w.args, w.active, w.inertia, w.iters,
@@ -1378,7 +1377,6 @@ extern "C" int eacb_kmeans_label(const float *X, int32_t n, int32_t d, const flo
     int *err = c.take<int>(1);
     int32_t *kk = c.take<int32_t>(1);
     int32_t *active = c.take<int32_t>(1);
-    int *namb = c.take<int>(1);
     int32_t *amb = c.take<int32_t>(n);
     TcScratch tc = TcScratch::carve(c, n, d, 1, k);
     tc.err = err;
@@ -1387,8 +1385,8 @@ extern "C" int eacb_kmeans_label(const float *X, int32_t n, int32_t d, const flo
     k_set2<<<1, 1, 0, st>>>(kk, active, k, 1);
     EACB_CHECK_LAUNCH();
     if (label_mode == 1)
-        return label_pass_tc(X, n, d, 1, C, kk, k, active, labels, dists, amb, namb, tc, st);
-    return label_pass_f32(X, n, d, 1, C, kk, k, active, labels, dists, amb, namb, tc, st);
+        return label_pass_tc(X, n, d, 1, C, kk, k, active, labels, dists, amb, tc, st);
+    return label_pass_f32(X, n, d, 1, C, kk, k, active, labels, dists, amb, tc, st);
 }
 
 extern "C" size_t eacb_kmeans_label_workspace_size(int32_t n, int32_t d, int32_t k)

@@ -116,6 +116,7 @@ struct TcScratch {
     float *nc;           // |c - mu|^2 (+inf for padding)
     float *cmax2;        // per partition max |c - mu|^2
     int *nblk;           // (behind cmax2) blocks of the float32 pass left with many open points
+    int *namb;           // (behind it) points left to the exact re-check
     int32_t *blk;        // and which
     float *mu;           // data mean
     double *part;        // column-sum partials
@@ -130,7 +131,7 @@ struct TcScratch {
 // label and distance.
 int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *C,
                   const int32_t *kk, int32_t kmax, const int32_t *active, int32_t *labels,
-                  float *dists, int32_t *amb, int *namb, TcScratch &s, cudaStream_t st);
+                  float *dists, int32_t *amb, TcScratch &s, cudaStream_t st);
 
 // About the data's mean (of a strided sample), once per scratch: the label
 // passes centre on it, which keeps their error bounds small; their results

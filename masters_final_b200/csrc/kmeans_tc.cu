@@ -652,8 +652,9 @@ TcScratch TcScratch::carve(Carver &c, int32_t n, int32_t D, int32_t P, int32_t k
     s.nx = c.take<float>((size_t)s.n_pad);
     s.B = c.take<uint8_t>((size_t)P * s.kt_max * kTN * s.Kp * 2);
     s.nc = c.take<float>((size_t)P * s.kt_max * kTN);
-    s.cmax2 = c.take<float>((size_t)P + 1);
+    s.cmax2 = c.take<float>((size_t)P + 2);
     s.nblk = (int *)(s.cmax2 + P);
+    s.namb = s.nblk + 1;
     s.blk = c.take<int32_t>((size_t)P * (((int64_t)n + kLabelPts - 1) / kLabelPts));
     s.mu = c.take<float>(32);
     s.part = c.take<double>((size_t)32 * kMeanBlocks);
@@ -693,7 +694,7 @@ int label_exact_points(const float *X, int32_t n, int32_t D, int32_t P, const fl
 
 int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *C,
                   const int32_t *kk, int32_t kmax, const int32_t *active, int32_t *labels,
-                  float *dists, int32_t *amb, int *namb, TcScratch &s, cudaStream_t st)
+                  float *dists, int32_t *amb, TcScratch &s, cudaStream_t st)
 {
     if (!s.points_ready) {
         int r = data_mean(X, n, D, s, st);
@@ -703,8 +704,7 @@ int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *
         EACB_CHECK_LAUNCH();
         s.points_ready = true;
     }
-    EACB_CUDA(cudaMemsetAsync(s.cmax2, 0, sizeof(float) * P, st));
-    EACB_CUDA(cudaMemsetAsync(namb, 0, sizeof(int), st));
+    EACB_CUDA(cudaMemsetAsync(s.cmax2, 0, sizeof(float) * ((size_t)P + 2), st));   // and namb
     k_prep_centroids<<<grid_for((int64_t)P * s.kt_max * kTN, 128), 128, 0, st>>>(
         C, kk, kmax, P, D, s.Kp, s.kt_max, s.mu, active, s.B, s.nc, s.cmax2);
     EACB_CHECK_LAUNCH();
@@ -745,7 +745,7 @@ int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *
         if ((ce = allow_max_dyn_smem(kern)) != cudaSuccess) return;
         kern<<<grid, kTThreads, smem_req, st>>>(X, n, D, s.Kp, C, kk, kmax, s.kt_max, P, ppc, active,
                                                 s.A, s.nx, s.B, s.nc, s.cmax2, E, nbuf, labels, dists,
-                                                amb, namb, s.err);
+                                                amb, s.namb, s.err);
     };
     const bool al = ((uintptr_t)X % 16 == 0) && ((uintptr_t)C % 16 == 0);
     if (D == 4 && al) go(k_label_tc<4, true>);
@@ -761,7 +761,7 @@ int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *
     ps.done(0.0);
     k_exact_all<<<296, 256, 0, st>>>(X, n, D, C, kk, kmax, P, active, s.err, labels, dists);
     EACB_CHECK_LAUNCH();
-    return label_exact_points(X, n, D, P, C, kk, kmax, labels, dists, amb, namb, s.err, st);
+    return label_exact_points(X, n, D, P, C, kk, kmax, labels, dists, amb, s.namb, s.err, st);
 }
 
 }  // namespace eacb
