@@ -436,29 +436,8 @@ k_label_tc(const float *__restrict__ X, int32_t n, int32_t D, int32_t Kp, const 
                         w2 = fminf(w2, o1);
                     }
                 }
-                // Column c's screened distance is within e(c) = E/2 (|x|^2 +
-                // |c|^2) of the exact one.  A column c* that the exact
-                // arithmetic could rank at or before the least screened one,
-                // w, has |x - c*|^2 <= |x - c_w|^2 <= w1 + |x|^2 + e(w), so
-                // |c*| and |c_w| are at most |x| + sqrt(w1 + |x|^2 + e(w))
-                // and at most the partition's largest norm.  Under the root
-                // |c_w| is at most the largest finite norm of its chunk
-                // (columns past K have an infinite one, and no other infinite
-                // or NaN norm can win).  No column outside w's chunk comes
-                // before w when the least of them is more than e(w) + e(c*)
-                // above it (the bound taken 1% wide for the rounding of this
-                // arithmetic, with an absolute part for products that
-                // underflow: 6 D of them, below 2^-126 each).
-                const float inf = __int_as_float(0x7f800000);
-                const float cm2 = cmax2[p];
+                const float inf = __int_as_float(0x7f800000), cm2 = cmax2[p];
                 constexpr int CK = kTcChunk;
-                static_assert(CK == 4, "the chunk's norms are one vector");
-                const float4 cn = *reinterpret_cast<const float4 *>(
-                    nc + ((int64_t)p * kt_max * kTN + CK * wi));
-                const float nw = fmaxf(fmaxf(cn.x < inf ? cn.x : 0.f, cn.y < inf ? cn.y : 0.f),
-                                       fmaxf(cn.z < inf ? cn.z : 0.f, cn.w < inf ? cn.w : 0.f));
-                const float rc = sqrtf(xn) + sqrtf(fmaxf(0.f, w1 + xn + 0.5f * E * (xn + nw)));
-                const float bound = 1.01f * E * (xn + fminf(rc * rc, cm2)) + 1e-35f;
                 // inside the chunk: direct float32 distances, within (D + 2)
                 // 2^-24 of the reference's (relative), so the least is
                 // certain when the next is beyond four times that
@@ -479,7 +458,20 @@ k_label_tc(const float *__restrict__ X, int32_t n, int32_t D, int32_t Kp, const 
                 const float thr = __fadd_ru(__fmul_ru(bd, 1.f + 4.f * (float)(D + 2) * 5.9604645e-8f),
                                             1e-38f);
                 const int64_t o = (int64_t)p * n + i;
-                if (w2 - w1 > bound && bd2 > thr && w >= 0 && cm2 == cm2) {
+                // No column outside the chunk comes before w either, when the
+                // least of their screened distances, w2 + |x|^2, is beyond w's
+                // by more than its error: column c's is within e(c) = E/2
+                // (|x|^2 + |c|^2) of the exact one, and a c* that the exact
+                // arithmetic could rank at or before w has |x - c*|^2 <= thr,
+                // so |c*| <= |x| + sqrt(thr), and at most the partition's
+                // largest norm.  (The bound is taken 5% wide for the rounding
+                // of w2 + |x|^2, at most 2^-24 of 2 (|x|^2 + |c*|^2) where 5%
+                // of e(c*) are 2.5 2^-24 of half of that or more, with an
+                // absolute part for products that underflow: 6 D of them,
+                // below 2^-126 each.)
+                const float rc = sqrtf(xn) + sqrtf(thr);
+                const float bound = 0.525f * E * (xn + fminf(rc * rc, cm2)) + 1e-35f;
+                if (w2 + xn > __fadd_ru(thr, bound) && bd2 > thr && w >= 0 && cm2 == cm2) {
                     load_row<DM, VEC>(C + (row0 + w) * D, D, cv);
                     labels[o] = w;
                     dists[o] = (float)exact_dist_reg<DM>(xv, cv, D);
