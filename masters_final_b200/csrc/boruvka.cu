@@ -2564,6 +2564,7 @@ struct Engine {
             return EACB_OK;
         }
         const int64_t ntiles = (n_in + kETile - 1) / kETile;
+        if (ntiles > scan.max_tiles) return EACB_ERR_WORKSPACE;
         EACB_CUDA(scan.clear(ntiles, false, st));
         k_edge_tile<MODE, Src><<<(unsigned)ntiles, kET, 0, st>>>(
             src, n_in, out, best, scan.status, scan.counter, &cnt[C_AUX0], err);

@@ -224,19 +224,6 @@ __device__ __forceinline__ float screen_dist(const float (&x)[DM], const float (
     return acc;
 }
 
-template <int DM>
-__device__ __forceinline__ double exact_dist_reg(const float (&x)[DM], const float (&c)[DM], int D)
-{
-    double dist = 0.0;
-#pragma unroll
-    for (int d = 0; d < DM; ++d)
-        if (d < D) {
-            const float diff = __fsub_rn(x[d], c[d]);
-            dist = __dadd_rn(dist, (double)__fmul_rn(diff, diff));
-        }
-    return dist;
-}
-
 // ---------------------------------------------------------------- labels --
 // columns of which only the least score is kept: the winner's chunk is
 // compared again at the end, a row of D floats per column (with eight columns
@@ -474,7 +461,7 @@ k_label_tc(const float *__restrict__ X, int32_t n, int32_t D, int32_t Kp, const 
                 if (w2 + xn > __fadd_ru(thr, bound) && bd2 > thr && w >= 0 && cm2 == cm2) {
                     load_row<DM, VEC>(C + (row0 + w) * D, D, cv);
                     labels[o] = w;
-                    dists[o] = (float)exact_dist_reg<DM>(xv, cv, D);
+                    dists[o] = (float)exact_dist<DM>(xv, cv, D);
                 } else {
                     amb[atomicAdd(namb, 1)] = (int32_t)o;
                 }
@@ -598,7 +585,7 @@ k_label_exact_tc(const float *__restrict__ X, int32_t n, int32_t D, const float 
             }
             if (d32 > thr) continue;
             load_row<DM, VEC>(Cp + (int64_t)k * D, D, cv);
-            const double dist = exact_dist_reg<DM>(xv, cv, D);
+            const double dist = exact_dist<DM>(xv, cv, D);
             // a NaN never compares as smaller, so the reference keeps one
             // only from centroid 0, and then to the end
             if (dist != dist) {
@@ -625,13 +612,6 @@ k_label_exact_tc(const float *__restrict__ X, int32_t n, int32_t D, const float 
         }
         __syncwarp();                           // the sums are rewritten by the next point
     }
-}
-
-size_t tc_scratch_bytes(int32_t n, int32_t D, int32_t P, int32_t kmax)
-{
-    Carver c(nullptr, 0);
-    TcScratch::carve(c, n, D, P, kmax);
-    return c.off;
 }
 
 TcScratch TcScratch::carve(Carver &c, int32_t n, int32_t D, int32_t P, int32_t kmax)

@@ -253,6 +253,7 @@ inline int scan_launch_tiles(const TIn *in, TOut *out, int64_t n, int64_t init, 
 {
     const int64_t ntiles = (n + scan_tile(ITEMS) - 1) / scan_tile(ITEMS);
     if (ntiles > (int64_t)0x7fffffff) return EACB_ERR_UNSUPPORTED;
+    if (ntiles > s.max_tiles) return EACB_ERR_WORKSPACE;
     EACB_CUDA(s.clear(ntiles, clear_err, st));
     if (vec)
         k_scan<TIn, TOut, true, ITEMS><<<(unsigned)ntiles, kScanThreads, 0, st>>>(

@@ -90,6 +90,3 @@ extern "C" void eacb_profile_read(int64_t *launches, double *ms, double *bytes, 
         if (count) count[i] = eacb::prof().count[i];
     }
 }
-
-namespace eacb {
-}  // namespace eacb
