@@ -64,7 +64,8 @@ constexpr int kCapCols = 40 * 1024;            // capped rows: columns per chunk
 constexpr int kCapSmem = kCapCols * 5;         // byte counters + 32-bit ranks
 constexpr int kMaxP = 255;
 // work queues: 0 count rows, 1 fill rows, 2 capped rows, 3 row order,
-// 4 neighbourhoods, 5 pair tiles (count), 6 pair tiles (fill)
+// 4 neighbourhoods, 5 and 6 the pair-tile items compared in the count and the
+// fill (k_pairs), 7 the others' (k_pairs_tc, then k_pairs_fill)
 constexpr int kQueues = 8;
 
 // pair tiles: 128 rows x 128 columns, labels as 16-bit words (below 2048)
@@ -1082,8 +1083,9 @@ k_pairs(PairCtx pc, TailCtx tc, const int32_t *order, const int64_t *cap_indptr,
 // Bound by the instructions that turn 128 x P labels into one-hot bytes and by
 // the two barriers around them (the product itself takes a tenth of the
 // time).  The count pass of 300,000 points and 100 partitions (545 cluster
-// columns on average) took 9.1 ms by comparison and takes 4.05; 4.56 with 16
-// warps instead of 32.  An item whose operands do not fit shared memory (more
+// columns on average) took 9.1 ms by comparison and takes 4.3 (4.05 with the
+// counts in tiles instead of rows, whose fill was slower; 4.56 then with 16
+// warps instead of 32).  An item whose operands do not fit shared memory (more
 // than about 700 cluster columns) is left to the comparison, and so is every
 // item when P * K passes the cluster map.
 constexpr int kTcPairThreads = 1024;

@@ -10,8 +10,8 @@
 // with the first index winning ties, the stored distance is float32 of it,
 // centroids are float32(float64(float32 sequential sum) / count), the
 // inertia is numpy's float32 pairwise sum of the distances and a partition
-// stops early when it changes by at most tol.  The float32 label pass below
-// screens all centroids and keeps the best two; when the runner-up is outside
+// stops early when it changes by at most tol.  The float32 label passes below
+// screen all centroids and keep the best two; when the runner-up is outside
 // the screening error bound of the winner only the winner's exact distance
 // is computed, otherwise the point is re-labelled in the reference's
 // arithmetic.  The labels are therefore identical to the reference's for any
@@ -43,7 +43,7 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src)
 }
 
 // ------------------------------------------------- float32 label pass --
-// The screen works on data centred at its mean, where |x - c|^2 = |x|^2 +
+// The screen works on data centred near its mean, where |x - c|^2 = |x|^2 +
 // 2 (|c|^2 / 2 - x.c): a centroid's score is its half norm less the dot
 // product, one fused multiply-add per dimension in the centroid's row order,
 // two points at a time (fma.rn.f32x2).  A thread holds 2 NP points in

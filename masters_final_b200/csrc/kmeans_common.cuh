@@ -118,7 +118,7 @@ struct TcScratch {
     int *nblk;           // (behind cmax2) blocks of the float32 pass left with many open points
     int *namb;           // (behind it) points left to the exact re-check
     int32_t *blk;        // and which
-    float *mu;           // data mean
+    float *mu;           // the centre (data_mean)
     double *part;        // column-sum partials
     int *err;
     bool points_ready;   // A / nx depend on X only
@@ -133,9 +133,9 @@ int label_pass_tc(const float *X, int32_t n, int32_t D, int32_t P, const float *
                   const int32_t *kk, int32_t kmax, const int32_t *active, int32_t *labels,
                   float *dists, int32_t *amb, TcScratch &s, cudaStream_t st);
 
-// About the data's mean (of a strided sample), once per scratch: the label
-// passes centre on it, which keeps their error bounds small; their results
-// do not depend on it.
+// A point amid the data (the median of the means of 32 parts of a strided
+// sample), once per scratch: the label passes centre on it, which keeps their
+// error bounds small; their results do not depend on it.
 int data_mean(const float *X, int32_t n, int32_t D, TcScratch &s, cudaStream_t st);
 
 // The reference's label and distance for the *namb listed (partition, point)

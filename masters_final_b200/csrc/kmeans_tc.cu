@@ -1,20 +1,20 @@
 // K-means label pass on tcgen05 tensor cores.
 //
-// dist(x, c) = |x|^2 - 2 x.c + |c|^2 on data centred at its mean.  The dot
+// dist(x, c) = |x|^2 - 2 x.c + |c|^2 on data centred near its mean.  The dot
 // products run as ONE BF16 GEMM with FP32 accumulation in tensor memory:
 // each float32 operand is split into three BF16 parts (h + m + l, ~24
 // significant bits) and the K dimension holds the six products that matter
 // (see put_row), the large h*h group last.  The epilogue (8 warps, one point
 // row per thread, half the columns per warp) reads the accumulator tile
 // from TMEM with tcgen05.ld, forms the screened distances and keeps the best
-// two of the minima of four columns per point, with the winner's four.  A
-// point whose best columns outside the winner's four, or whose distances
-// inside it, are not apart by more than the proven error bound is
-// re-labelled in the reference's arithmetic; every other point gets its
-// winner's exact reference distance.  Labels therefore equal the reference's
+// two of the minima of four columns per point, with the winner's four.  Those
+// four are compared by direct float32 distances; a point whose other three, or
+// whose least column outside them, are not certainly behind is re-labelled in
+// the reference's arithmetic; every other point gets its winner's exact
+// reference distance.  Labels therefore equal the reference's
 // (MyML/MyML/cluster/KMeans.py:453-490) for any input.  2,000,000 x 8, ten
 // partitions of about 1,000: 7.8 ms a pass with an index and a runner-up per
-// column (six instructions), 6.3 now (two and a half).
+// column (six instructions), 6.25 now (two and a half).
 //
 // Shapes: M = 128 points per CTA, N <= 128 centroids per MMA tile, K = 6d
 // padded to a multiple of 16 (<= 192).  Operands are pre-arranged in global

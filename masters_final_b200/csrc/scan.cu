@@ -3,11 +3,12 @@
 // Replaces MyML/MyML/utils/scan.py:144-249 (scan_gpu: a recursive Blelloch
 // scan with one launch per level plus a fix-up pass, int only) and the CPU
 // scans :42-72.  One launch: each CTA takes the next tile index from an
-// atomic counter, loads 16 elements per thread with 128-bit loads that a warp
-// makes back to back, scans them with warp shuffles and the warps' totals
-// with one more, obtains its tile prefix by looking back over its
-// predecessors' published aggregates, and writes its outputs.  HBM traffic is
-// one read and one write of the stream.  A short stream takes one CTA.
+// atomic counter, loads 128 or 64 bytes of the wider type per thread with
+// 128-bit loads that a warp makes back to back, scans them with warp shuffles
+// and the warps' totals with one more, obtains its tile prefix by looking back
+// over its predecessors' published aggregates, and writes its outputs.  HBM
+// traffic is one read and one write of the stream.  A short stream takes one
+// CTA.
 #include "eacb_common.cuh"
 #include "scan_impl.cuh"
 
