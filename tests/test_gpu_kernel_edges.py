@@ -367,3 +367,62 @@ def test_final_clustering_sampled_plan(n):
     first = {}
     want = np.array([first.setdefault(int(x), len(first)) for x in group])
     assert np.array_equal(labels, want)
+
+
+def _block_matrix(n, blocks, kind, offset=0):
+    """All pairs of n points in equal blocks: light entries inside a block,
+    heavier ones between blocks ("apart"), every weight everywhere ("mixed"),
+    or only the heaviest few between blocks ("late")."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + blocks)
+    a, b = torch.triu_indices(n, n, 1, device="cuda")
+    inside = a * blocks // n == b * blocks // n
+    lo, hi = {"apart": (20, 100), "mixed": (256, 0), "late": (250, 252)}[kind]
+    w = torch.where(inside, torch.randint(0, lo, a.shape, generator=g, device="cuda"),
+                    torch.randint(hi, 256, a.shape, generator=g, device="cuda"))
+    ip = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    ip[1:] = torch.cumsum(torch.bincount(a, minlength=n), 0)
+    dat = torch.empty(w.numel() + offset, dtype=torch.uint8, device="cuda")[offset:]
+    dat.copy_(w)
+    return ip, b.int(), dat
+
+
+@pytest.mark.parametrize("n", [2900, 5000])
+@pytest.mark.parametrize("blocks", [2, 10, 100, 300, 1500])
+@pytest.mark.parametrize("kind", ["apart", "mixed", "late"])
+def test_final_blocks(n, blocks, kind):
+    """Dense matrices of few to many components, on both sides of the estimate
+    that decides between the pairs' phase and narrow ones: the clusters equal
+    those of the ordinary phases (which weights one byte off take), and the
+    blocks where they are apart."""
+    from masters_final_b200.EAC.eac import sp_sl_lifetime_csr
+    got = sp_sl_lifetime_csr(*_block_matrix(n, blocks, kind), n, 255)
+    want = sp_sl_lifetime_csr(*_block_matrix(n, blocks, kind, 1), n, 255)
+    assert got[0] == want[0]
+    assert np.array_equal(got[1], want[1])
+    if kind == "apart":
+        assert got[0] == blocks
+        assert np.array_equal(got[1], np.arange(n) * blocks // n)
+
+
+def test_final_time_entries_between_components():
+    """Entries between hundreds of components take no longer than between a
+    few (a quarter for the timing's spread): they took half as long again when
+    all of them went through the pairs of components."""
+    import torch
+    from masters_final_b200.EAC.eac import sp_sl_lifetime_csr
+
+    def ms(blocks):
+        m = _block_matrix(11_600, blocks, "apart")
+        best = float("inf")
+        for _ in range(8):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            sp_sl_lifetime_csr(*m, 11_600, 255)
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+
+    assert ms(300) < 1.25 * ms(10)
