@@ -2576,9 +2576,9 @@ struct Engine {
     // are lighter, which usually join the components; sample() queues the
     // estimate of their weights (outer), and check() looks at the columns that
     // no phase reads then.  (Blocks of equal size, entries
-    // between all: 11,600 points, 300 blocks 1.87 -> 0.60 ms, 2 blocks 1.02 ->
-    // 0.78; 5,000 points, 100 blocks 0.73 -> 0.51; 30,000 points, 100 blocks 4.6
-    // -> 1.1; 0.88, 1.82, 0.67 and 5.8 with ordinary phases alone.)
+    // between all: 11,600 points, 300 blocks 1.87 -> 0.66 ms, 2 blocks 1.02 ->
+    // 0.84; 5,000 points, 100 blocks 0.73 -> 0.52; 30,000 points, 100 blocks 4.6
+    // -> 1.4; 0.88, 1.82, 0.67 and 5.8 with ordinary phases alone.)
     template <typename Build, typename Split, typename Sample, typename Check>
     int run_phased_retry(Pack pk, std::vector<Phase> plan, Build build, Split split, Sample sample,
                          Check check, int64_t nnz, int64_t pair_max, cudaStream_t st)
