@@ -937,6 +937,13 @@ k_fill_empty(const float *X, int32_t n, int32_t D, float *dists, const int64_t *
     namespace cg = cooperative_groups;
     const cg::cluster_group cl = cg::this_cluster();
     const int CL = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    // (a block alone: with many equal keys a step settles one point and is
+    // mostly its barriers; 16,000 points of four distances, 984 empty clusters
+    // 16.6 ms with cluster barriers, 12.7 with the block's)
+    auto sync = [&]() {
+        if (CL > 1) cl.sync();
+        else __syncthreads();
+    };
     __shared__ int s_small[2], s_fb[2], s_bs[2];       // this block's counts, by step parity
     __shared__ float s_key[kFillSeqMax];
     __shared__ int32_t s_arg[kFillSeqMax];
@@ -948,7 +955,7 @@ k_fill_empty(const float *X, int32_t n, int32_t D, float *dists, const int64_t *
     int32_t *sel = sel_all + (int64_t)p * n;           // positions of A, then of B
     const int gt = rank * kFillThreads + (int)threadIdx.x, gs = CL * kFillThreads;
     for (int64_t i = gt; i < n; i += gs) args0[i] = (int32_t)i;
-    cl.sync();
+    sync();
     int lo = 0, hi = n - 1;
     for (int step = 0; hi - lo + 1 > kFillSeqMax; ++step) {
         if (step > kFillRounds) {                      // a NaN pivot does not shrink the range
@@ -965,7 +972,7 @@ k_fill_empty(const float *X, int32_t n, int32_t D, float *dists, const int64_t *
         // the smalls of the range
         const int mine = fill_smalls(key, c0, c1, mid);
         if (threadIdx.x == 0) s_small[ph] = mine;
-        cl.sync();
+        sync();
         int NS = 0;
         for (int q = 0; q < CL; ++q) NS += *cl.map_shared_rank(&s_small[ph], q);
         // where the two readings meet and which element is read last
@@ -995,7 +1002,7 @@ k_fill_empty(const float *X, int32_t n, int32_t D, float *dists, const int64_t *
             s_fb[ph] = fb;
             s_bs[ph] = bs;
         }
-        cl.sync();
+        sync();
         int64_t base = 0;
         int nA = 0, M = 0;
         for (int q = 0; q < CL; ++q) {
@@ -1011,7 +1018,7 @@ k_fill_empty(const float *X, int32_t n, int32_t D, float *dists, const int64_t *
                 sel[nA + M - 1 - (int)(before & 0xffffffffll)] = t;
             }
         });
-        cl.sync();
+        sync();
         if (k <= r) {
             for (int64_t m = gt; m < M; m += gs) {
                 const int a = sel[m], b = sel[nA + m];
@@ -1038,14 +1045,14 @@ k_fill_empty(const float *X, int32_t n, int32_t D, float *dists, const int64_t *
                 okey[dst] = key[t];
                 oarg[dst] = args[t];
             });
-            cl.sync();
+            sync();
             for (int64_t t = gt; t < L; t += gs) {
                 key[t] = okey[t];
                 args[t] = oarg[t];
             }
             lo = r + 1;
         }
-        cl.sync();
+        sync();
     }
     if (rank != 0) return;
     const int L = hi - lo + 1;
