@@ -2616,8 +2616,8 @@ struct Engine {
             if (prof().enabled) prof().bytes[PROF_PHASE] += 8.0 * (double)Ep;   // words written
             int64_t nc = 0;
             unsigned long long oh[256];
-            if ((s = run<SEL_MST>(pk, Ep, V, st, &n_mst, &nc, sample, pair_max ? oh : nullptr)))
-                return s;
+            const bool ask = pair_max && q + 1 < plan.size() && narrow < kPairNarrow;
+            if ((s = run<SEL_MST>(pk, Ep, V, st, &n_mst, &nc, sample, ask ? oh : nullptr))) return s;
             merged = merged || nc < V;
             V = nc;
             ++q;
@@ -2635,7 +2635,7 @@ struct Engine {
             const int lo = plan[q].lo, hi = plan.back().hi;
             const bool pairs = V <= pair_max && 2 * V * V <= Emax;
             int cut = hi;
-            if (pairs && narrow < kPairNarrow) {
+            if (pairs && ask) {
                 const double each = (double)nnz / kOuterSample;
                 double all = 0.0, light = 0.0;
                 for (int w = lo + 1; w <= hi; ++w) all += each * (double)oh[w];
